@@ -138,6 +138,24 @@ def test_gemm_simt_kernels_agree_bit_for_bit(M):
     assert torch.equal(out, out2)
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(1, 4), (15, 20), (16, 508), (33, 512), (40, 516), (7, 1556)])
+def test_gemm_simt_few_tokens_agree_bit_for_bit(M, N, K):
+    """Up to 16 tokens of 32-bit operands: one lane chains each block of 16 k and another adds the blocks up.  A bias and a sum
+    into the output, around the stage of 512 k and the rows of a block: the same bits as the kernel that reads element by
+    element."""
+    torch.manual_seed(1000 * M + K)
+    a, w = torch.randn(M, K).cuda(), torch.randn(N, K).cuda()
+    b, base = torch.randn(N).cuda(), torch.randn(M, N).cuda()
+    out, out2 = base.clone(), base.clone()
+    ops().gemm_simt(a, w, out, b, True)
+    shifted_a = torch.empty(M * K + 1, device="cuda")[1:].view(M, K)       # 4 bytes past a 16-byte boundary
+    shifted_a.copy_(a)
+    ops().gemm_simt(shifted_a, w, out2, b, True)
+    assert torch.equal(out, out2)
+    close(out, base.double() + a.double() @ w.double().T + b.double(), "float32", scale=float(K) ** 0.5 * 4, what="gemm")
+
+
 # ------------------------------------------------------------------ attention pieces
 def build_cache(seqs_kv, nkv, d, page_size, num_pages, dtype, seed=0, page_order="shuffled"):
     """Scatter each sequence's keys/values into pages; returns cache tensors and the block
