@@ -100,9 +100,9 @@ gemm_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W,
 
 // The same sums, faster: operands come in 16-byte pieces (four consecutive k of a row), the
 // next PF K blocks are already in registers (or on their way) while one is multiplied, and
-// shared memory is double-buffered (one barrier per block of 16).  The order of the sums
-// forbids cutting K among CTAs, so with few tokens and a narrow output the bytes in flight
-// are all the parallelism there is: that kernel keeps eight blocks ahead.  A thread's rows and columns are strided
+// shared memory is double-buffered (one barrier per block of 16): up to 16 rows of bfloat16, and
+// rows dealt to groups.  The order of the sums forbids cutting K among CTAs, so the bytes in
+// flight are all the parallelism there is: eight blocks ahead.  A thread's rows and columns are strided
 // (row ty + i * BM/TM, column tx + j * BN/TN), so a warp reads consecutive words.  Every output is
 // still the same chains of 16 and the same compensated sum in k order as in the kernel above:
 // bit for bit the same result (a zero-padded tail adds +0 to a chain).  Needs K and the leading
@@ -252,7 +252,7 @@ gemm_simt_fast_kernel(const TA* __restrict__ A, const TA* __restrict__ W,
   }
 }
 
-// The same sums again for a handful of tokens (M <= 16) of 32-bit operands, as a stream of weights.  Bound: HBM (a weight is
+// The same sums again for a handful of tokens of 32-bit operands (in groups of 8), as a stream of weights.  Bound: HBM (a weight is
 // read once and multiplied M times; 2 M + 7 M / 16 operations for 4 bytes).  The kernels above give a thread whole outputs, so
 // K is a serial chain of barriers for one 64-column CTA; here the blocks of 16 k of one row go to the 32 lanes of a warp
 // (lane l chains block l of 512 consecutive k), and the block sums then pass through shared memory to one lane per output,
@@ -280,7 +280,10 @@ gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, c
   float* Ws = As + 2 * T * kFewRow;                  // [2][kFewWarps * R][kFewRow]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* parts = Ws + 2 * kFewWarps * R * kFewRow + warp * 32 * (R * T + 1);     // [block][output], one more float between blocks
-  const int n0 = blockIdx.x * (kFewWarps * R);
+  // groups of T tokens of the same weight rows are neighbours in the grid: the rows come from memory once
+  const int groups = (M + T - 1) / T, g0 = (int)(blockIdx.x % (unsigned)groups) * T;
+  A += (size_t)g0 * lda; out += (size_t)g0 * ldo; M -= g0;
+  const int n0 = (int)(blockIdx.x / (unsigned)groups) * (kFewWarps * R);
   // one row of 512 k: 128 pieces of 16 bytes, a warp takes 32 neighbours at a time; what lies outside is filled with zeros
   auto copy_row = [&](const float* src, bool there, float* dst, int k0, int piece) {
     const int k = k0 + piece * 4;
@@ -384,7 +387,162 @@ static int launch_few(const float* A, const float* W, const float* bias, void* o
     once.forget();
     return fail("gemm_simt: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(cudaGetLastError()));
   }
-  ilb::launch(gemm_simt_few_kernel<TO, T, R>, dim3((N + kFewWarps * R - 1) / (kFewWarps * R)), dim3(kFewWarps * 32), smem, stream,
+  ilb::launch(gemm_simt_few_kernel<TO, T, R>, dim3((unsigned)((N + kFewWarps * R - 1) / (kFewWarps * R) * ((M + T - 1) / T))), dim3(kFewWarps * 32), smem, stream,
+              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate);
+  return check_launch("gemm_simt");
+}
+
+// The same sums for many tokens.  Bound: the 32-bit pipes (per output and block of 16 k: 16 multiply-adds and 7 operations of the
+// compensated sum).  A warp has a 32 x 32 tile and a lane 8 x 4 of it, rows in fours: three 16-byte reads of shared memory for 32
+// products.  Two rows go through one packed instruction (fma.rn.f32x2: each half rounds as fmaf does; a - b is fma(b, -1, a), one
+// rounding like __fsub_rn), at the same rate of the pipes and half the instructions to issue.  Operands come in 16-byte pieces, 32 k
+// ahead in registers, 16 rows x 2 pieces a warp and request (whole sectors; rows of k lie 4 floats beyond a multiple of 32, so
+// the transposed stores take different banks).  Row tiles of the same columns are neighbours in the grid: a weight tile comes from
+// memory once.  One layer's products of the 8B sizes, against 128 x 128 tiles of 8 x 8 (256 threads, the chains as separate
+// instructions, 64 to 128 CTAs for 4,096 columns): 64 tokens 5.03 -> 1.64 ms, 128: 5.15 -> 2.72, 200: 5.86 -> 3.98, 512: 8.74 ->
+// 8.00, 1,024: 15.9 -> 15.1.  Measured and dropped: separate instructions here (200 tokens 4.77), three blocks an SM at 168
+// registers (4.58: the reads are no longer a step ahead), 8 x 8 a lane with 4-byte cp.async (4.59; 512 tokens 6.87).
+__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
+constexpr int kWideM = 64, kWideN = 64, kWideK = 32;
+
+template <typename TA, typename TO>
+__global__ void __launch_bounds__(kWideM * kWideN / 32, 2)
+gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias, TO* __restrict__ out,
+                      int M, int N, int K, int lda, int ldw, int ldo, int accumulate) {
+  constexpr int BM = kWideM, BN = kWideN, BK = kWideK;
+  constexpr int WARPS = (BM / 32) * (BN / 32);
+  constexpr int HALVES = BK / 8;                                   // pairs of pieces of a row
+  constexpr int CA = BM / 16 * HALVES / WARPS, CW = BN / 16 * HALVES / WARPS;   // requests of 16 rows x 2 pieces a warp makes per stage
+  static_assert(CA * WARPS * 16 == BM * HALVES && CW * WARPS * 16 == BN * HALVES, "requests divide evenly");
+  __shared__ __align__(16) float As[2][BK][BM + 4];
+  __shared__ __align__(16) float Ws[2][BK][BN + 4];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m_tiles = (M + BM - 1) / BM;
+  const int m0 = (int)(blockIdx.x % (unsigned)m_tiles) * BM, n0 = (int)(blockIdx.x / (unsigned)m_tiles) * BN;
+  const int r0 = (warp / (BN / 32)) * 32 + (lane >> 3) * 4;        // rows r0 .. + 3 and r0 + 16 .. + 19
+  const int c0 = (warp % (BN / 32)) * 32 + (lane & 7) * 4;         // columns c0 .. + 3
+  const bool has_rows = m0 + (warp / (BN / 32)) * 32 < M;
+  const int frow = lane & 15, fpiece = lane >> 4;
+  Vec4<TA> ra[CA], rw[CW];
+  auto fetch = [&](int k0, bool with_w, bool with_a) {
+#pragma unroll
+    for (int i = 0; i < CW; ++i) {
+      const int c = warp + i * WARPS, n = n0 + (c / HALVES) * 16 + frow, k = k0 + ((c % HALVES) * 2 + fpiece) * 4;
+      if (with_w) { if (n < N && k < K) rw[i].load(W + (size_t)n * ldw + k); else rw[i].zero(); }
+    }
+#pragma unroll
+    for (int i = 0; i < CA; ++i) {
+      const int c = warp + i * WARPS, m = m0 + (c / HALVES) * 16 + frow, k = k0 + ((c % HALVES) * 2 + fpiece) * 4;
+      if (with_a) { if (m < M && k < K) ra[i].load(A + (size_t)m * lda + k); else ra[i].zero(); }
+    }
+  };
+  auto stash = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < CW; ++i) {
+      const int c = warp + i * WARPS, row = (c / HALVES) * 16 + frow, k = ((c % HALVES) * 2 + fpiece) * 4;
+      float f[4];
+      rw[i].get(f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) Ws[buf][k + j][row] = f[j];
+    }
+#pragma unroll
+    for (int i = 0; i < CA; ++i) {
+      const int c = warp + i * WARPS, row = (c / HALVES) * 16 + frow, k = ((c % HALVES) * 2 + fpiece) * 4;
+      float f[4];
+      ra[i].get(f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) As[buf][k + j][row] = f[j];
+    }
+  };
+  uint64_t acc[4][4], lost[4][4];                                  // [pair of rows][column]
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = lost[i][j] = 0;
+  const uint64_t minus = pack2(-1.f, -1.f);
+  ilb::pdl_launch_dependents();
+  fetch(0, true, false);                                           // (weights belong to no earlier kernel)
+  ilb::pdl_wait();
+  fetch(0, false, true);
+  stash(0);
+  __syncthreads();
+  const int blocks = (K + BK - 1) / BK;
+  for (int b = 0; b < blocks; ++b) {
+    const int buf = b & 1;
+    if (b + 1 < blocks) fetch((b + 1) * BK, true, true);
+    if (has_rows) {
+#pragma unroll
+      for (int h = 0; h < BK; h += 16) {
+        uint64_t part[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part[i][j] = 0;
+#pragma unroll
+      for (int kk = 0; kk < 16; ++kk) {
+        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[buf][h + kk][r0]);
+        const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[buf][h + kk][r0 + 16]);
+        const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][h + kk][c0]);
+        const uint64_t a[4] = {a0.x, a0.y, a1.x, a1.y};
+        const uint64_t w[4] = {pack2(w4.x, w4.x), pack2(w4.y, w4.y), pack2(w4.z, w4.z), pack2(w4.w, w4.w)};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) part[i][j] = fma2(a[i], w[j], part[i][j]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint64_t s = add2(acc[i][j], part[i][j]);
+          const uint64_t bp = fma2(acc[i][j], minus, s);           // s - acc
+          const uint64_t ea = fma2(fma2(bp, minus, s), minus, acc[i][j]);
+          const uint64_t eb = fma2(bp, minus, part[i][j]);
+          lost[i][j] = add2(lost[i][j], add2(ea, eb));
+          acc[i][j] = s;
+        }
+      }
+    }
+    if (b + 1 < blocks) stash(buf ^ 1);                            // (read last before the barrier at the end of block b - 1)
+    __syncthreads();
+  }
+  if (!has_rows) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float v[2][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint64_t t = add2(acc[i][j], lost[i][j]);
+      unpack2(t, v[0][j], v[1][j]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = m0 + r0 + (i >> 1) * 16 + (i & 1) * 2 + h;
+      if (m >= M) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int n = n0 + c0 + j;
+        if (n >= N) continue;
+        float r = v[h][j];
+        if (bias != nullptr) r += bias[n];
+        TO* o = out + (size_t)m * ldo + n;
+        if (accumulate) r = to_float(*o) + r;
+        *o = from_float<TO>(r);
+      }
+    }
+  }
+}
+
+template <typename TA, typename TO>
+static int launch_wide(const TA* A, const TA* W, const float* bias, void* out, int M, int N, int K, int lda, int ldw, int ldo,
+                       int accumulate, cudaStream_t stream) {
+  const long long tiles = (long long)((M + kWideM - 1) / kWideM) * ((N + kWideN - 1) / kWideN);
+  ILB_REQUIRE(tiles <= 2147483647LL, "gemm_simt: grid too large for M=%d N=%d", M, N);
+  ilb::launch(gemm_simt_wide_kernel<TA, TO>, dim3((unsigned)tiles), dim3(kWideM * kWideN / 32), 0, stream,
               A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate);
   return check_launch("gemm_simt");
 }
@@ -397,16 +555,16 @@ static int launch(const void* A, const void* W, const float* bias, void* out, in
                       (uintptr_t)A % (4 * sizeof(TA)) == 0 && (uintptr_t)W % (4 * sizeof(TA)) == 0;
   const bool grouped = block_group != nullptr;       // groups are dealt in blocks of kGroupRows rows: the 16-row tiles
   if constexpr (std::is_same<TA, float>::value) {
-    // 16-byte pieces for cp.async; up to 16 tokens: a lane adds up one output, so rows a warp x tokens <= 32, and with 16
-    // tokens (two rows a warp) the arithmetic already takes as long as the stream of weights.
-    if (pieces && !grouped && M <= 16) {
+    // 16-byte pieces for cp.async; a lane adds up one output, so rows a warp x tokens <= 32.  The arithmetic grows with every
+    // group of 8 tokens: one layer of the 8B sizes, this kernel against the tiles below: 24 tokens 0.86 / 1.31 ms, 40 tokens
+    // 1.42 / 1.56, 64 tokens 2.27 / 1.64.
+    if (pieces && !grouped && M <= 40) {
       const float* a = (const float*)A;
       const float* w = (const float*)W;
       if (M == 1) return launch_few<TO, 1, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
       if (M == 2) return launch_few<TO, 2, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
       if (M <= 4) return launch_few<TO, 4, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
-      if (M <= 8) return launch_few<TO, 8, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
-      return launch_few<TO, 16, 2>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
+      return launch_few<TO, 8, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
     }
   }
   if (pieces && (M <= 16 || grouped)) {
@@ -415,10 +573,7 @@ static int launch(const void* A, const void* W, const float* bias, void* out, in
     ilb::launch(gemm_simt_fast_kernel<TA, TO, BM, BN, TM, TN, 8>, dim3(grid), dim3((BM / TM) * (BN / TN)), 0, stream,
         (const TA*)A, (const TA*)W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, block_group, group_stride);
   } else if (pieces) {
-    constexpr int BM = 128, BN = 128, TM = 8, TN = 8;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    ilb::launch(gemm_simt_fast_kernel<TA, TO, BM, BN, TM, TN, 2>, dim3(grid), dim3((BM / TM) * (BN / TN)), 0, stream,
-        (const TA*)A, (const TA*)W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, block_group, group_stride);
+    return launch_wide<TA, TO>((const TA*)A, (const TA*)W, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
   } else if (M <= 16 || grouped) {
     constexpr int BM = 16, BN = 32, TM = 2, TN = 2;
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);

@@ -156,6 +156,23 @@ def test_gemm_simt_few_tokens_agree_bit_for_bit(M, N, K):
     close(out, base.double() + a.double() @ w.double().T + b.double(), "float32", scale=float(K) ** 0.5 * 4, what="gemm")
 
 
+@pytest.mark.parametrize("in_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K", [(17, 65, 20), (33, 15, 516), (40, 33, 512), (41, 64, 32), (63, 65, 36), (65, 63, 4), (129, 130, 100), (200, 96, 1028)])
+def test_gemm_simt_many_tokens_agree_bit_for_bit(M, N, K, in_dtype):
+    """Groups of 8 tokens, and 64 x 64 tiles of packed products: around the groups, the tiles, the 32 rows of a warp and the stage
+    of 32 k, with a bias and a sum into the output, the same bits as the kernel that reads element by element."""
+    torch.manual_seed(1000 * M + K)
+    a, w = torch.randn(M, K).to(in_dtype).cuda(), torch.randn(N, K).to(in_dtype).cuda()
+    b, base = torch.randn(N).cuda(), torch.randn(M, N).cuda()
+    out, out2 = base.clone(), base.clone()
+    ops().gemm_simt(a, w, out, b, True)
+    shifted_a = torch.empty(M * K + 1, device="cuda", dtype=in_dtype)[1:].view(M, K)      # one element past a 16-byte boundary
+    shifted_a.copy_(a)
+    ops().gemm_simt(shifted_a, w, out2, b, True)
+    assert torch.equal(out, out2)
+    close(out, base.double() + a.double() @ w.double().T + b.double(), "float32", scale=float(K) ** 0.5 * 4, what="gemm")
+
+
 # ------------------------------------------------------------------ attention pieces
 def build_cache(seqs_kv, nkv, d, page_size, num_pages, dtype, seed=0, page_order="shuffled"):
     """Scatter each sequence's keys/values into pages; returns cache tensors and the block
