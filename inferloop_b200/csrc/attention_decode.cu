@@ -19,9 +19,10 @@
 //            warp takes 16 keys of every tile: S = Q K^T, online softmax in 32-bit, O += P V
 //            with ldmatrix from the swizzled tiles.
 //   merge    a group of up to 16 query heads: the two warps' (max, sum, O) become one record
-//            in the CTA; row r of it is SENT to CTA r % S of the cluster (asynchronous stores
+//            in the CTA, each warp taking half of the columns; without a cluster (S = 1) they write
+//            the rows out, else row r is SENT to CTA r % S of the cluster (asynchronous stores
 //            that count on the owner's mbarrier), and the owner adds the S records of its rows
-//            in the order of the CTAs from its own shared memory.  One cluster barrier, at
+//            in the order of the CTAs from its own shared memory, a warp per row.  One cluster barrier, at
 //            the start (so that every mbarrier is ready); no scratch buffer, no tickets, no
 //            second pass through L2.  Larger groups run in passes of 16 heads whose records
 //            stay where they are and are read by the cluster between two barriers.
@@ -31,6 +32,12 @@
 //            and patches them into the tile in shared memory.  The producer warp then reads
 //            nothing that the preceding kernel writes and starts its stream before the
 //            dependency wait.
+// Bound: the bytes of the cache behind about 6 us of a chain that no byte hides (dependency wait, projection row, norm, the first
+// tile, the two merges).  What was in that chain and need not be: positions read after the wait, norm weights missing L1, the
+// new key made inside its tile, one warp merging for two, a thread walking the records of every element of a row, and the
+// cluster form of the merge with nobody to meet.  Launch after launch, 32 / 8 heads: 1 x 1,030 keys 9.3 -> 6.8 us, 8 x about 770
+// 13.5 -> 11.4, 64 x about 770 46.5 -> 40.9 (31 of bytes); 40 / 8 heads, 19 x about 520: 19.4 -> 16.1; 64 / 8 heads, 2 x about
+// 4,500: 18.8 -> 16.5.
 //   pooled   (kMode 2) a window with pooled blocks before it: the tiles of a second set of pages (row b =
 //            the mean of block b of `pool` positions) come first in the deal, then the window's;
 //            values may have another head size (DV) than keys, q comes ready, and with `turn` the
@@ -196,26 +203,47 @@ __device__ __forceinline__ void tile_step(RowState<DV>& st, const uint32_t (&q)[
   }
 }
 
+// A row of D 32-bit values into L1, 16 bytes a lane, without waiting for it.
+template <int D>
+__device__ __forceinline__ void touch_row(const float* row, int lane) {
+  float a, b, c, d;
+  if (lane < D / 4)
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "l"(row + lane * 4));
+}
+
 // Rows g and g + 8 of the warp's query heads from the fused projection output, as A
 // fragments: per-head RMSNorm in 32-bit (sum over the row's four threads), then the rotation
 // of pairs (i, i + D/2), which a thread holds both members of; rounded to bfloat16 once.
+// A chain of loads, each with the latency of L2: all of a row is asked for before any of it is
+// used, and the norm's weights are in L1 already (`touch_row`; the angles asked for beside the row spilled, and the spills slowed
+// the tile loop from 0.45 to 0.7 us a tile).  `two`: rows 8 .. hold heads at all.
 template <int D>
 __device__ __forceinline__ void load_q_fused(uint32_t (&q)[D / 16][4], const __nv_bfloat16* row0, const __nv_bfloat16* row1,
-                                             const float* weight, float eps, const float2* cs, int lane) {
+                                             const float* weight, float eps, const float2* cs, int lane, bool two) {
   const int t = lane & 3;
+  __nv_bfloat162 raw[D / 16][2];                         // [kk][c, c + 8], c = 16 kk + 2 t
+  auto ask = [&](const __nv_bfloat16* row) {
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        raw[kk][h] = row ? *reinterpret_cast<const __nv_bfloat162*>(row + kk * 16 + 2 * t + 8 * h) : __floats2bfloat162_rn(0.f, 0.f);
+  };
+  ask(row0);
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    const __nv_bfloat16* row = r == 0 ? row0 : row1;
-    float x[D / 16][4];                                  // [kk][c, c+1, c+8, c+9], c = 16 kk + 2 t
+    if (r == 1 && !two) {
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) q[kk][1] = q[kk][3] = 0u;
+      break;
+    }
+    if (r == 1) ask(row1);
+    const bool there = (r == 0 ? row0 : row1) != nullptr;
+    float x[D / 16][4];                                  // [kk][c, c+1, c+8, c+9]
     float ss = 0.f;
 #pragma unroll
     for (int kk = 0; kk < D / 16; ++kk) {
-      const int c = kk * 16 + 2 * t;
-      __nv_bfloat162 a = __floats2bfloat162_rn(0.f, 0.f), b = a;
-      if (row) {
-        a = *reinterpret_cast<const __nv_bfloat162*>(row + c);
-        b = *reinterpret_cast<const __nv_bfloat162*>(row + c + 8);
-      }
+      const __nv_bfloat162 a = raw[kk][0], b = raw[kk][1];
       x[kk][0] = __low2float(a); x[kk][1] = __high2float(a); x[kk][2] = __low2float(b); x[kk][3] = __high2float(b);
 #pragma unroll
       for (int e = 0; e < 4; ++e) ss = fmaf(x[kk][e], x[kk][e], ss);
@@ -234,11 +262,9 @@ __device__ __forceinline__ void load_q_fused(uint32_t (&q)[D / 16][4], const __n
     if (cs != nullptr) {
 #pragma unroll
       for (int kk = 0; kk < D / 32; ++kk) {                // column i < D/2 pairs with i + D/2 = block kk + D/32
-        const int c = kk * 16 + 2 * t;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int i = c + (e & 1) + (e >> 1) * 8;
-          const float2 w = __ldg(cs + i);
+          const float2 w = __ldg(cs + kk * 16 + 2 * t + (e & 1) + (e >> 1) * 8);
           const float a = x[kk][e], b = x[kk + D / 32][e];
           // products and sums rounded separately, as the reference's scalar code does
           x[kk][e] = __fsub_rn(__fmul_rn(a, w.x), __fmul_rn(b, w.y));
@@ -248,8 +274,8 @@ __device__ __forceinline__ void load_q_fused(uint32_t (&q)[D / 16][4], const __n
     }
 #pragma unroll
     for (int kk = 0; kk < D / 16; ++kk) {
-      q[kk][r] = row ? pack_bf16(x[kk][0], x[kk][1]) : 0u;
-      q[kk][2 + r] = row ? pack_bf16(x[kk][2], x[kk][3]) : 0u;
+      q[kk][r] = there ? pack_bf16(x[kk][0], x[kk][1]) : 0u;
+      q[kk][2 + r] = there ? pack_bf16(x[kk][2], x[kk][3]) : 0u;
     }
   }
 }
@@ -335,57 +361,73 @@ __device__ __forceinline__ void load_q_variant(uint32_t (&q)[D / 16][4], const _
   }
 }
 
-// The step's own key and value (row `r` of a tile whose K slices start at `ks`, V slices at
-// `vs`): normed and rotated key, raw value, written over what TMA brought for that row, and
-// to the cache at `k_dst` / `v_dst` if those are not null.  Lane l holds elements
-// E l .. E l + E - 1 of each half of the head (E = D / 64), the members of its rotation pairs.
+// The step's own key and value: asked for before the first tile is looked at; normed and rotated (the value stays as it is)
+// while the tiles are on their way, stored to the cache at `k_dst` / `v_dst` if those are not null, and kept in shared memory
+// (`row`: key, then value; registers it would hold through the tile loop are dear there), from where `patch_row` writes them over
+// what TMA brought.  Lane l holds elements E l .. E l + E - 1 of each half of the head (E = D / 64), the members of its rotation pairs.
 template <int D>
-__device__ __forceinline__ void patch_new_key(uint32_t ks, uint32_t vs, int r, const __nv_bfloat16* k_src,
-                                              const __nv_bfloat16* v_src, const float* k_weight, float eps, const float2* cs,
-                                              __nv_bfloat16* k_dst, __nv_bfloat16* v_dst, int lane) {
-  constexpr int E = D / 64;
-  constexpr uint32_t kSlice = kKeys * 128;
-  float k[2][E], v[2][E];
-  float ss = 0.f;
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int e = h * (D / 2) + E * lane + i;
-      k[h][i] = __bfloat162float(k_src[e]);
-      v[h][i] = __bfloat162float(v_src[e]);
-      ss = fmaf(k[h][i], k[h][i], ss);
-    }
-  if (k_weight != nullptr) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float inv = 1.0f / sqrtf(ss / (float)D + eps);
+struct NewKey {
+  static constexpr int E = D / 64;
+  __nv_bfloat16 k[2][E], v[2][E];
+  float2 angle[E];
+  static __device__ __forceinline__ int element(int h, int i, int lane) { return h * (D / 2) + E * lane + i; }
+  __device__ __forceinline__ void ask(const __nv_bfloat16* k_src, const __nv_bfloat16* v_src, const float2* cs, int lane) {
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int i = 0; i < E; ++i) k[h][i] = k[h][i] * inv * __ldg(k_weight + h * (D / 2) + E * lane + i);
+      for (int i = 0; i < E; ++i) { k[h][i] = k_src[element(h, i, lane)]; v[h][i] = v_src[element(h, i, lane)]; }
+#pragma unroll
+    for (int i = 0; i < E; ++i) angle[i] = cs != nullptr ? __ldg(cs + E * lane + i) : make_float2(1.f, 0.f);
   }
-  if (cs != nullptr) {
+  __device__ __forceinline__ void make(const float* k_weight, float eps, bool rotate, __nv_bfloat16* k_dst, __nv_bfloat16* v_dst,
+                                       __nv_bfloat16* row, int lane) {
+    float x[2][E];
+    float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const float2 w = __ldg(cs + E * lane + i);
-      const float a = k[0][i], b = k[1][i];
-      k[0][i] = __fsub_rn(__fmul_rn(a, w.x), __fmul_rn(b, w.y));
-      k[1][i] = __fadd_rn(__fmul_rn(a, w.y), __fmul_rn(b, w.x));
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < E; ++i) { x[h][i] = __bfloat162float(k[h][i]); ss = fmaf(x[h][i], x[h][i], ss); }
+    if (k_weight != nullptr) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float inv = 1.0f / sqrtf(ss / (float)D + eps);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < E; ++i) x[h][i] = x[h][i] * inv * __ldg(k_weight + element(h, i, lane));
     }
+    if (rotate) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const float a = x[0][i], b = x[1][i];
+        x[0][i] = __fsub_rn(__fmul_rn(a, angle[i].x), __fmul_rn(b, angle[i].y));
+        x[1][i] = __fadd_rn(__fmul_rn(a, angle[i].y), __fmul_rn(b, angle[i].x));
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const int e = element(h, i, lane);
+        const __nv_bfloat16 kb = __float2bfloat16_rn(x[h][i]);
+        row[e] = kb; row[D + e] = v[h][i];
+        if (k_dst != nullptr) { k_dst[e] = kb; v_dst[e] = v[h][i]; }
+      }
+    __syncwarp();
   }
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int e = h * (D / 2) + E * lane + i;
-      const __nv_bfloat16 kb = __float2bfloat16_rn(k[h][i]), vb = __float2bfloat16_rn(v[h][i]);
-      const uint32_t off = (uint32_t)(e >> 6) * kSlice + (uint32_t)r * 128u +
-                           (uint32_t)(((((e & 63) * 2) >> 4) ^ (r & 7)) << 4) + (uint32_t)(((e & 63) * 2) & 15);
-      asm volatile("st.shared.b16 [%0], %1;" ::"r"(ks + off), "h"(*reinterpret_cast<const unsigned short*>(&kb)) : "memory");
-      asm volatile("st.shared.b16 [%0], %1;" ::"r"(vs + off), "h"(*reinterpret_cast<const unsigned short*>(&vb)) : "memory");
-      if (k_dst != nullptr) { k_dst[e] = kb; v_dst[e] = vb; }
-    }
+};
+
+// Row `r` of the tile whose K slices start at `ks`, V slices at `vs`, from the row that NewKey made: 16 bytes a lane.
+template <int D>
+__device__ __forceinline__ void patch_row(uint32_t ks, uint32_t vs, int r, const __nv_bfloat16* row, int lane) {
+  constexpr uint32_t kSlice = kKeys * 128;
+  constexpr int kPieces = D / 8;                           // of a key; as many of a value
+  if (lane < 2 * kPieces) {
+    const int piece = lane % kPieces;
+    const uint4 v = *reinterpret_cast<const uint4*>(row + lane * 8);
+    const uint32_t to = swz((lane < kPieces ? ks : vs) + (uint32_t)(piece >> 3) * kSlice, r, piece & 7);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+  }
   __syncwarp();
 }
 
@@ -481,9 +523,12 @@ __device__ __forceinline__ void patch_new_key_variant(uint32_t ks, uint32_t vs, 
   __syncwarp();
 }
 
+template <int D, int kMode>
+__host__ __device__ constexpr int fresh_bytes() { return kMode == 0 ? 2 * D * 2 : 0; }
+
 // kMode: 0 the stock input stage (or none), 1 its variants, 2 pooled blocks before a window.
 template <int D, int DV, int kStages, int kMode>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, D == 64 ? 5 : 4)      // (the prologue's loads in flight would take twice the registers)
 decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
               const __grid_constant__ CUtensorMap map_k_run, const __grid_constant__ CUtensorMap map_v_run,
               const __grid_constant__ CUtensorMap map_pk, const __grid_constant__ CUtensorMap map_pv, const Params p) {
@@ -507,7 +552,8 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   // Records that the cluster sends here: [source CTA][row of this CTA][DV + 4] (O, max, sum)
   constexpr int kRecIn = DV + 4;
   const uint32_t inbox_bar = smem_u32(bars + 2 * kStages + 1);
-  float* inbox = reinterpret_cast<float*>(bars + 2 * kStages + 2);
+  __nv_bfloat16* fresh_row = reinterpret_cast<__nv_bfloat16*>(bars + 2 * kStages + 2);     // the step's own key and value (kMode 0)
+  float* inbox = reinterpret_cast<float*>(bars + 2 * kStages + 2 + fresh_bytes<D, kMode>() / 8);
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -517,6 +563,7 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   // where they are and the cluster reads them between two barriers.
   const bool push = p.split > 1 && p.nq / p.nkv <= 16;
   const int rows_cap = p.rows_cap;                         // rows an owner holds at most (push)
+  const bool direct = !kPool && p.split == 1 && p.nq / p.nkv <= 16;      // one CTA has the whole sequence: its warps write the rows
   int rows_mine = 0;
   if (push) {
     const int G0 = p.nq / p.nkv, r0 = (int)blockIdx.x;
@@ -536,13 +583,20 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   // one that writes the new position's key and value, nothing the producer warp reads comes
   // from the preceding kernel: it starts the stream of tiles without waiting for it.  Everyone
   // else reads the projection output and waits.
+  // (The consumers read the projection output, but learn their place, and bring the norms' weights into L1, before they wait.)
   const bool stream_early = p.qkv != nullptr && p.k_write != nullptr;
-  if (!(stream_early && (threadIdx.x >> 5) == kConsumers)) pdl_wait();
+  const bool wait_later = stream_early && warp != kConsumers;
+  if (!stream_early) pdl_wait();
+  if (!kPool && wait_later && p.q_weight != nullptr) touch_row<D>(p.q_weight, lane);
+  if (!kPool && wait_later && p.k_weight != nullptr) touch_row<D>(p.k_weight, lane);
 
   const int G = p.nq / p.nkv;
   const int rank = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z / p.chunks, chunk = blockIdx.z % p.chunks;
   const int tok = p.cu_q[seq];
-  if (p.cu_q[seq + 1] - tok != 1) return;                  // the whole cluster leaves together
+  if (p.cu_q[seq + 1] - tok != 1) {                        // the whole cluster leaves together
+    if (wait_later) pdl_wait();                            // (a launch never completes before the one it follows)
+    return;
+  }
   const int pos = p.positions[tok];
   const int lo = first_key(pos, p.window);
   const int hi = pos + 1;
@@ -552,6 +606,7 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   // the clusters that take part for this sequence, and this one's run of tiles
   int chunks_on = all_tiles / (kSplit * kChunkTiles);
   chunks_on = chunks_on < 1 ? 1 : (chunks_on > p.chunks ? p.chunks : chunks_on);
+  if (wait_later) pdl_wait();
   if (chunk >= chunks_on) return;                          // (the whole cluster: nothing has been sent yet)
   const int per_chunk = (all_tiles + chunks_on - 1) / chunks_on;
   const int deal0 = chunk * per_chunk;                     // this cluster's first tile, of all of them
@@ -643,12 +698,19 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
     } else {
       // ------------------------------------------------------------ consumers
       const int g = lane >> 2, t = lane & 3;
-      RowState<DV> st;
-      st.init();
       bool live[2];
       uint32_t q[D / 16][4];
 #pragma unroll
       for (int r = 0; r < 2; ++r) live[r] = rb + g + 8 * r < G;
+      const bool two = G - rb > 8;                         // rows 8 .. of the MMA hold heads
+      // the warp whose keys of the CTA's last tile include the step's own position
+      const bool patches = kMode == 0 && p.qkv != nullptr && p.k_write != nullptr && n_my > 0 && pos >= key_of(n_my - 1) + warp * 16 &&
+                           pos < key_of(n_my - 1) + warp * 16 + 16;
+      NewKey<D> fresh;                                     // (made in the first pass)
+      if (patches && pass == 0) {
+        const __nv_bfloat16* row = p.qkv + (size_t)tok * p.qkv_stride;
+        fresh.ask(row + (size_t)(p.nq + kvh) * D, row + (size_t)(p.nq + p.nkv + kvh) * D, p.rope ? p.rope + (size_t)tok * (D / 2) : nullptr, lane);
+      }
       if (!kPool && p.qkv != nullptr) {
         const __nv_bfloat16* base_q = p.qkv + (size_t)tok * p.qkv_stride + (size_t)(kvh * G + rb) * D;
         if constexpr (kVariant)
@@ -656,7 +718,7 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
                             p.q_weight, p.eps, p.rope ? p.rope + (size_t)tok * (p.rotary_dim / 2) : nullptr, lane, p.mode, p.rotary_dim);
         else
           load_q_fused<D>(q, live[0] ? base_q + (size_t)g * D : nullptr, live[1] ? base_q + (size_t)(g + 8) * D : nullptr,
-                          p.q_weight, p.eps, p.rope ? p.rope + (size_t)tok * (D / 2) : nullptr, lane);
+                          p.q_weight, p.eps, p.rope ? p.rope + (size_t)tok * (D / 2) : nullptr, lane, two);
       } else {
         const __nv_bfloat16* row0 = live[0] ? p.q + (size_t)tok * p.q_stride + (size_t)(kvh * G + rb + g) * D : nullptr;
         const __nv_bfloat16* row1 = live[1] ? p.q + (size_t)tok * p.q_stride + (size_t)(kvh * G + rb + g + 8) * D : nullptr;
@@ -669,6 +731,15 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
           q[kk][3] = row1 ? *reinterpret_cast<const uint32_t*>(row1 + c + 8) : 0u;
         }
       }
+      if (patches && pass == 0) {
+        const int blk = pos / p.page_size;
+        const int pg = blk < p.max_blocks ? __ldg(table + blk) : -1;
+        const bool store = pg >= 0 && pg < p.num_pages;      // never write outside the pool
+        const size_t at = store ? (((size_t)pg * p.nkv + kvh) * p.page_size + (pos % p.page_size)) * D : 0;
+        fresh.make(p.k_weight, p.eps, p.rope != nullptr, store ? p.k_write + at : nullptr, store ? p.v_write + at : nullptr, fresh_row, lane);
+      }
+      RowState<DV> st;
+      st.init();
       bool ok = true;
       for (int j = 0; j < n_my && ok; ++j) {
         const int it = it0 + j, s = it % kStages;
@@ -676,26 +747,24 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
         if (!ok) break;
         const int key0 = key_of(j) + warp * 16;
         const int see_lo = in_pool(j) ? 0 : lo, see_hi = in_pool(j) ? n_pooled : hi;
-        if constexpr (!kPool) if (p.qkv != nullptr && p.k_write != nullptr && pos >= key0 && pos < key0 + 16) {
-          // this warp's slice of this tile holds the step's own position: its key and value
-          // are not in the cache yet (the tile came with whatever the page held there)
+        if (patches && j == n_my - 1) {
+          // the step's own key and value are not in the tile (it came with whatever the page held there)
+          patch_row<D>(base + s * kStage, base + s * kStage + kTensor, pos % kKeys, fresh_row, lane);
+          // TMA will write this stage again later: order these ordinary stores before it
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        if constexpr (kVariant) if (p.qkv != nullptr && p.k_write != nullptr && pos >= key0 && pos < key0 + 16) {
+          // the same, made here
           const __nv_bfloat16* row = p.qkv + (size_t)tok * p.qkv_stride;
           const int blk = pos / p.page_size;
           const int pg = blk < p.max_blocks ? __ldg(table + blk) : -1;
           const bool store = pass == 0 && pg >= 0 && pg < p.num_pages;     // never write outside the pool
           const size_t at = store ? (((size_t)pg * p.nkv + kvh) * p.page_size + (pos % p.page_size)) * D : 0;
-          if constexpr (kVariant)
-            patch_new_key_variant<D>(base + s * kStage, base + s * kStage + kTensor, pos % kKeys,
-                                     row + (size_t)(p.nq + kvh) * D, row + (size_t)(p.nq + p.nkv + kvh) * D, p.k_weight, p.eps,
-                                     p.rope ? p.rope + (size_t)tok * (p.rotary_dim / 2) : nullptr, store ? p.k_write + at : nullptr,
-                                     store ? p.v_write + at : nullptr, lane, p.mode, p.rotary_dim, p.v_mode,
-                                     p.v_first ? p.v_first + ((size_t)tok * p.nkv + kvh) * D : nullptr, p.v_lambda);
-          else
-            patch_new_key<D>(base + s * kStage, base + s * kStage + kTensor, pos % kKeys,
-                             row + (size_t)(p.nq + kvh) * D, row + (size_t)(p.nq + p.nkv + kvh) * D, p.k_weight, p.eps,
-                             p.rope ? p.rope + (size_t)tok * (D / 2) : nullptr, store ? p.k_write + at : nullptr,
-                             store ? p.v_write + at : nullptr, lane);
-          // TMA will write this stage again later: order these ordinary stores before it
+          patch_new_key_variant<D>(base + s * kStage, base + s * kStage + kTensor, pos % kKeys,
+                                   row + (size_t)(p.nq + kvh) * D, row + (size_t)(p.nq + p.nkv + kvh) * D, p.k_weight, p.eps,
+                                   p.rope ? p.rope + (size_t)tok * (p.rotary_dim / 2) : nullptr, store ? p.k_write + at : nullptr,
+                                   store ? p.v_write + at : nullptr, lane, p.mode, p.rotary_dim, p.v_mode,
+                                   p.v_first ? p.v_first + ((size_t)tok * p.nkv + kvh) * D : nullptr, p.v_lambda);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         if (key0 < see_hi)
@@ -705,66 +774,85 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
       }
       if (!ok && lane == 0) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
       __syncwarp();
-      if (push) {
-        // The two warps' records become one (in the order warp 0, warp 1): warp 1 leaves its
-        // fragments in the ring, lane by lane, once both warps are past their last tile.
-        float l2[2];
+      if (push || direct) {
+        // The two warps' records become one (warp 0's terms first).  Warp w keeps the w-th half of the columns and leaves the
+        // other half in the ring, lane by lane, once both warps are past their last tile; rows that hold no head stay out.
+        float l2[2] = {0.f, 0.f};
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
+          if (r == 1 && !two) break;
           float l = st.l[r];
           l += __shfl_xor_sync(0xffffffffu, l, 1);
           l += __shfl_xor_sync(0xffffffffu, l, 2);
           l2[r] = l;
         }
-        constexpr int kDump = DV / 2 + 4;                    // floats a lane leaves: O fragments, two maxima, two sums
-        float* dump = reinterpret_cast<float*>(smem);        // [kDump][32]
-        static_assert(kDump * 32 * 4 <= kStages * (int)kStage, "a warp's fragments must fit the tile ring");
+        constexpr int kHalf = DV / 16;                       // 8-wide column blocks a warp keeps
+        constexpr int kDump = kHalf * 4 + 4;                 // floats a lane leaves: O fragments, two maxima, two sums
+        float* dump = reinterpret_cast<float*>(smem);        // [warp][kDump][32]
+        static_assert(2 * kDump * 32 * 4 <= kStages * (int)kStage, "the warps' fragments must fit the tile ring");
         asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory");
-        if (warp == 1) {
+        float* give = dump + warp * (kDump * 32) + lane;
+        const float* take = dump + (warp ^ 1) * (kDump * 32) + lane;
 #pragma unroll
-          for (int i = 0; i < DV / 8; ++i)
+        for (int r = 0; r < 2; ++r) {
+          if (r == 1 && !two) break;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) dump[(i * 4 + c) * 32 + lane] = st.o[i][c];
+          for (int i = 0; i < kHalf; ++i)
 #pragma unroll
-          for (int r = 0; r < 2; ++r) { dump[(DV / 2 + r) * 32 + lane] = st.m[r]; dump[(DV / 2 + 2 + r) * 32 + lane] = l2[r]; }
+            for (int c = 2 * r; c < 2 * r + 2; ++c) give[(i * 4 + c) * 32] = warp == 0 ? st.o[kHalf + i][c] : st.o[i][c];
+          give[(kHalf * 4 + r) * 32] = st.m[r];
+          give[(kHalf * 4 + 2 + r) * 32] = l2[r];
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory");
-        if (warp == 0) {
-          float f0[2], f1[2];
+        const uint32_t me = (uint32_t)rank;
+        const bool odd = (t & 1) != 0;
+        const int col0 = warp * (DV / 2);
+        const bool out_pairs = p.out_stride % 2 == 0 && (uintptr_t)p.out % 4 == 0;
 #pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const float m1 = dump[(DV / 2 + r) * 32 + lane], l1 = dump[(DV / 2 + 2 + r) * 32 + lane];
-            const float m = fmaxf(st.m[r], m1);
-            f0[r] = st.m[r] == -INFINITY ? 0.f : exp2f(st.m[r] - m);
-            f1[r] = m1 == -INFINITY ? 0.f : exp2f(m1 - m);
-            st.m[r] = m;
-            l2[r] = l2[r] * f0[r] + l1 * f1[r];
-          }
+        for (int r = 0; r < 2; ++r) {
+          if (r == 1 && !two) break;
+          const float m_other = take[(kHalf * 4 + r) * 32], l_other = take[(kHalf * 4 + 2 + r) * 32];
+          const float m = fmaxf(st.m[r], m_other);
+          const float f_mine = st.m[r] == -INFINITY ? 0.f : exp2f(st.m[r] - m);
+          const float f_other = m_other == -INFINITY ? 0.f : exp2f(m_other - m);
+          const float f0 = warp == 0 ? f_mine : f_other, f1 = warp == 0 ? f_other : f_mine;
+          const float l = warp == 0 ? l2[r] * f0 + l_other * f1 : l_other * f0 + l2[r] * f1;
+          float o[kHalf][2];
 #pragma unroll
-          for (int i = 0; i < DV / 8; ++i)
+          for (int i = 0; i < kHalf; ++i)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) st.o[i][c] = st.o[i][c] * f0[c >> 1] + dump[(i * 4 + c) * 32 + lane] * f1[c >> 1];
-          // Row g + 8r goes to CTA (row % S), place row / S.  A lane holds pairs of columns;
-          // neighbours of a quad trade one pair so that each sends 16 bytes at a time.
-          const uint32_t me = (uint32_t)rank;
-          const bool odd = (t & 1) != 0;
+            for (int c = 0; c < 2; ++c) {
+              const float other = take[(i * 4 + 2 * r + c) * 32];
+              o[i][c] = warp == 0 ? st.o[i][2 * r + c] * f0 + other * f1 : other * f0 + st.o[kHalf + i][2 * r + c] * f1;
+            }
+          const int row = g + 8 * r;
+          if (direct) {                                      // nobody else has keys of this sequence
+            if (live[r]) {
+              __nv_bfloat16* dst = p.out + (size_t)tok * p.out_stride + (size_t)(kvh * G + row) * DV + col0 + 2 * t;
 #pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const int row = g + 8 * r;
-            const uint32_t owner = (uint32_t)(row % kSplit);
-            const uint32_t at = smem_u32(inbox) + 4u * (uint32_t)((me * rows_cap + row / kSplit) * kRecIn);
-            const uint32_t dst = peer_addr(at, owner), bar = peer_addr(inbox_bar, owner);
-#pragma unroll
-            for (int i0 = 0; i0 < DV / 8; i0 += 2) {
-              const float ax = st.o[i0][2 * r], ay = st.o[i0][2 * r + 1], bx = st.o[i0 + 1][2 * r], by = st.o[i0 + 1][2 * r + 1];
-              const float rx = __shfl_xor_sync(0xffffffffu, odd ? ax : bx, 1), ry = __shfl_xor_sync(0xffffffffu, odd ? ay : by, 1);
-              if (live[r]) {
-                if (!odd) st_peer_v4(dst + 4u * (uint32_t)(i0 * 8 + 2 * t), bar, ax, ay, rx, ry);
-                else st_peer_v4(dst + 4u * (uint32_t)((i0 + 1) * 8 + 2 * (t - 1)), bar, rx, ry, bx, by);
+              for (int i = 0; i < kHalf; ++i) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(l > 0.f ? o[i][0] / l : 0.f, l > 0.f ? o[i][1] / l : 0.f);
+                if (out_pairs) *reinterpret_cast<__nv_bfloat162*>(dst + i * 8) = h;
+                else { dst[i * 8] = h.x; dst[i * 8 + 1] = h.y; }
               }
             }
-            if (live[r] && t == 0) st_peer_v2(dst + 4u * (uint32_t)DV, bar, st.m[r], l2[r]);
+            continue;
           }
+          // Row g + 8r goes to CTA (row % S), place row / S.  A lane holds pairs of columns;
+          // neighbours of a quad trade one pair so that each sends 16 bytes at a time.
+          const uint32_t owner = (uint32_t)(row % kSplit);
+          const uint32_t at = smem_u32(inbox) + 4u * (uint32_t)((me * rows_cap + row / kSplit) * kRecIn);
+          const uint32_t dst = peer_addr(at, owner), bar = peer_addr(inbox_bar, owner);
+#pragma unroll
+          for (int i0 = 0; i0 < kHalf; i0 += 2) {
+            const float ax = o[i0][0], ay = o[i0][1], bx = o[i0 + 1][0], by = o[i0 + 1][1];
+            const float rx = __shfl_xor_sync(0xffffffffu, odd ? ax : bx, 1), ry = __shfl_xor_sync(0xffffffffu, odd ? ay : by, 1);
+            if (live[r]) {
+              if (!odd) st_peer_v4(dst + 4u * (uint32_t)(col0 + i0 * 8 + 2 * t), bar, ax, ay, rx, ry);
+              else st_peer_v4(dst + 4u * (uint32_t)(col0 + (i0 + 1) * 8 + 2 * (t - 1)), bar, rx, ry, bx, by);
+            }
+          }
+          if (live[r] && t == 0 && warp == 0) st_peer_v2(dst + 4u * (uint32_t)DV, bar, m, l);
         }
       } else {
       // both consumer warps are past their last tile before a record overwrites the ring
@@ -781,6 +869,7 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
       }
       }
     }
+    if (direct) return;
     if (push) {
       // ---- merge of the rows this CTA owns, from its own shared memory, CTA after CTA
       if (rows_mine > 0) {
@@ -811,17 +900,39 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
             });
           }
         } else
-        for (int e = threadIdx.x; e < rows_mine * DV; e += kThreads) {
-          const int slot = e / DV, c = e % DV, row = slot * kSplit + rank;
-          float m_all, l_all;
-          const float o = merged(slot, c, m_all, l_all);
+        // A warp per row: lane i has record i's maximum and sum, every lane DV / 32 columns of all records.
+        for (int slot = warp; slot < rows_mine; slot += kConsumers + 1) {
+          constexpr int kCols = DV / 32;
+          const float* first = inbox + (size_t)slot * kRecIn;
+          const int row = slot * kSplit + rank;
+          const float m = lane < n_rec ? first[(size_t)lane * rows_cap * kRecIn + DV] : -INFINITY;
+          const float l = lane < n_rec ? first[(size_t)lane * rows_cap * kRecIn + DV + 1] : 0.f;
+          const float m_all = warp_max(m);
+          const float f = m == -INFINITY ? 0.f : exp2f(m - m_all);
+          const float l_all = warp_sum(l * f);
+          float o[kCols];
+#pragma unroll
+          for (int c = 0; c < kCols; ++c) o[c] = 0.f;
+#pragma unroll 4
+          for (int i = 0; i < n_rec; ++i) {
+            const float fi = __shfl_sync(0xffffffffu, f, i);
+            const float* rcd = first + (size_t)i * rows_cap * kRecIn + lane * kCols;
+#pragma unroll
+            for (int c = 0; c < kCols; c += 2) {
+              const float2 v = *reinterpret_cast<const float2*>(rcd + c);
+              o[c] += v.x * fi; o[c + 1] += v.y * fi;
+            }
+          }
           if (chunks_on == 1) {
-            p.out[(size_t)tok * p.out_stride + (size_t)(kvh * G + row) * DV + c] = __float2bfloat16_rn(l_all > 0.f ? o / l_all : 0.f);
+            __nv_bfloat16* dst = p.out + (size_t)tok * p.out_stride + (size_t)(kvh * G + row) * DV + lane * kCols;
+#pragma unroll
+            for (int c = 0; c < kCols; ++c) dst[c] = __float2bfloat16_rn(l_all > 0.f ? o[c] / l_all : 0.f);
           } else {
             // this cluster's record of the row, for the owner that comes last
             float* rcd = p.scratch + ((((size_t)seq * p.nkv + kvh) * p.chunks + chunk) * 16 + row) * (DV + 2);
-            rcd[c] = o;
-            if (c == 0) { rcd[DV] = m_all; rcd[DV + 1] = l_all; }
+#pragma unroll
+            for (int c = 0; c < kCols; ++c) rcd[lane * kCols + c] = o[c];
+            if (lane == 0) { rcd[DV] = m_all; rcd[DV + 1] = l_all; }
           }
         }
         if (chunks_on > 1) {
@@ -963,8 +1074,8 @@ int cache_map(CUtensorMap* out, const void* ptr, int d, int page_size, int nkv, 
 }
 
 // Ring, alignment slack, barriers and the flag; the records that a cluster sends to this CTA follow.
-template <int D, int DV, int STAGES>
-constexpr size_t ring_bytes() { return (size_t)STAGES * (D / 64 + DV / 64) * kKeys * 128 + 1024 + (2 * STAGES + 2) * 8; }
+template <int D, int DV, int STAGES, int V>
+constexpr size_t ring_bytes() { return (size_t)STAGES * (D / 64 + DV / 64) * kKeys * 128 + 1024 + (2 * STAGES + 2) * 8 + fresh_bytes<D, V>(); }
 
 // Rows of a group of `group` query heads that one CTA of a cluster of `split` owns at most,
 // and the bytes of the records sent to it (none when the records stay where they are).
@@ -975,7 +1086,7 @@ template <int D, int DV, int STAGES, int V>
 int configure() {
   static OncePerDevice once;
   if (once.first()) {
-    constexpr size_t smem = ring_bytes<D, DV, STAGES>() + (size_t)2 * kMaxSplit * (DV + 4) * 4;   // the most a launch asks for
+    constexpr size_t smem = ring_bytes<D, DV, STAGES, V>() + (size_t)2 * kMaxSplit * (DV + 4) * 4;   // the most a launch asks for
     static_assert(smem <= 227 * 1024, "tile ring does not fit shared memory");
     cudaError_t e = cudaFuncSetAttribute(decode_kernel<D, DV, STAGES, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) once.forget();
@@ -1001,7 +1112,7 @@ int active_clusters(int split, size_t extra) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(split, 64, 8);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = ring_bytes<D, DV, STAGES>() + extra;
+  cfg.dynamicSmemBytes = ring_bytes<D, DV, STAGES, V>() + extra;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
@@ -1016,7 +1127,7 @@ int active_clusters(int split, size_t extra) {
 template <int D, int DV, int STAGES, int V>
 int launch(const CUtensorMap (&m)[6], const Params& p, size_t extra, cudaStream_t stream) {
   if (configure<D, DV, STAGES, V>()) return -1;
-  ilb::launch_cluster(decode_kernel<D, DV, STAGES, V>, dim3(p.split, p.nkv, p.n_seqs * p.chunks), dim3(kThreads), ring_bytes<D, DV, STAGES>() + extra, stream,
+  ilb::launch_cluster(decode_kernel<D, DV, STAGES, V>, dim3(p.split, p.nkv, p.n_seqs * p.chunks), dim3(kThreads), ring_bytes<D, DV, STAGES, V>() + extra, stream,
                       p.split, m[0], m[1], m[2], m[3], m[4], m[5], p);
   return check_launch("attention decode");
 }

@@ -699,6 +699,17 @@ def test_decode_attention_with_the_input_stage_inside(nq, nkv, d, page_size, win
     run_fused_decode(nq, nkv, d, page_size, window, use_norm, use_rope, [1, 2, 16, 17, 32, 33, 48, 64, 65, 100, 257, 700, 1031])
 
 
+@pytest.mark.parametrize("nq,nkv,d,page_size,window", [(16, 16, 128, 16, 0), (144, 16, 128, 16, 0), (32, 16, 64, 32, 40),
+                                                      (256, 16, 64, 16, 0), (272, 16, 64, 16, 0)])
+def test_decode_attention_of_more_sequences_than_ctas(nq, nkv, d, page_size, window):
+    """So many (sequence, kv head) pairs that each gets one CTA: its two warps write the rows out themselves (groups of 1, 2, 9
+    and 16 heads; 17 run in passes).  Lengths that leave the second warp without a key, and the new position on the edges of
+    the warps' 16 keys, of tiles and of pages."""
+    lens = [1, 2, 15, 16, 17, 31, 32, 33, 48, 49, 64, 65, 97, 100, 129, 200] * 3
+    assert ops().attention_decode_plan(len(lens), nq, nkv, d, page_size)[0] == 1
+    run_fused_decode(nq, nkv, d, page_size, window, True, True, lens, key_ulp=True)
+
+
 @pytest.mark.parametrize("lens,window", [([9000], 0), ([5000, 70], 0), ([3, 8200], 3000), ([4100, 4200, 300], 0)])
 def test_decode_attention_of_few_long_sequences(lens, window):
     """With few sequences several clusters share one (sequence, kv head): each takes a run of
@@ -712,7 +723,7 @@ def test_decode_attention_of_few_long_sequences(lens, window):
     assert int(_tc_state(torch.device("cuda", 0)).attn_counters.abs().sum()) == 0       # tickets are back at zero
 
 
-def run_fused_decode(nq, nkv, d, page_size, window, use_norm, use_rope, lens, long_context=False):
+def run_fused_decode(nq, nkv, d, page_size, window, use_norm, use_rope, lens, long_context=False, key_ulp=False):
     o = ops()
     torch.manual_seed(nq + d + page_size)
     eps, theta = 1e-6, 1e4
@@ -760,7 +771,13 @@ def run_fused_decode(nq, nkv, d, page_size, window, use_norm, use_rope, lens, lo
     for s, n in enumerate(lens):             # the new key and value are in the cache now, exactly as the separate kernel rounds them
         page, slot = int(btable[s, (n - 1) // page_size]), (n - 1) % page_size
         assert torch.equal(v_cache[page, :, slot].cpu().double(), v_new[s])
-        close(k_cache[page, :, slot], k_new[s], "bfloat16", scale=float(k_new[s].abs().max()), what="new key")
+        if key_ulp:
+            # both are bfloat16 roundings of values at most a few 2^-24 of the largest apart, so they are the same or
+            # neighbours: at most 2^-7 of the value (among 100,000 keys some lie on a tie)
+            err, ref_k = (k_cache[page, :, slot].cpu().double() - k_new[s]).abs(), k_new[s].abs()
+            assert (err <= 2.0 ** -7 * ref_k + 2.0 ** -20 * ref_k.max()).all() and (err > 0).double().mean() < 0.01
+        else:
+            close(k_cache[page, :, slot], k_new[s], "bfloat16", scale=float(k_new[s].abs().max()), what="new key")
 
 
 @pytest.mark.parametrize("q_len,cluster", [(1, True), (1, False), (5, True)])
