@@ -815,15 +815,20 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
           const float m = fmaxf(st.m[r], m_other);
           const float f_mine = st.m[r] == -INFINITY ? 0.f : exp2f(st.m[r] - m);
           const float f_other = m_other == -INFINITY ? 0.f : exp2f(m_other - m);
-          const float f0 = warp == 0 ? f_mine : f_other, f1 = warp == 0 ? f_other : f_mine;
-          const float l = warp == 0 ? l2[r] * f0 + l_other * f1 : l_other * f0 + l2[r] * f1;
+          // one product is rounded before the other joins it: warp 1's, or in a record that goes nowhere warp 0's (which joined
+          // the sum first there), the same in both warps
+          const bool fused_mine = (warp == 0) != direct;
+          auto join = [&](float mine, float other) {
+            return fused_mine ? fmaf(mine, f_mine, __fmul_rn(other, f_other)) : fmaf(other, f_other, __fmul_rn(mine, f_mine));
+          };
+          const float l = warp == 1 ? fmaf(l2[r], f_mine, __fmul_rn(l_other, f_other)) : fmaf(l_other, f_other, __fmul_rn(l2[r], f_mine));
           float o[kHalf][2];
 #pragma unroll
           for (int i = 0; i < kHalf; ++i)
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
               const float other = take[(i * 4 + 2 * r + c) * 32];
-              o[i][c] = warp == 0 ? st.o[i][2 * r + c] * f0 + other * f1 : other * f0 + st.o[kHalf + i][2 * r + c] * f1;
+              o[i][c] = join(warp == 0 ? st.o[i][2 * r + c] : st.o[kHalf + i][2 * r + c], other);
             }
           const int row = g + 8 * r;
           if (direct) {                                      // nobody else has keys of this sequence
@@ -909,18 +914,18 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
           const float l = lane < n_rec ? first[(size_t)lane * rows_cap * kRecIn + DV + 1] : 0.f;
           const float m_all = warp_max(m);
           const float f = m == -INFINITY ? 0.f : exp2f(m - m_all);
-          const float l_all = warp_sum(l * f);
-          float o[kCols];
+          float o[kCols], l_all = 0.f;                       // (the sums in the order of the CTAs)
 #pragma unroll
           for (int c = 0; c < kCols; ++c) o[c] = 0.f;
 #pragma unroll 4
           for (int i = 0; i < n_rec; ++i) {
             const float fi = __shfl_sync(0xffffffffu, f, i);
+            l_all = fmaf(__shfl_sync(0xffffffffu, l, i), fi, l_all);
             const float* rcd = first + (size_t)i * rows_cap * kRecIn + lane * kCols;
 #pragma unroll
             for (int c = 0; c < kCols; c += 2) {
               const float2 v = *reinterpret_cast<const float2*>(rcd + c);
-              o[c] += v.x * fi; o[c + 1] += v.y * fi;
+              o[c] = fmaf(v.x, fi, o[c]); o[c + 1] = fmaf(v.y, fi, o[c + 1]);
             }
           }
           if (chunks_on == 1) {
