@@ -203,12 +203,15 @@ __device__ __forceinline__ void tile_step(RowState<DV>& st, const uint32_t (&q)[
   }
 }
 
-// A row of D 32-bit values into L1, 16 bytes a lane, without waiting for it.
+// A row of D 32-bit values into L1, without waiting for it.  A value a lane and request: the same lines as wider loads would bring,
+// from any 4-byte boundary (a vector that is a view of a larger buffer).
 template <int D>
 __device__ __forceinline__ void touch_row(const float* row, int lane) {
-  float a, b, c, d;
-  if (lane < D / 4)
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "l"(row + lane * 4));
+#pragma unroll
+  for (int i = 0; i < D; i += 32) {
+    float x;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(x) : "l"(row + i + lane));
+  }
 }
 
 // Rows g and g + 8 of the warp's query heads from the fused projection output, as A
