@@ -88,6 +88,7 @@ struct Params {
   // to write are null) and patched into the tile that holds their position.
   const __nv_bfloat16* qkv; int qkv_stride;
   const float* q_weight; const float* k_weight; float eps;
+  int settled;                         // the weights are older than the launches this one may overlap: they are read before the dependency wait
   const float2* rope;                  // [tokens][rotary_dim / 2] (cos, sin)
   __nv_bfloat16* k_write; __nv_bfloat16* v_write;
   // Variants of the input stage (bits of `mode`, as in qk_norm_rope.cu): 1 = the rotation pairs
@@ -586,12 +587,15 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   // one that writes the new position's key and value, nothing the producer warp reads comes
   // from the preceding kernel: it starts the stream of tiles without waiting for it.  Everyone
   // else reads the projection output and waits.
-  // (The consumers read the projection output, but learn their place, and bring the norms' weights into L1, before they wait.)
+  // (The consumers read the projection output, but learn their place, and bring settled norm weights into L1, before they wait.
+  // A line of L1 that was read too early would stay as it was; weights that the launch before may still be writing are not touched.)
   const bool stream_early = p.qkv != nullptr && p.k_write != nullptr;
   const bool wait_later = stream_early && warp != kConsumers;
   if (!stream_early) pdl_wait();
-  if (!kPool && wait_later && p.q_weight != nullptr) touch_row<D>(p.q_weight, lane);
-  if (!kPool && wait_later && p.k_weight != nullptr) touch_row<D>(p.k_weight, lane);
+  if (!kPool && wait_later && p.settled) {
+    if (p.q_weight != nullptr) touch_row<D>(p.q_weight, lane);
+    if (p.k_weight != nullptr) touch_row<D>(p.k_weight, lane);
+  }
 
   const int G = p.nq / p.nkv;
   const int rank = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z / p.chunks, chunk = blockIdx.z % p.chunks;
@@ -1212,7 +1216,7 @@ ILB_EXPORT long long ilb_attention_decode_scratch_floats(int n_seqs, int nkv, in
 ILB_EXPORT long long ilb_attention_decode_counters(int n_seqs, int nkv) { return (long long)n_seqs * nkv * 16; }
 
 namespace {
-struct InputStage { int mode = 0, rotary_dim = 0, v_mode = 0; void* v_first = nullptr; const float* v_lambda = nullptr; };
+struct InputStage { int settled = 0, mode = 0, rotary_dim = 0, v_mode = 0; void* v_first = nullptr; const float* v_lambda = nullptr; };
 
 int decode_common(const void* q, const void* qkv, int qkv_stride, const float* q_weight, const float* k_weight, float eps,
                   const float* rope, const InputStage& in, int write_kv, void* out, const void* k_cache, const void* v_cache, const int* positions,
@@ -1244,7 +1248,7 @@ int decode_common(const void* q, const void* qkv, int qkv_stride, const float* q
   p.split = 1; p.scale_log2 = scale * kLog2e;
   p.qkv = (const __nv_bfloat16*)qkv; p.qkv_stride = qkv_stride; p.q_weight = q_weight; p.k_weight = k_weight; p.eps = eps;
   p.rope = (const float2*)rope;
-  p.mode = in.mode; p.rotary_dim = in.rotary_dim > 0 ? in.rotary_dim : d; p.v_mode = in.v_mode;
+  p.settled = in.settled; p.mode = in.mode; p.rotary_dim = in.rotary_dim > 0 ? in.rotary_dim : d; p.v_mode = in.v_mode;
   p.v_first = (__nv_bfloat16*)in.v_first; p.v_lambda = in.v_lambda;
   p.k_write = (qkv != nullptr && write_kv) ? (__nv_bfloat16*)const_cast<void*>(k_cache) : nullptr;
   p.v_write = (qkv != nullptr && write_kv) ? (__nv_bfloat16*)const_cast<void*>(v_cache) : nullptr;
@@ -1272,9 +1276,9 @@ ILB_EXPORT int ilb_attention_decode_tma(const void* q, void* out, const void* k_
 // [tokens, (nq + 2 nkv) d]: per-head RMSNorm (q_weight / k_weight [d], or null), rotation over
 // the whole head (rope [tokens, d/2, 2] cos/sin, or null), and, if write_kv, the new key and
 // value stored to the cache.  What qk_norm_rope.cu and this kernel do in two launches.
-// `mode`, `rotary_dim` and the value mixing (`v_mode`, `v_first`, `v_lambda`) are described at Params.
+// `settled`, `mode`, `rotary_dim` and the value mixing (`v_mode`, `v_first`, `v_lambda`) are described at Params.
 ILB_EXPORT int ilb_attention_decode_fused(const void* qkv, int qkv_stride, const float* q_weight, const float* k_weight,
-                                          float eps, const float* rope, int mode, int rotary_dim, int v_mode, void* v_first,
+                                          float eps, int settled, const float* rope, int mode, int rotary_dim, int v_mode, void* v_first,
                                           const float* v_lambda, int write_kv, void* out, void* k_cache,
                                           void* v_cache, const int* positions, const int* cu_q, const int* block_table,
                                           int max_blocks, int page_size, int num_pages, int window, float scale,
@@ -1288,7 +1292,7 @@ ILB_EXPORT int ilb_attention_decode_fused(const void* qkv, int qkv_stride, const
   ILB_REQUIRE(v_mode == 0 || (v_first != nullptr && write_kv), "attention decode: value mixing needs the first values and a cache write");
   ILB_REQUIRE(v_mode != 2 || v_lambda != nullptr, "attention decode: value mixing needs its coefficient");
   InputStage in;
-  in.mode = mode; in.rotary_dim = rotary_dim; in.v_mode = v_mode; in.v_first = v_first; in.v_lambda = v_lambda;
+  in.settled = settled; in.mode = mode; in.rotary_dim = rotary_dim; in.v_mode = v_mode; in.v_first = v_first; in.v_lambda = v_lambda;
   return decode_common(nullptr, qkv, qkv_stride, q_weight, k_weight, eps, rope, in, write_kv, out, k_cache, v_cache, positions,
                        cu_q, block_table, max_blocks, page_size, num_pages, window, scale, n_seqs, nq, nkv, d, 0, out_stride,
                        long_context, scratch, scratch_floats, counters, n_counters, error_flag, stream);

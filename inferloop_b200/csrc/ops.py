@@ -1457,10 +1457,11 @@ def attention_decode_fused_supported(dtype: torch.dtype, cache_dtype: torch.dtyp
 def attention_decode_fused(qkv, out, q_weight, k_weight, eps, rope_table, k_cache, v_cache, write_kv, positions, cu_q,
                            block_table, window, scale, n_seqs, nq, nkv, d, long_context: bool = False, mode: int = 0,
                            rotary_dim: Optional[int] = None, v_first: Optional[torch.Tensor] = None,
-                           v_lambda: Optional[torch.Tensor] = None, v_keep: bool = False) -> None:
+                           v_lambda: Optional[torch.Tensor] = None, v_keep: bool = False, settled: bool = False) -> None:
     """Decode attention with the per-head q/k norm, the rotation and the cache write of the
     step's own key and value inside the attention kernel (one launch instead of two).  `mode`,
-    `rotary_dim`, `v_first`, `v_lambda` and `v_keep` as in `qk_norm_rope_cache`."""
+    `rotary_dim`, `v_first`, `v_lambda` and `v_keep` as in `qk_norm_rope_cache`.  `settled`: no launch since the step's
+    first writes the norm weights (a bound model's): the kernel asks for them while the launch before it is still running."""
     v_mode = 0
     if v_keep or v_lambda is not None:
         _need(v_first, "first values", torch.bfloat16); _need(v_lambda, "value mixing coefficient", torch.float32)
@@ -1478,7 +1479,8 @@ def attention_decode_fused(qkv, out, q_weight, k_weight, eps, rope_table, k_cach
     num_pages, _, page_size, _ = k_cache.shape
     st = _tc_state(qkv.device)
     _call("attention_decode", "ilb_attention_decode_fused", _ptr(qkv), _i(qkv.stride(0)), _ptr(q_weight), _ptr(k_weight),
-          _f(eps if eps and eps > 0 else 1e-6), _ptr(rope_table), _i(mode), _i(d if rotary_dim is None else rotary_dim), _i(v_mode),
+          _f(eps if eps and eps > 0 else 1e-6), _i(1 if settled else 0), _ptr(rope_table), _i(mode), _i(d if rotary_dim is None else rotary_dim),
+          _i(v_mode),
           _ptr(v_first if v_mode else None), _ptr(v_lambda if v_mode == 2 else None), _i(1 if write_kv else 0), _ptr(out),
           _ptr(k_cache), _ptr(v_cache), _ptr(positions),
           _ptr(cu_q), _ptr(block_table), _i(block_table.shape[1]), _i(page_size), _i(num_pages), _i(window or 0),

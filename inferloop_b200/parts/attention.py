@@ -297,7 +297,7 @@ class GQAttention(Mixer):
                                        long_context=step.max_kv_len >= ops.DECODE_LONG_CONTEXT, mode=self.mode,
                                        rotary_dim=self.rotary_dim or None, v_first=v_first,
                                        v_lambda=self.v_lambda if self.value_mix == "mixed" else None,
-                                       v_keep=self.value_mix == "first")
+                                       v_keep=self.value_mix == "first", settled=True)
             self._finish(o, qkv, gate_col0, residual, out)
             return
         q = ws.buffer("attn.q", (T, self.nq * self.d), dt)

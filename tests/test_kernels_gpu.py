@@ -710,34 +710,63 @@ def test_decode_attention_of_more_sequences_than_ctas(nq, nkv, d, page_size, win
     run_fused_decode(nq, nkv, d, page_size, window, True, True, lens, key_ulp=True)
 
 
-@pytest.mark.parametrize("mode", [0, 1])
-@pytest.mark.parametrize("d", [64, 128])
-def test_decode_attention_takes_norm_weights_on_any_boundary(d, mode):
-    """Norm weights may be views of one flat buffer, 4, 8 or 12 bytes past a 16-byte boundary, of the stock input stage and of a
-    variant (pairs of neighbours): the bits of the call whose weights lie on the boundary, in the output and in the cache."""
+def norm_weight_case(d, mode, seed):
+    """A few sequences and `run(q_weight, k_weight, **options)`, which answers the output and both caches."""
     o = ops()
-    torch.manual_seed(d + mode)
+    torch.manual_seed(seed)
     nq, nkv, page, lens = 6, 2, 16, [1, 17, 100, 300]
     S = len(lens)
     old = [(torch.randn(n, nkv, d), torch.randn(n, nkv, d)) for n in lens]
     k_cache, v_cache, btable = build_cache(old, nkv, d, page, sum(-(-n // page) for n in lens) + 1, torch.bfloat16)
     qkv, rope = torch.randn(S, (nq + 2 * nkv) * d).bfloat16().cuda(), torch.randn(S, d // 2, 2).cuda()
     positions, cu, btable = torch.tensor([n - 1 for n in lens], dtype=torch.int32).cuda(), torch.arange(S + 1, dtype=torch.int32).cuda(), btable.cuda()
+
+    def run(qw, kw, before=None, **options):
+        kc, vc, out = k_cache.cuda(), v_cache.cuda(), torch.full((S, nq * d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        if before is not None:
+            before()
+        o.attention_decode_fused(qkv, out, qw, kw, 1e-6, rope, kc, vc, True, positions, cu, btable, 0, d ** -0.5, S, nq, nkv, d, mode=mode, **options)
+        o.check_device_errors()
+        return out, kc, vc
+    return run
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("d", [64, 128])
+def test_decode_attention_takes_norm_weights_on_any_boundary(d, mode):
+    """Norm weights may be views of one flat buffer, 4, 8 or 12 bytes past a 16-byte boundary, of the stock input stage and of a
+    variant (pairs of neighbours): the bits of the call whose weights lie on the boundary, in the output and in the cache."""
+    run = norm_weight_case(d, mode, d + mode)
     weights = 1 + 0.1 * torch.randn(2, d).cuda()
 
-    def run(shift):
+    def at(shift):
         flat = torch.full((2 * d + 8,), float("nan"), device="cuda")
         qw, kw = flat[shift:shift + d], flat[4 + shift + d:4 + shift + 2 * d]
         qw.copy_(weights[0]); kw.copy_(weights[1])
         assert qw.data_ptr() % 16 == kw.data_ptr() % 16 == 4 * shift
-        kc, vc, out = k_cache.cuda(), v_cache.cuda(), torch.full((S, nq * d), float("nan"), dtype=torch.bfloat16, device="cuda")
-        o.attention_decode_fused(qkv, out, qw, kw, 1e-6, rope, kc, vc, True, positions, cu, btable, 0, d ** -0.5, S, nq, nkv, d, mode=mode)
-        o.check_device_errors()
-        return out, kc, vc
-    on_boundary = run(0)
+        return run(qw, kw, settled=True)
+    on_boundary = at(0)
     assert torch.isfinite(on_boundary[0]).all()
     for shift in (1, 2, 3):
-        assert all(torch.equal(a, b) for a, b in zip(on_boundary, run(shift)))
+        assert all(torch.equal(a, b) for a, b in zip(on_boundary, at(shift)))
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_decode_attention_takes_norm_weights_of_the_launch_before(mode):
+    """Weights that the launch right before writes (a long product of one row): launches overlap, the weights are those it
+    leaves, whatever the buffer held."""
+    d, K = 128, 16384
+    run = norm_weight_case(d, mode, 5 + mode)
+    x, m = torch.randn(1, K).bfloat16().cuda(), (torch.randn(2 * d, K) / K ** 0.5).bfloat16().cuda()
+    w = torch.zeros(1, 2 * d, device="cuda")
+    make = lambda: ops().gemm_simt(x, m, w)
+    make()
+    want = run(w[0, :d].clone(), w[0, d:].clone())
+    for _ in range(3):
+        w.zero_()
+        got = run(w[0, :d], w[0, d:], before=make)
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
 
 
 @pytest.mark.parametrize("lens,window", [([9000], 0), ([5000, 70], 0), ([3, 8200], 3000), ([4100, 4200, 300], 0)])
