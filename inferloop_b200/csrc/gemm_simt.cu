@@ -273,7 +273,7 @@ constexpr size_t few_smem(int T, int R) {
 template <typename TO, int T, int R>
 __global__ void __launch_bounds__(kFewWarps * 32)
 gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                     TO* __restrict__ out, int M, int N, int K, int lda, int ldw, int ldo, int accumulate) {
+                     TO* __restrict__ out, int M, int N, int K, int lda, int ldw, int ldo, int accumulate, int settled) {
   static_assert(T * R <= 32, "one lane adds up one output");
   extern __shared__ __align__(16) float few[];
   float* As = few;                                   // [2][T][kFewRow]
@@ -312,8 +312,9 @@ gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, c
   auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
   const int rounds = (K + kFewK - 1) / kFewK, blocks = (K + 15) / 16;
   ilb::pdl_launch_dependents();
-  fetch_w(0);                                        // (weights belong to no earlier kernel)
+  if (settled) fetch_w(0);
   ilb::pdl_wait();
+  if (!settled) fetch_w(0);
   fetch_a(0);
   commit();
   float acc = 0.f, lost = 0.f;                       // of output `lane` = r * T + t
@@ -380,7 +381,7 @@ gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 
 template <typename TO, int T, int R>
 static int launch_few(const float* A, const float* W, const float* bias, void* out, int M, int N, int K, int lda, int ldw,
-                      int ldo, int accumulate, cudaStream_t stream) {
+                      int ldo, int accumulate, int settled, cudaStream_t stream) {
   static ilb::OncePerDevice once;
   constexpr size_t smem = few_smem(T, R);
   if (once.first() && cudaFuncSetAttribute(gemm_simt_few_kernel<TO, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
@@ -388,7 +389,7 @@ static int launch_few(const float* A, const float* W, const float* bias, void* o
     return fail("gemm_simt: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(cudaGetLastError()));
   }
   ilb::launch(gemm_simt_few_kernel<TO, T, R>, dim3((unsigned)((N + kFewWarps * R - 1) / (kFewWarps * R) * ((M + T - 1) / T))), dim3(kFewWarps * 32), smem, stream,
-              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate);
+              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, settled);
   return check_launch("gemm_simt");
 }
 
@@ -412,7 +413,7 @@ constexpr int kWideM = 64, kWideN = 64, kWideK = 32;
 template <typename TA, typename TO>
 __global__ void __launch_bounds__(kWideM * kWideN / 32, 2)
 gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias, TO* __restrict__ out,
-                      int M, int N, int K, int lda, int ldw, int ldo, int accumulate) {
+                      int M, int N, int K, int lda, int ldw, int ldo, int accumulate, int settled) {
   constexpr int BM = kWideM, BN = kWideN, BK = kWideK;
   constexpr int WARPS = (BM / 32) * (BN / 32);
   constexpr int HALVES = BK / 8;                                   // pairs of pieces of a row
@@ -465,9 +466,9 @@ gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const 
     for (int j = 0; j < 4; ++j) acc[i][j] = lost[i][j] = 0;
   const uint64_t minus = pack2(-1.f, -1.f);
   ilb::pdl_launch_dependents();
-  fetch(0, true, false);                                           // (weights belong to no earlier kernel)
+  if (settled) fetch(0, true, false);
   ilb::pdl_wait();
-  fetch(0, false, true);
+  fetch(0, !settled, true);
   stash(0);
   __syncthreads();
   const int blocks = (K + BK - 1) / BK;
@@ -539,17 +540,17 @@ gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const 
 
 template <typename TA, typename TO>
 static int launch_wide(const TA* A, const TA* W, const float* bias, void* out, int M, int N, int K, int lda, int ldw, int ldo,
-                       int accumulate, cudaStream_t stream) {
+                       int accumulate, int settled, cudaStream_t stream) {
   const long long tiles = (long long)((M + kWideM - 1) / kWideM) * ((N + kWideN - 1) / kWideN);
   ILB_REQUIRE(tiles <= 2147483647LL, "gemm_simt: grid too large for M=%d N=%d", M, N);
   ilb::launch(gemm_simt_wide_kernel<TA, TO>, dim3((unsigned)tiles), dim3(kWideM * kWideN / 32), 0, stream,
-              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate);
+              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, settled);
   return check_launch("gemm_simt");
 }
 
 template <typename TA, typename TO>
 static int launch(const void* A, const void* W, const float* bias, void* out, int M, int N, int K,
-                  int lda, int ldw, int ldo, int accumulate, cudaStream_t stream,
+                  int lda, int ldw, int ldo, int accumulate, int settled, cudaStream_t stream,
                   const int* block_group = nullptr, long long group_stride = 0) {
   const bool pieces = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
                       (uintptr_t)A % (4 * sizeof(TA)) == 0 && (uintptr_t)W % (4 * sizeof(TA)) == 0;
@@ -561,10 +562,10 @@ static int launch(const void* A, const void* W, const float* bias, void* out, in
     if (pieces && !grouped && M <= 40) {
       const float* a = (const float*)A;
       const float* w = (const float*)W;
-      if (M == 1) return launch_few<TO, 1, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
-      if (M == 2) return launch_few<TO, 2, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
-      if (M <= 4) return launch_few<TO, 4, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
-      return launch_few<TO, 8, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
+      if (M == 1) return launch_few<TO, 1, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
+      if (M == 2) return launch_few<TO, 2, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
+      if (M <= 4) return launch_few<TO, 4, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
+      return launch_few<TO, 8, 4>(a, w, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
     }
   }
   if (pieces && (M <= 16 || grouped)) {
@@ -573,7 +574,7 @@ static int launch(const void* A, const void* W, const float* bias, void* out, in
     ilb::launch(gemm_simt_fast_kernel<TA, TO, BM, BN, TM, TN, 8>, dim3(grid), dim3((BM / TM) * (BN / TN)), 0, stream,
         (const TA*)A, (const TA*)W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, block_group, group_stride);
   } else if (pieces) {
-    return launch_wide<TA, TO>((const TA*)A, (const TA*)W, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
+    return launch_wide<TA, TO>((const TA*)A, (const TA*)W, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
   } else if (M <= 16 || grouped) {
     constexpr int BM = 16, BN = 32, TM = 2, TN = 2;
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
@@ -590,20 +591,22 @@ static int launch(const void* A, const void* W, const float* bias, void* out, in
 
 // in_dtype: element type of A and W; out_dtype: element type of out.
 // accumulate != 0 adds the product (and bias) to what `out` already holds.
+// `settled`: no launch that this one may overlap writes W: the kernels for 32-bit operands of few tokens and for many tokens ask
+// for its first rows ahead of the dependency wait (small products: 1.3 against 1.6 us launch after launch).
 ILB_EXPORT int ilb_gemm_simt(const void* A, const void* W, const float* bias, void* out,
                              int in_dtype, int out_dtype, int M, int N, int K, int lda, int ldw,
-                             int ldo, int accumulate, cudaStream_t stream) {
+                             int ldo, int accumulate, int settled, cudaStream_t stream) {
   ILB_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_simt: bad sizes M=%d N=%d K=%d", M, N, K);
   ILB_REQUIRE(lda >= K && ldw >= K && ldo >= N, "gemm_simt: leading dimensions too small");
   ILB_REQUIRE((long long)((N + 31) / 32) <= 2147483647LL && (M + 15) / 16 <= 65535,
               "gemm_simt: grid too large for M=%d", M);
   if (M == 0) return 0;
   if (in_dtype == kF32 && out_dtype == kF32)
-    return launch<float, float>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
+    return launch<float, float>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
   if (in_dtype == kBF16 && out_dtype == kF32)
-    return launch<__nv_bfloat16, float>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
+    return launch<__nv_bfloat16, float>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
   if (in_dtype == kBF16 && out_dtype == kBF16)
-    return launch<__nv_bfloat16, __nv_bfloat16>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
+    return launch<__nv_bfloat16, __nv_bfloat16>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
   return fail("gemm_simt: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
 }
 
@@ -622,11 +625,11 @@ ILB_EXPORT int ilb_gemm_simt_grouped(const void* A, const void* W, void* out, in
   ILB_REQUIRE(M % 16 == 0 && M / 16 <= 65535, "gemm_simt_grouped: rows must come in blocks of 16 (at most 65535 blocks), found M=%d", M);
   if (M == 0) return 0;
   if (in_dtype == kF32 && out_dtype == kF32)
-    return launch<float, float>(A, W, nullptr, out, M, N, K, lda, ldw, ldo, 0, stream, block_group, group_stride);
+    return launch<float, float>(A, W, nullptr, out, M, N, K, lda, ldw, ldo, 0, 0, stream, block_group, group_stride);
   if (in_dtype == kBF16 && out_dtype == kF32)
-    return launch<__nv_bfloat16, float>(A, W, nullptr, out, M, N, K, lda, ldw, ldo, 0, stream, block_group, group_stride);
+    return launch<__nv_bfloat16, float>(A, W, nullptr, out, M, N, K, lda, ldw, ldo, 0, 0, stream, block_group, group_stride);
   if (in_dtype == kBF16 && out_dtype == kBF16)
-    return launch<__nv_bfloat16, __nv_bfloat16>(A, W, nullptr, out, M, N, K, lda, ldw, ldo, 0, stream, block_group, group_stride);
+    return launch<__nv_bfloat16, __nv_bfloat16>(A, W, nullptr, out, M, N, K, lda, ldw, ldo, 0, 0, stream, block_group, group_stride);
   return fail("gemm_simt_grouped: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
 }
 

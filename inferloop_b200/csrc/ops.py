@@ -905,8 +905,9 @@ def decode_advance(tokens: torch.Tensor, positions: torch.Tensor, kv_len: torch.
 
 # --------------------------------------------------------------------------- GEMM
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
-              bias: Optional[torch.Tensor] = None, accumulate: bool = False) -> None:
-    """out (+)= a @ w.T (+ bias) with 32-bit fused multiply-adds in a fixed order."""
+              bias: Optional[torch.Tensor] = None, accumulate: bool = False, settled: bool = False) -> None:
+    """out (+)= a @ w.T (+ bias) with 32-bit fused multiply-adds in a fixed order.  `settled`: no launch still in flight writes
+    `w` (a bound weight): its first rows are asked for while the launch before is still running."""
     _need(a, "gemm a"); _need(w, "gemm w", a.dtype); _need(out, "gemm out")
     _need(bias, "gemm bias", torch.float32)
     M, K = a.shape
@@ -917,7 +918,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
         raise KernelError("gemm: accumulation needs a 32-bit output")
     _call("gemm_simt", "ilb_gemm_simt", _ptr(a), _ptr(w), _ptr(bias), _ptr(out), _i(_code(a)),
           _i(_code(out)), _i(M), _i(N), _i(K), _i(K), _i(K), _i(N), _i(1 if accumulate else 0),
-          _stream(out))
+          _i(1 if settled else 0), _stream(out))
 
 
 # --------------------------------------------------------------------------- attention

@@ -16,8 +16,9 @@ from ..csrc import ops
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor,
            bias: Optional[torch.Tensor] = None, accumulate: bool = False) -> None:
-    """out (+)= x @ weight.T (+ bias).  `accumulate` adds into a 32-bit `out`."""
+    """out (+)= x @ weight.T (+ bias).  `accumulate` adds into a 32-bit `out`.  `weight` is a bound one: no launch of the step
+    writes it (its first tiles are read while the launch before is still running)."""
     if x.dtype == torch.bfloat16 and ops.gemm_tc_eligible(x, weight, out):
         ops.gemm_tc(x, weight, out, bias, accumulate)
     else:
-        ops.gemm_simt(x, weight, out, bias, accumulate)
+        ops.gemm_simt(x, weight, out, bias, accumulate, settled=True)

@@ -173,6 +173,27 @@ def test_gemm_simt_many_tokens_agree_bit_for_bit(M, N, K, in_dtype):
     close(out, base.double() + a.double() @ w.double().T + b.double(), "float32", scale=float(K) ** 0.5 * 4, what="gemm")
 
 
+@pytest.mark.parametrize("M,in_dtype", [(1, torch.float32), (4, torch.float32), (8, torch.float32), (16, torch.bfloat16), (40, torch.float32),
+                                        (100, torch.float32), (100, torch.bfloat16)])
+def test_gemm_simt_takes_a_matrix_of_the_launch_before(M, in_dtype):
+    """The matrix is the result of the launch right before (a long product): launches overlap, the product is that of what it
+    leaves, whatever the buffer held."""
+    N, K, inner = 40, 520, 12288
+    torch.manual_seed(M)
+    a = torch.randn(M, K).to(in_dtype).cuda()
+    x, y = torch.randn(N, inner).to(in_dtype).cuda(), (torch.randn(K, inner) / inner ** 0.5).to(in_dtype).cuda()
+    w, out, want = torch.empty(N, K, dtype=in_dtype, device="cuda"), torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    ops().gemm_simt(x, y, w)
+    torch.cuda.synchronize()
+    ops().gemm_simt(a, w.clone(), want)
+    for _ in range(3):
+        w.zero_()
+        torch.cuda.synchronize()
+        ops().gemm_simt(x, y, w)
+        ops().gemm_simt(a, w, out)
+        assert torch.equal(out, want)
+
+
 # ------------------------------------------------------------------ attention pieces
 def build_cache(seqs_kv, nkv, d, page_size, num_pages, dtype, seed=0, page_order="shuffled"):
     """Scatter each sequence's keys/values into pages; returns cache tensors and the block
