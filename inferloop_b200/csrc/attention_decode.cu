@@ -1097,15 +1097,17 @@ inline size_t inbox_bytes(int d, int group, int split) { return (size_t)split * 
 template <int D, int DV, int STAGES, int V>
 int configure() {
   static OncePerDevice once;
-  if (once.first()) {
-    constexpr size_t smem = ring_bytes<D, DV, STAGES, V>() + (size_t)2 * kMaxSplit * (DV + 4) * 4;   // the most a launch asks for
-    static_assert(smem <= 227 * 1024, "tile ring does not fit shared memory");
-    cudaError_t e = cudaFuncSetAttribute(decode_kernel<D, DV, STAGES, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) once.forget();
-    if (e != cudaSuccess) return fail("attention decode: cannot reserve %zu bytes of shared memory", smem);
-    cudaFuncSetAttribute(decode_kernel<D, DV, STAGES, V>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(decode_kernel<D, DV, STAGES, V>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  }
+  constexpr size_t smem = ring_bytes<D, DV, STAGES, V>() + (size_t)2 * kMaxSplit * (DV + 4) * 4;   // the most a launch asks for
+  static_assert(smem <= 227 * 1024, "tile ring does not fit shared memory");
+  const cudaError_t e = once.run([] {
+    const cudaError_t e = cudaFuncSetAttribute(decode_kernel<D, DV, STAGES, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) {
+      cudaFuncSetAttribute(decode_kernel<D, DV, STAGES, V>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      cudaFuncSetAttribute(decode_kernel<D, DV, STAGES, V>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
+    return e;
+  });
+  if (e != cudaSuccess) return fail("attention decode: cannot reserve %zu bytes of shared memory", smem);
   return 0;
 }
 

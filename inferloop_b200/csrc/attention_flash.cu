@@ -526,11 +526,8 @@ template <int D>
 int launch_prefill(const PrefillParams& p, int n_tiles, cudaStream_t stream) {
   static OncePerDevice once;
   const size_t smem = prefill_smem<D>();
-  if (once.first()) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) once.forget();
-    if (e != cudaSuccess) return fail("attention prefill: cannot reserve %zu bytes of shared memory", smem);
-  }
+  if (once.run([&] { return cudaFuncSetAttribute(prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
+    return fail("attention prefill: cannot reserve %zu bytes of shared memory", smem);
   ilb::launch(prefill_kernel<D>, dim3(n_tiles, p.cache.nkv), dim3(kWarps * 32), smem, stream, p);
   return check_launch("attention prefill");
 }
@@ -539,11 +536,8 @@ template <int D>
 int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   static OncePerDevice once;
   const size_t smem = decode_smem<D>();
-  if (once.first()) {
-    cudaError_t e = cudaFuncSetAttribute(decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) once.forget();
-    if (e != cudaSuccess) return fail("attention decode: cannot reserve %zu bytes of shared memory", smem);
-  }
+  if (once.run([&] { return cudaFuncSetAttribute(decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
+    return fail("attention decode: cannot reserve %zu bytes of shared memory", smem);
   ilb::launch(decode_kernel<D>, dim3(p.cache.nkv, p.n_seqs, p.max_chunks), dim3(kWarps * 32), smem, stream, p);
   return check_launch("attention decode");
 }

@@ -182,11 +182,8 @@ ILB_EXPORT int ilb_attention_mix(
 #define ILB_LAUNCH(TQ, TC)                                                                                              \
   do {                                                                                                                  \
     static OncePerDevice once;                                                                                          \
-    if (once.first() && cudaFuncSetAttribute(attention_mix_kernel<TQ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                             200 * 1024) != cudaSuccess) {                                              \
-      once.forget();                                                                                                    \
+    if (once.run([] { return cudaFuncSetAttribute(attention_mix_kernel<TQ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); }) != cudaSuccess) \
       return fail("attention_mix: cannot set the shared memory size: %s", cudaGetErrorString(cudaGetLastError()));      \
-    }                                                                                                                   \
     ilb::launch(attention_mix_kernel<TQ, TC>, dim3(n_tokens), dim3(kMixThreads), smem, stream, (const TQ*)q, (TQ*)out,  \
                 (const TC*)k_cache, (const TC*)v_cache, a);                                                             \
   } while (0)
@@ -840,11 +837,8 @@ ILB_EXPORT int ilb_attention_mix_tc(
 #define ILB_HD(KT)                                                                                                        \
   do {                                                                                                                    \
     static OncePerDevice once;                                                                                            \
-    if (once.first() && cudaFuncSetAttribute(attention_mix_heads_kernel<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                             200 * 1024) != cudaSuccess) {                                                \
-      once.forget();                                                                                                      \
+    if (once.run([] { return cudaFuncSetAttribute(attention_mix_heads_kernel<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); }) != cudaSuccess) \
       return fail("attention_mix_tc: cannot set the shared memory size: %s", cudaGetErrorString(cudaGetLastError()));     \
-    }                                                                                                                     \
     ilb::launch(attention_mix_heads_kernel<KT>, dim3(n_seqs, max_chunks), dim3(kHdThreads),                               \
                 mix_heads_smem(nq, nkv, d, dv, KT), stream, a);                                                           \
   } while (0)
@@ -859,11 +853,8 @@ ILB_EXPORT int ilb_attention_mix_tc(
 #define ILB_TC(DV)                                                                                                        \
   do {                                                                                                                    \
     static OncePerDevice once;                                                                                            \
-    if (once.first() && cudaFuncSetAttribute(attention_mix_tc_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                             220 * 1024) != cudaSuccess) {                                                \
-      once.forget();                                                                                                      \
+    if (once.run([] { return cudaFuncSetAttribute(attention_mix_tc_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); }) != cudaSuccess) \
       return fail("attention_mix_tc: cannot set the shared memory size: %s", cudaGetErrorString(cudaGetLastError()));     \
-    }                                                                                                                     \
     ilb::launch(attention_mix_tc_kernel<DV>, grid, dim3(kTcThreads), smem, stream, a);                                    \
   } while (0)
   if (dv <= 64) ILB_TC(64); else ILB_TC(128);

@@ -613,11 +613,8 @@ int launch(const Maps& m, const Params& p, int n_tiles, cudaStream_t stream) {
                           (1 + 2 * kStagesK + 2 * kStagesV + 10 + 2) * 8 + (size_t)QB * 768 * 4;
   static_assert(smem <= 227 * 1024, "tiles do not fit shared memory");
   static OncePerDevice once;
-  if (once.first()) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<D, DV, QB, POOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) once.forget();
-    if (e != cudaSuccess) return fail("attention (tensor cores): cannot reserve %zu bytes of shared memory", smem);
-  }
+  if (once.run([&] { return cudaFuncSetAttribute(prefill_tc_kernel<D, DV, QB, POOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
+    return fail("attention (tensor cores): cannot reserve %zu bytes of shared memory", smem);
   ilb::launch(prefill_tc_kernel<D, DV, QB, POOL>, dim3(p.nkv, n_tiles), dim3(64 + 256 * QB), smem, stream, m.q, m.k, m.v, m.k_run, m.v_run,
               m.pk, m.pv, p);
   return check_launch("attention prefill (tensor cores)");

@@ -175,11 +175,8 @@ template <typename TI, int Q>
 static int scan_launch(const DeltaParams& p, cudaStream_t stream) {
   const size_t smem = sizeof(float) * scan_smem_floats(32 * Q);
   static OncePerDevice once;
-  if (smem > 48 * 1024 && once.first() &&
-      cudaFuncSetAttribute(delta_scan_kernel<TI, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    once.forget();
+  if (smem > 48 * 1024 && once.run([&] { return cudaFuncSetAttribute(delta_scan_kernel<TI, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
     return fail("delta_scan: cannot reserve %zu bytes of shared memory", smem);
-  }
   ilb::launch(delta_scan_kernel<TI, Q>, dim3(p.heads, (p.dv + kCols - 1) / kCols, p.n_seqs), dim3(kScanThreads), smem, stream, p);
   return check_launch("delta_scan");
 }
@@ -855,11 +852,8 @@ static int chunks_mma_launch(const DeltaParams& p, const float* scratch, int* er
   constexpr size_t smem = ChunksMma<KP, RING>::kSmem;
   static_assert(smem <= 227 * 1024, "the ring does not fit shared memory");
   static OncePerDevice once;
-  if (smem > 48 * 1024 && once.first() &&
-      cudaFuncSetAttribute(delta_chunks_mma_kernel<KP, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    once.forget();
+  if (smem > 48 * 1024 && once.run([&] { return cudaFuncSetAttribute(delta_chunks_mma_kernel<KP, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
     return fail("delta_chunks: cannot reserve %zu bytes of shared memory", smem);
-  }
   ilb::launch(delta_chunks_mma_kernel<KP, RING>, dim3(p.heads, padded_cols(p.dv) / kCols, p.n_seqs), dim3(KP * 2), smem, stream, p, scratch, error_flag);
   return check_launch("delta_chunks");
 }
@@ -874,10 +868,8 @@ template <int RH>
 static int chunks_launch(const DeltaParams& p, const float* scratch, cudaStream_t stream) {
   const size_t smem = sizeof(float) * chunks_smem_floats(16 * RH);
   static OncePerDevice once;
-  if (once.first() && cudaFuncSetAttribute(delta_chunks_kernel<RH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    once.forget();
+  if (once.run([&] { return cudaFuncSetAttribute(delta_chunks_kernel<RH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
     return fail("delta_chunks: cannot reserve %zu bytes of shared memory", smem);
-  }
   ilb::launch(delta_chunks_kernel<RH>, dim3(p.heads, padded_cols(p.dv) / kCols, p.n_seqs), dim3(kChunkThreads), smem, stream, p, scratch);
   return check_launch("delta_chunks");
 }
@@ -888,10 +880,8 @@ static int prep_launch(const DeltaParams& p, float* scratch, int n_blocks, cudaS
   const size_t smem = sizeof(float) * prep_smem_floats(KP, padded_cols(p.dv));
   ILB_REQUIRE(smem <= 200 * 1024, "delta_prep: states of %d x %d do not fit the block's shared memory", p.d, p.dv);
   static OncePerDevice once;
-  if (once.first() && cudaFuncSetAttribute(delta_prep_kernel<TI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) {
-    once.forget();
+  if (once.run([&] { return cudaFuncSetAttribute(delta_prep_kernel<TI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); }) != cudaSuccess)
     return fail("delta_prep: cannot reserve shared memory");
-  }
   ilb::launch(delta_prep_kernel<TI>, dim3(n_blocks, p.heads), dim3(kPrepThreads), smem, stream, p, scratch, KP);
   return check_launch("delta_prep");
 }

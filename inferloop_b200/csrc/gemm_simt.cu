@@ -384,10 +384,8 @@ static int launch_few(const float* A, const float* W, const float* bias, void* o
                       int ldo, int accumulate, int settled, cudaStream_t stream) {
   static ilb::OncePerDevice once;
   constexpr size_t smem = few_smem(T, R);
-  if (once.first() && cudaFuncSetAttribute(gemm_simt_few_kernel<TO, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    once.forget();
+  if (once.run([] { return cudaFuncSetAttribute(gemm_simt_few_kernel<TO, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
     return fail("gemm_simt: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(cudaGetLastError()));
-  }
   ilb::launch(gemm_simt_few_kernel<TO, T, R>, dim3((unsigned)((N + kFewWarps * R - 1) / (kFewWarps * R) * ((M + T - 1) / T))), dim3(kFewWarps * 32), smem, stream,
               A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, settled);
   return check_launch("gemm_simt");

@@ -1250,13 +1250,14 @@ int configure() {
   constexpr size_t smem = smem_bytes<BN, STAGES, SWAP, MS>();
   static_assert(smem <= 227 * 1024, "stage ring does not fit shared memory");
   static OncePerDevice once;
-  if (once.first()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, SWAP, MS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) once.forget();
-    if (e != cudaSuccess) return fail("gemm_tc: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+  const cudaError_t e = once.run([] {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, SWAP, MS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     // two CTAs of the small rings share an SM only with the largest shared-memory carve-out
-    cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, SWAP, MS>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  }
+    if (e == cudaSuccess)
+      cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, SWAP, MS>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e;
+  });
+  if (e != cudaSuccess) return fail("gemm_tc: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
   return 0;
 }
 
@@ -1581,10 +1582,8 @@ bool pair_wanted(const PairPlan& pp, int epilogue) {
 
 int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const CUtensorMap& mo, const PairParams& p, int n_pairs, cudaStream_t stream) {
   static OncePerDevice once;
-  if (once.first()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem);
-    if (e != cudaSuccess) { once.forget(); return fail("gemm_tc: cannot reserve %zu bytes of shared memory: %s", kPairSmem, cudaGetErrorString(e)); }
-  }
+  const cudaError_t e = once.run([] { return cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem); });
+  if (e != cudaSuccess) return fail("gemm_tc: cannot reserve %zu bytes of shared memory: %s", kPairSmem, cudaGetErrorString(e));
   ilb::launch_cluster(gemm_pair_kernel, dim3(2 * n_pairs), dim3(192), kPairSmem, stream, 2, mx, my, mo, p);
   return check_launch("gemm_tc");
 }

@@ -155,19 +155,15 @@ ILB_EXPORT int ilb_streams_read(const float* x, const float* a, const float* nor
   const size_t smem = (size_t)width * sizeof(float);
   static OncePerDevice once_f, once_b;
   if (out_dtype == kF32 || normed == nullptr) {
-    if (smem > 48 * 1024 && once_f.first() &&
-        cudaFuncSetAttribute(streams_read_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess) {
-      once_f.forget();
+    if (smem > 48 * 1024 &&
+        once_f.run([] { return cudaFuncSetAttribute(streams_read_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); }) != cudaSuccess)
       return fail("streams_read: cannot reserve shared memory");
-    }
     ilb::launch(streams_read_kernel<float>, dim3(n_tokens), dim3(threads), smem, stream, x, a, norm_weight, (float*)normed, u_out,
                 y_zero, width, streams, eps);
   } else if (out_dtype == kBF16) {
-    if (smem > 48 * 1024 && once_b.first() &&
-        cudaFuncSetAttribute(streams_read_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess) {
-      once_b.forget();
+    if (smem > 48 * 1024 &&
+        once_b.run([] { return cudaFuncSetAttribute(streams_read_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); }) != cudaSuccess)
       return fail("streams_read: cannot reserve shared memory");
-    }
     ilb::launch(streams_read_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(threads), smem, stream, x, a, norm_weight,
                 (__nv_bfloat16*)normed, u_out, y_zero, width, streams, eps);
   } else {

@@ -827,13 +827,11 @@ ILB_EXPORT int ilb_mlstm_chunks(const void* proj, int ld, int col_q, int col_k, 
   const int vec = ((uintptr_t)proj % 16 == 0 && ld % 8 == 0 && col_q % 8 == 0 && col_k % 8 == 0 && col_v % 8 == 0 && d % 8 == 0 && dv % 8 == 0) ? 1 : 0;
   const size_t sa = local_smem(d), sc = out_smem(d);
   static OncePerDevice once;
-  if (once.first()) {
-    if (cudaFuncSetAttribute(mlstm_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local_smem(kMaxRows)) != cudaSuccess ||
-        cudaFuncSetAttribute(mlstm_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem(kMaxRows)) != cudaSuccess) {
-      once.forget();
-      return fail("mlstm_chunks: cannot reserve shared memory");
-    }
-  }
+  if (once.run([] {
+        const cudaError_t e = cudaFuncSetAttribute(mlstm_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local_smem(kMaxRows));
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(mlstm_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem(kMaxRows));
+      }) != cudaSuccess)
+    return fail("mlstm_chunks: cannot reserve shared memory");
   const int tiles = (dv + kTileCols - 1) / kTileCols;
   ilb::launch(mlstm_local_kernel, dim3(n_chunks, heads, tiles), dim3(kChunkThreads), sa, stream, p, s, vec);
   if (int rc = check_launch("mlstm_local")) return rc;

@@ -398,11 +398,8 @@ template <int MS, int BN, int kStages>
 static int launch_tiles(const void* A, const void* W, const Params& p, int rows, int groups, int lda, cudaStream_t stream) {
   static OncePerDevice once;
   constexpr size_t smem = smem_bytes<MS, BN, kStages>();
-  if (once.first() &&
-      cudaFuncSetAttribute(moe_gemm_kernel<MS, BN, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    once.forget();
+  if (once.run([] { return cudaFuncSetAttribute(moe_gemm_kernel<MS, BN, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
     return fail("moe_gemm: cannot reserve %zu bytes of shared memory", smem);
-  }
   CUtensorMap ma, mw;
   if (make_map(&ma, A, rows, p.K, lda, kRows)) return -1;
   if (make_map(&mw, W, (long long)groups * p.N, p.K, p.K, BN)) return -1;
@@ -414,11 +411,8 @@ template <int BN, int kStages>
 static int launch_persistent(const void* A, const void* W, const Params& p, int rows, int groups, int lda, cudaStream_t stream) {
   static OncePerDevice once;
   constexpr size_t smem = smem_bytes<1, BN, kStages>() + 64;
-  if (once.first() &&
-      cudaFuncSetAttribute(moe_gemm_persistent_kernel<BN, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    once.forget();
+  if (once.run([] { return cudaFuncSetAttribute(moe_gemm_persistent_kernel<BN, kStages>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
     return fail("moe_gemm: cannot reserve %zu bytes of shared memory", smem);
-  }
   CUtensorMap ma, mw;
   if (make_map(&ma, A, rows, p.K, lda, kRows)) return -1;
   if (make_map(&mw, W, (long long)groups * p.N, p.K, p.K, BN)) return -1;

@@ -871,11 +871,10 @@ ILB_EXPORT int ilb_conv_rows_norm_cache(
 #define ILB_CR(T, V, MT, TT)                                                                                                        \
   do {                                                                                                                              \
     static OncePerDevice once;                                                                                                      \
-    if (smem > 48 * 1024 && once.first() &&                                                                                         \
-        cudaFuncSetAttribute(conv_rows_norm_kernel<T, V, MT, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) != cudaSuccess) { \
-      once.forget();                                                                                                                \
+    if (smem > 48 * 1024 && once.run([] {                                                                                           \
+          return cudaFuncSetAttribute(conv_rows_norm_kernel<T, V, MT, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);     \
+        }) != cudaSuccess)                                                                                                          \
       return fail("conv_rows_norm: cannot reserve %d bytes of shared memory", kMost);                                               \
-    }                                                                                                                               \
     ilb::launch(conv_rows_norm_kernel<T, V, MT, TT>, dim3(blocks), dim3(threads), smem, stream, (const T*)qkv, (T*)q_out, (T*)k_cache, \
                 (T*)v_cache, c);                                                                                                    \
   } while (0)

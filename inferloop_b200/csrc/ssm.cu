@@ -364,18 +364,15 @@ static int scan_launch(const ScanParams& p, int n_blocks, cudaStream_t stream) {
   const bool local = p.pass == kPassLocal;
   // several threads a column (a state of more than 64 rows) need more than the default 48 KB: ask once for the most
   static OncePerDevice once;
-  if (once.first()) {
-    const int most = (int)(sizeof(float) * scan_smem_floats(256, 4));
-    bool ok = true;
-    ok = ok && cudaFuncSetAttribute(ssm_scan_kernel<TI, 32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
-    ok = ok && cudaFuncSetAttribute(ssm_scan_kernel<TI, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
-    ok = ok && cudaFuncSetAttribute(ssm_scan_kernel<TI, 64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
-    ok = ok && cudaFuncSetAttribute(ssm_scan_kernel<TI, 64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
-    if (!ok) {
-      once.forget();
-      return fail("ssm_scan: cannot reserve %d bytes of shared memory", most);
-    }
-  }
+  const int most = (int)(sizeof(float) * scan_smem_floats(256, 4));
+  if (once.run([most] {
+        cudaError_t e = cudaFuncSetAttribute(ssm_scan_kernel<TI, 32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssm_scan_kernel<TI, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssm_scan_kernel<TI, 64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssm_scan_kernel<TI, 64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        return e;
+      }) != cudaSuccess)
+    return fail("ssm_scan: cannot reserve %d bytes of shared memory", most);
   if (NPER == 16) {
     if (local) ilb::launch(ssm_scan_kernel<TI, 16, true>, grid, block, smem, stream, p);
     else ilb::launch(ssm_scan_kernel<TI, 16, false>, grid, block, smem, stream, p);
