@@ -530,13 +530,14 @@ __device__ __forceinline__ void patch_new_key_variant(uint32_t ks, uint32_t vs, 
 template <int D, int kMode>
 __host__ __device__ constexpr int fresh_bytes() { return kMode == 0 ? 2 * D * 2 : 0; }
 
-// kMode: 0 the stock input stage (or none), 1 its variants, 2 pooled blocks before a window.
+// kMode: 0 the stock input stage (or none), 1 its variants, 2 pooled blocks before a window, 3 the same with five CTAs to an SM
+// where 2 has four (see `five_ctas_pay`).
 template <int D, int DV, int kStages, int kMode>
-__global__ void __launch_bounds__(kThreads, D == 64 ? 5 : 4)      // (the prologue's loads in flight would take twice the registers)
+__global__ void __launch_bounds__(kThreads, D == 64 || kMode == 3 ? 5 : 4)      // (the prologue's loads in flight would take twice the registers)
 decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
               const __grid_constant__ CUtensorMap map_k_run, const __grid_constant__ CUtensorMap map_v_run,
               const __grid_constant__ CUtensorMap map_pk, const __grid_constant__ CUtensorMap map_pv, const Params p) {
-  constexpr bool kVariant = kMode == 1, kPool = kMode == 2;
+  constexpr bool kVariant = kMode == 1, kPool = kMode >= 2;
   static_assert(kPool || D == DV, "values of another head size come with the pooled form");
   constexpr int kSlices = D / 64, kSlicesV = DV / 64;
   constexpr uint32_t kSlice = kKeys * 128;                 // bytes: one slice of one tensor of a tile
@@ -1192,6 +1193,36 @@ int launch_for(const CUtensorMap (&m)[6], Params& p, int long_context, long long
   return launch<D, DV, 3, V>(m, p, extra, stream);
 }
 
+// Pooled blocks, keys of 128 and values of 64: the kernel wants 164 registers, which leaves four CTAs to an SM; at 128 (five, with
+// 48 bytes spilled) a launch takes 2 to 9 % longer where nothing else changes.  Five pay where they
+//   - make room for clusters twice as wide, of up to four (143 to 175 pairs of a sequence and a kv head, 297 to 370; 32 / 8 heads,
+//     windows of 256, us with four / five: 19 x 547 keys 10.4 / 8.8, 40 x 824 18.3 / 12.0; clusters of 8 instead of 4 or 16
+//     instead of 8 gain nothing: 10 x 815 7.9 / 9.2, 24 / 2 heads, 18 x 700 7.1 / 10.4),
+//   - or give a crowded launch air.  The device holds the clusters that the occupancy calculator counts only when they come in a
+//     lucky order: from 86 % of them on, of 8 CTAs, from 93 % on, of 4 or 16, some wait for others to end (8 x 820 9.2 / 7.7, 4 x
+//     781 8.5 / 7.0, 17 x 723 10.2 / 8.7, 80 x 863 34.3 / 21.9, but 16 x 649 8.0 / 8.7, 64 x 921 19.7 / 21.5).  Where several
+//     clusters share a long sequence the crowd is what counts, whatever five do about it (1 x 40,000, blocks of 2: 26.5 / 20.2, 2
+//     x 17,000 23.7 / 18.8; 1 x 17,000, where half of the clusters have nothing to do, 17.4 / 18.1).
+bool crowded(int split, long long clusters, int room) {
+  return clusters * 100 > room * (split == 8 ? 86LL : split >= 4 ? 93LL : 100LL);
+}
+template <int V>
+int room_for(int nq, int nkv, int split, int stages) {
+  const size_t extra = inbox_bytes(64, nq / nkv, split);
+  return stages == 12 ? active_clusters<128, 64, 12, V>(split, extra) : stages == 6 ? active_clusters<128, 64, 6, V>(split, extra)
+                                                                                    : active_clusters<128, 64, 3, V>(split, extra);
+}
+bool five_ctas_pay(int n_seqs, int nq, int nkv, int long_context) {
+  int split4, split5, stages4, stages5, chunks4, chunks5;
+  plan_for<128, 64, 2>(n_seqs, nq, nkv, long_context, split4, stages4, chunks4);
+  plan_for<128, 64, 3>(n_seqs, nq, nkv, long_context, split5, stages5, chunks5);
+  const long long pairs = (long long)n_seqs * nkv;
+  const bool four_crowd = crowded(split4, pairs * chunks4, room_for<2>(nq, nkv, split4, stages4));
+  if (chunks4 > 1 || chunks5 > 1) return four_crowd;
+  if (split5 > split4 && split5 <= 4) return true;
+  return four_crowd && !crowded(split5, pairs, room_for<3>(nq, nkv, split5, stages5));
+}
+
 }  // namespace
 
 // Geometry this kernel is built for; everything else takes the ticketed kernel of attention_flash.
@@ -1207,6 +1238,17 @@ ILB_EXPORT int ilb_attention_decode_plan(int n_seqs, int nq, int nkv, int d, int
               "attention decode: no plan for this geometry");
   if (d == 64) plan_for<64>(n_seqs, nq, nkv, long_context, *split, *stages, *chunks);
   else plan_for<128>(n_seqs, nq, nkv, long_context, *split, *stages, *chunks);
+  return 0;
+}
+
+// The same for pooled blocks before a window, keys of 128 and values of 64, with the CTAs to an SM that its kernel is built for.
+ILB_EXPORT int ilb_attention_decode_pooled_plan(int n_seqs, int nq, int nkv, int page_size, int long_context, int* split, int* stages,
+                                                int* chunks, int* ctas) {
+  ILB_REQUIRE(ilb_attention_decode_tma_supported(nq, nkv, 128, page_size) && n_seqs > 0 && split && stages && chunks && ctas,
+              "attention decode: no plan for this geometry");
+  *ctas = five_ctas_pay(n_seqs, nq, nkv, long_context) ? 5 : 4;
+  if (*ctas == 5) plan_for<128, 64, 3>(n_seqs, nq, nkv, long_context, *split, *stages, *chunks);
+  else plan_for<128, 64, 2>(n_seqs, nq, nkv, long_context, *split, *stages, *chunks);
   return 0;
 }
 
@@ -1328,6 +1370,7 @@ ILB_EXPORT int ilb_attention_decode_pooled(const void* q, void* out, const void*
   p.chunks = 1; p.scratch = scratch; p.counters = counters;
   p.p_table = p_table; p.p_num_pages = p_num_pages; p.pool = pool; p.turn = (const float2*)turn;
   if (d == 64) return launch_for<64, 64, 2>(m, p, long_context, scratch_floats, n_counters, stream);
+  if (dv == 64 && five_ctas_pay(n_seqs, nq, nkv, long_context)) return launch_for<128, 64, 3>(m, p, long_context, scratch_floats, n_counters, stream);
   if (dv == 64) return launch_for<128, 64, 2>(m, p, long_context, scratch_floats, n_counters, stream);
   return launch_for<128, 128, 2>(m, p, long_context, scratch_floats, n_counters, stream);
 }

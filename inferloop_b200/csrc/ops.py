@@ -1430,6 +1430,17 @@ def attention_decode_plan(n_seqs: int, nq: int, nkv: int, d: int, page_size: int
     return split.value, stages.value, chunks.value
 
 
+def attention_pooled_decode_plan(n_seqs: int, nq: int, nkv: int, page_size: int, long_context: bool = False) -> tuple:
+    """(CTAs of a cluster, stages, clusters that may share a sequence, CTAs to an SM) of single tokens over a window and pooled
+    blocks, keys of 128 and values of 64."""
+    lib = load_module("attention_decode")
+    found = [ctypes.c_int(0) for _ in range(4)]
+    lib.ilb_attention_decode_pooled_plan.restype = ctypes.c_int
+    if lib.ilb_attention_decode_pooled_plan(_i(n_seqs), _i(nq), _i(nkv), _i(page_size), _i(1 if long_context else 0), *map(ctypes.byref, found)) != 0:
+        raise KernelError(lib.ilb_last_error().decode())
+    return tuple(f.value for f in found)
+
+
 def attention_decode_tma(q, out, k_cache, v_cache, positions, cu_q, block_table, window, scale, n_seqs,
                          nq, nkv, d, long_context: bool = False) -> None:
     """Split-KV decode whose tiles come by TMA and whose partial results meet inside a

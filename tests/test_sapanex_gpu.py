@@ -612,6 +612,22 @@ def test_attention_over_a_window_and_pooled_blocks(nq, nkv, d, dv, size, pool, p
             ops.TC_ATTENTION_ENABLED = True
 
 
+@pytest.mark.parametrize("nq,nkv,n,split,ctas", [(32, 8, 4, 16, 5), (32, 8, 8, 8, 5), (32, 8, 10, 4, 4), (32, 8, 19, 4, 5), (32, 8, 40, 2, 5), (32, 8, 64, 1, 4),
+                                                  (32, 8, 80, 1, 5), (24, 2, 19, 8, 4), (68, 4, 90, 2, 5), (16, 8, 30, 2, 4)])
+def test_pooled_blocks_for_many_single_tokens(nq, nkv, n, split, ctas):
+    """Keys of 128 and values of 64: the form with five CTAs to an SM where it makes room for wider clusters or gives a crowded
+    launch air (groups of 17 heads too, which run in passes), the one with four elsewhere, each against the plain result."""
+    from inferloop_b200.csrc import ops
+    found = ops.attention_pooled_decode_plan(n, nq, nkv, 16)
+    assert (found[0], found[3]) == (split, ctas), found
+    size, pool, starts = 40, 4, [(37 * i) % 180 for i in range(n)]
+    case = pooled_case(nq, nkv, 128, 64, size, pool, 16, [1] * n, starts, torch.bfloat16, nq + n)
+    ref = case[-1]
+    out = run_pooled(case, [1] * n, starts, nq, nkv, 128, 64, size)
+    err = (out - ref).abs().max()
+    assert err <= 1.2e-2 * float(ref.abs().max()), f"{float(err):.3e} of {float(ref.abs().max()):.3e}"
+
+
 @pytest.mark.parametrize("size,pool", [(50, 8), (20, 3), (1, 1)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_every_edge_of_a_window_and_of_a_block(size, pool, dtype):
