@@ -100,9 +100,10 @@ gemm_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W,
 
 // The same sums, faster: operands come in 16-byte pieces (four consecutive k of a row), the
 // next PF K blocks are already in registers (or on their way) while one is multiplied, and
-// shared memory is double-buffered (one barrier per block of 16): up to 16 rows of bfloat16, and
-// rows dealt to groups.  The order of the sums forbids cutting K among CTAs, so the bytes in
-// flight are all the parallelism there is: eight blocks ahead.  A thread's rows and columns are strided
+// shared memory is double-buffered (one barrier per block of 16).  Two shapes: 16 x 64 for up to 16 rows of
+// bfloat16 and rows dealt to groups (the order of the sums forbids cutting K among CTAs, so the bytes in
+// flight are all the parallelism there is: eight blocks ahead), and 128 x 128 where `big_tiles`
+// says so.  A thread's rows and columns are strided
 // (row ty + i * BM/TM, column tx + j * BN/TN), so a warp reads consecutive words.  Every output is
 // still the same chains of 16 and the same compensated sum in k order as in the kernel above:
 // bit for bit the same result (a zero-padded tail adds +0 to a chain).  Needs K and the leading
@@ -546,6 +547,22 @@ static int launch_wide(const TA* A, const TA* W, const float* bias, void* out, i
   return check_launch("gemm_simt");
 }
 
+// Whether many tokens take 128 x 128 tiles (the kernel of 8 x 8 outputs a thread, a CTA to an SM) and not the 64 x 64 ones above
+// (two to an SM).  Both are bound by the 32-bit pipes, so the time is the rounds a launch takes: counted in rounds of the small
+// tiles (372 us at K = 4,096), a round of big ones takes 1.957 with 32-bit operands and 1.9 with bfloat16, 0.06 more once for
+// its fill, and a last round with one small tile to an SM at most takes 0.6.  Measured, big / small tiles, us: bfloat16 512 x
+// 4,096 x 4,096 735 / 762, 1,024 x 4,096 1,425 / 1,334, 1,024 x 24,576 7,614 / 7,818, 2,048 x 24,576 14,872 / 15,574, 200 x 6,144
+// 729 / 582; 32 bits 512 x 4,096 759 / 760, 1,024 x 4,096 1,473 / 1,333, 2,048 x 6,144 4,314 / 3,958, 2,048 x 24,576 15,297 / 15,643.
+constexpr int kSms = 148;
+static bool big_tiles(int M, int N, bool wide_operands) {
+  const long long small = (long long)((M + kWideM - 1) / kWideM) * ((N + kWideN - 1) / kWideN);
+  const long long big = (long long)((M + 127) / 128) * ((N + 127) / 128);
+  const long long rest = small % (2 * kSms);
+  const long long t_small = small / (2 * kSms) * 1000 + (rest == 0 ? 0 : rest <= kSms ? 600 : 1000);
+  const long long t_big = (big + kSms - 1) / kSms * (wide_operands ? 1957 : 1900) + 60;
+  return t_big < t_small;
+}
+
 template <typename TA, typename TO>
 static int launch(const void* A, const void* W, const float* bias, void* out, int M, int N, int K,
                   int lda, int ldw, int ldo, int accumulate, int settled, cudaStream_t stream,
@@ -570,6 +587,11 @@ static int launch(const void* A, const void* W, const float* bias, void* out, in
     constexpr int BM = 16, BN = 64, TM = 4, TN = 2;            // 4 warps, one per group of rows ty, ty + 4, ty + 8, ty + 12
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     ilb::launch(gemm_simt_fast_kernel<TA, TO, BM, BN, TM, TN, 8>, dim3(grid), dim3((BM / TM) * (BN / TN)), 0, stream,
+        (const TA*)A, (const TA*)W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, block_group, group_stride);
+  } else if (pieces && big_tiles(M, N, sizeof(TA) == 4)) {
+    constexpr int BM = 128, BN = 128, TM = 8, TN = 8;
+    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+    ilb::launch(gemm_simt_fast_kernel<TA, TO, BM, BN, TM, TN, 2>, dim3(grid), dim3((BM / TM) * (BN / TN)), 0, stream,
         (const TA*)A, (const TA*)W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, block_group, group_stride);
   } else if (pieces) {
     return launch_wide<TA, TO>((const TA*)A, (const TA*)W, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
@@ -607,6 +629,9 @@ ILB_EXPORT int ilb_gemm_simt(const void* A, const void* W, const float* bias, vo
     return launch<__nv_bfloat16, __nv_bfloat16>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, settled, stream);
   return fail("gemm_simt: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
 }
+
+// Rows and columns of a tile of the kernel that a product of many tokens on 16-byte (bfloat16: 8-byte) boundaries takes, 64 or 128 (for tests and notes).
+ILB_EXPORT int ilb_gemm_simt_tile(int M, int N, int in_dtype) { return big_tiles(M, N, in_dtype == kF32) ? 128 : kWideM; }
 
 // The same product for rows that are dealt to groups in blocks of 16 (ilb_gemm_simt_group_rows):
 // block b of A (rows 16 b .. 16 b + 15) is multiplied by the matrix W + block_group[b] *

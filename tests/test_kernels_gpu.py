@@ -173,6 +173,23 @@ def test_gemm_simt_many_tokens_agree_bit_for_bit(M, N, K, in_dtype):
     close(out, base.double() + a.double() @ w.double().T + b.double(), "float32", scale=float(K) ** 0.5 * 4, what="gemm")
 
 
+@pytest.mark.parametrize("M,N,K,in_dtype", [(500, 4001, 36, torch.bfloat16), (1000, 4700, 20, torch.bfloat16), (1000, 4700, 20, torch.float32)])
+def test_gemm_simt_big_tiles_agree_bit_for_bit(M, N, K, in_dtype):
+    """Where 128 x 128 tiles are the faster ones, with a bias and a sum into the output, the last row and column tiles partly
+    empty: the same bits as the kernel that reads element by element."""
+    from inferloop_b200.csrc.build import load_module
+    assert load_module("gemm_simt").ilb_gemm_simt_tile(M, N, 0 if in_dtype == torch.float32 else 1) == 128
+    torch.manual_seed(M + K)
+    a, w = torch.randn(M, K).to(in_dtype).cuda(), torch.randn(N, K).to(in_dtype).cuda()
+    b, base = torch.randn(N).cuda(), torch.randn(M, N).cuda()
+    out, out2 = base.clone(), base.clone()
+    ops().gemm_simt(a, w, out, b, True)
+    shifted_a = torch.empty(M * K + 1, device="cuda", dtype=in_dtype)[1:].view(M, K)      # one element past a boundary of the wide loads
+    shifted_a.copy_(a)
+    ops().gemm_simt(shifted_a, w, out2, b, True)
+    assert torch.equal(out, out2)
+
+
 @pytest.mark.parametrize("M,in_dtype", [(1, torch.float32), (4, torch.float32), (8, torch.float32), (16, torch.bfloat16), (40, torch.float32),
                                         (100, torch.float32), (100, torch.bfloat16)])
 def test_gemm_simt_takes_a_matrix_of_the_launch_before(M, in_dtype):
