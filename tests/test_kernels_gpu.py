@@ -748,6 +748,44 @@ def test_decode_attention_of_more_sequences_than_ctas(nq, nkv, d, page_size, win
     run_fused_decode(nq, nkv, d, page_size, window, True, True, lens, key_ulp=True)
 
 
+MANY_LENS = [1, 2, 15, 16, 17, 31, 32, 33, 48, 49, 64, 65, 97, 100, 129, 200] * 3
+
+
+@pytest.mark.parametrize("mode,part,mix", [(1, 1, None), (1 | 2 | 4, 2, None), (2, 1, None), (0, 1, "keep"), (0, 1, "mix")])
+@pytest.mark.parametrize("nq,nkv,d,page_size,window", [(16, 16, 128, 16, 0), (144, 16, 64, 16, 40)])
+def test_variants_of_the_input_stage_for_more_sequences_than_ctas(nq, nkv, d, page_size, window, mode, part, mix):
+    """A CTA per (sequence, kv head) behind each variant of the input stage: pairs of neighbours over all of the head or a part,
+    the norm behind the rotation, no norm weights, values kept or mixed."""
+    assert ops().attention_decode_plan(len(MANY_LENS), nq, nkv, d, page_size)[0] == 1
+    run_fused_decode(nq, nkv, d, page_size, window, True, True, MANY_LENS, key_ulp=True, mode=mode, rd=d // part, mix=mix)
+
+
+@pytest.mark.parametrize("nq,nkv,d,window", [(16, 16, 128, 0), (32, 16, 64, 40), (144, 16, 128, 0)])
+def test_ready_queries_for_more_sequences_than_ctas(nq, nkv, d, window):
+    """The same without the input stage (the step's keys in the cache already), and the same bits into an output that starts off
+    a 4-byte boundary, which is written an element at a time."""
+    o = ops()
+    torch.manual_seed(nq + d)
+    S = len(MANY_LENS)
+    assert o.attention_decode_plan(S, nq, nkv, d, 16)[0] == 1
+    seqs = [(torch.randn(n, nkv, d).bfloat16().double(), torch.randn(n, nkv, d).bfloat16().double()) for n in MANY_LENS]
+    k_cache, v_cache, table = build_cache(seqs, nkv, d, 16, sum(-(-n // 16) for n in MANY_LENS) + 3, torch.bfloat16)
+    q = torch.randn(S, nq * d).bfloat16()
+    positions, cu = torch.tensor([n - 1 for n in MANY_LENS], dtype=torch.int32).cuda(), torch.arange(S + 1, dtype=torch.int32).cuda()
+    outs = []
+    for shift in (0, 1):
+        out = torch.full((S * nq * d + 2,), float("nan"), dtype=torch.bfloat16, device="cuda")
+        view = out[shift:shift + S * nq * d].view(S, nq * d)
+        assert view.data_ptr() % 4 == 2 * shift
+        o.attention_decode_tma(q.cuda(), view, k_cache.cuda(), v_cache.cuda(), positions, cu, table.cuda(), window, d ** -0.5, S, nq, nkv, d)
+        o.check_device_errors()
+        assert torch.isnan(out[:shift]).all() and torch.isnan(out[shift + S * nq * d:]).all()      # nothing beside it
+        outs.append(view)
+    assert torch.equal(outs[0], outs[1])
+    ref = torch.stack([ref_attention(q[s].double().view(nq, d), *seqs[s], MANY_LENS[s] - 1, window).reshape(-1) for s in range(S)])
+    close_flash(outs[0], ref, max(float(v.abs().max()) for _, v in seqs), "decode with a CTA per sequence")
+
+
 def norm_weight_case(d, mode, seed):
     """A few sequences and `run(q_weight, k_weight, **options)`, which answers the output and both caches."""
     o = ops()
@@ -820,8 +858,10 @@ def test_decode_attention_of_few_long_sequences(lens, window):
     assert int(_tc_state(torch.device("cuda", 0)).attn_counters.abs().sum()) == 0       # tickets are back at zero
 
 
-def run_fused_decode(nq, nkv, d, page_size, window, use_norm, use_rope, lens, long_context=False, key_ulp=False):
+def run_fused_decode(nq, nkv, d, page_size, window, use_norm, use_rope, lens, long_context=False, key_ulp=False, mode=0, rd=None, mix=None):
+    """`mode`, `rd`: the input stage's variants; `mix`: "keep" or "mix" the values with those of a first layer."""
     o = ops()
+    rd = d if rd is None else rd
     torch.manual_seed(nq + d + page_size)
     eps, theta = 1e-6, 1e4
     S = len(lens)
@@ -830,25 +870,39 @@ def run_fused_decode(nq, nkv, d, page_size, window, use_norm, use_rope, lens, lo
     qkv = torch.randn(S, (nq + 2 * nkv) * d).to(torch.bfloat16)
     qw, kw = (1 + 0.1 * torch.randn(d)).float(), (1 + 0.1 * torch.randn(d)).float()
     positions = torch.tensor([n - 1 for n in lens], dtype=torch.int32)
-    inv = torch.tensor([theta ** (-(2.0 * i) / d) for i in range(d // 2)], dtype=torch.float64)
-    table = torch.empty(S, d // 2, 2, device="cuda")
+    inv = torch.tensor([theta ** (-(2.0 * i) / rd) for i in range(rd // 2)], dtype=torch.float64)
+    table = torch.empty(S, rd // 2, 2, device="cuda")
     o.rope_table(positions.cuda(), inv.cuda(), table)
+    weights = use_norm and not mode & o.NORM_UNWEIGHTED
 
     def norm(t, w):
-        return t / torch.sqrt((t * t).mean(-1, keepdim=True) + eps) * w.double() if use_norm else t
+        return t / torch.sqrt((t * t).mean(-1, keepdim=True) + eps) * (w.double() if weights else 1.0) if use_norm else t
 
     def rope(t, pos):
         if not use_rope:
             return t
         ang = pos.double()[:, None] * inv[None, :]
         c, s_ = torch.cos(ang)[:, None, :], torch.sin(ang)[:, None, :]
+        if mode & o.ROPE_INTERLEAVED:
+            a, b = t[..., 0:rd:2], t[..., 1:rd:2]
+            return torch.cat([torch.stack([a * c - b * s_, a * s_ + b * c], dim=-1).flatten(-2), t[..., rd:]], dim=-1)
         a, b = t[..., :d // 2], t[..., d // 2:]
         return torch.cat([a * c - b * s_, a * s_ + b * c], dim=-1)
 
+    def ready(t, w):
+        t = norm(rope(t, positions), w) if mode & o.NORM_AFTER_ROTATION else rope(norm(t, w), positions)
+        return t.to(torch.bfloat16).double()
+
     x = qkv.double()
-    q_new = rope(norm(x[:, :nq * d].view(S, nq, d), qw), positions).to(torch.bfloat16).double()
-    k_new = rope(norm(x[:, nq * d:(nq + nkv) * d].view(S, nkv, d), kw), positions).to(torch.bfloat16).double()
+    q_new = ready(x[:, :nq * d].view(S, nq, d), qw)
+    k_new = ready(x[:, nq * d:(nq + nkv) * d].view(S, nkv, d), kw)
     v_new = x[:, (nq + nkv) * d:].view(S, nkv, d)
+    options = dict(mode=mode, rotary_dim=rd)
+    if mix is not None:
+        v_first, lam = torch.randn(S, nkv * d).to(torch.bfloat16), torch.tensor([0.375])
+        options.update(v_first=v_first.cuda(), **({"v_keep": True} if mix == "keep" else {"v_lambda": lam.cuda()}))
+        if mix == "mix":
+            v_new = ((1 - 0.375) * v_new + 0.375 * v_first.double().view(S, nkv, d)).to(torch.bfloat16).double()
     # the cache holds the old keys; the slot of the new position holds something else
     padded = [(torch.cat([k, torch.full((1, nkv, d), 5.0, dtype=torch.float64)]), torch.cat([v, torch.full((1, nkv, d), -3.0, dtype=torch.float64)]))
               for k, v in old]
@@ -858,16 +912,22 @@ def run_fused_decode(nq, nkv, d, page_size, window, use_norm, use_rope, lens, lo
     out = torch.full((S, nq * d), float("nan"), dtype=torch.bfloat16, device="cuda")
     cu = torch.arange(S + 1, dtype=torch.int32).cuda()
     for _ in range(2):                       # the second run finds the new key already in the cache: same answer
-        o.attention_decode_fused(qkv.cuda(), out, qw.cuda() if use_norm else None, kw.cuda() if use_norm else None, eps,
+        o.attention_decode_fused(qkv.cuda(), out, qw.cuda() if weights else None, kw.cuda() if weights else None, eps,
                                  table if use_rope else None, k_cache, v_cache, True, positions.cuda(), cu, btable.cuda(),
-                                 window, 1.0 / math.sqrt(d), S, nq, nkv, d, long_context=long_context)
+                                 window, 1.0 / math.sqrt(d), S, nq, nkv, d, long_context=long_context, **options)
     o.check_device_errors()
     ref = torch.stack([ref_attention(q_new[s], torch.cat([old[s][0], k_new[s:s + 1]]), torch.cat([old[s][1], v_new[s:s + 1]]),
                                      lens[s] - 1, window).reshape(-1) for s in range(S)])
     close_flash(out, ref, max(float(v.abs().max()) for _, v in padded), "decode with input stage")
     for s, n in enumerate(lens):             # the new key and value are in the cache now, exactly as the separate kernel rounds them
         page, slot = int(btable[s, (n - 1) // page_size]), (n - 1) % page_size
-        assert torch.equal(v_cache[page, :, slot].cpu().double(), v_new[s])
+        got_v = v_cache[page, :, slot].cpu().double()
+        if mix == "mix":       # (products of 12 bits and their sum round to 32 bits before bfloat16: the same value, or a tie's neighbour)
+            assert ((got_v - v_new[s]).abs() <= 2.0 ** -7 * v_new[s].abs() + 2.0 ** -20).all()
+        else:
+            assert torch.equal(got_v, v_new[s])
+        if mix == "keep":
+            assert torch.equal(options["v_first"][s].cpu().double().view(nkv, d), v_new[s])
         if key_ulp:
             # both are bfloat16 roundings of values at most a few 2^-24 of the largest apart, so they are the same or
             # neighbours: at most 2^-7 of the value (among 100,000 keys some lie on a tie)
