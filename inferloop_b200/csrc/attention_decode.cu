@@ -32,16 +32,14 @@
 //            and patches them into the tile in shared memory.  The producer warp then reads
 //            nothing that the preceding kernel writes and starts its stream before the
 //            dependency wait.
-// Bound: the bytes of the cache behind about 6 us of a chain that no byte hides (dependency wait, projection row, norm, the first
-// tile, the two merges).  What was in that chain and need not be: positions read after the wait, norm weights missing L1, the
-// new key made inside its tile, one warp merging for two, a thread walking the records of every element of a row, and the
-// cluster form of the merge with nobody to meet.  Launch after launch, 32 / 8 heads: 1 x 1,030 keys 9.3 -> 6.8 us, 8 x about 770
-// 13.5 -> 11.4, 64 x about 770 46.5 -> 40.9 (31 of bytes); 40 / 8 heads, 19 x about 520: 19.4 -> 16.1; 64 / 8 heads, 2 x about
-// 4,500: 18.8 -> 16.5.
 //   pooled   (kMode 2) a window with pooled blocks before it: the tiles of a second set of pages (row b =
 //            the mean of block b of `pool` positions) come first in the deal, then the window's;
 //            values may have another head size (DV) than keys, q comes ready, and with `turn` the
 //            merged row is turned back in pairs (i, i + DV / 2) as it is written.
+// Bound: the bytes of the cache behind a chain that no byte hides (dependency wait, projection row, norm, the first tile, the two
+// merges): 6 us at 1 x 1,030 keys of 32 / 8 heads (6.7 in all; 9.1 before positions were read and settled norm weights touched
+// ahead of the wait, the new key made ahead of its tile, and the merges dealt to both warps and a warp a row), 10 us at 64 x 770
+// (41 in all, 46 before).  Further shapes: the table of the profile of this kernel.
 // Every mbarrier wait is bounded; on expiry a flag is raised and the CTA leaves (or, in the
 // form with cluster barriers, still walks to them), so nobody is left waiting.  No multicast.
 //

@@ -258,9 +258,10 @@ gemm_simt_fast_kernel(const TA* __restrict__ A, const TA* __restrict__ W,
 // K is a serial chain of barriers for one 64-column CTA; here the blocks of 16 k of one row go to the 32 lanes of a warp
 // (lane l chains block l of 512 consecutive k), and the block sums then pass through shared memory to one lane per output,
 // which adds them in k order with the same compensated sum: bit for bit the results above.  A warp has R rows of W, so a
-// piece of A read from shared memory serves R products.  Operands come by cp.async, whole lines at a time, two stages of 512
-// k; blocks of 16 floats lie 20 floats apart, so eight lanes' 16-byte reads (one block each) touch all 32 banks once.
-// Measured (4 layers of the 8B sizes with the output matrix, 4 tokens, one decode step): 7.14 -> 2.01 ms, of which the weights
+// piece of A read from shared memory serves R products.  Operands come by cp.async, whole lines at a time, 512 k a stage, one
+// stage ahead of the one that is multiplied (two buffers); blocks of 16 floats lie 20 floats apart, so eight lanes' 16-byte reads
+// (one block each) touch all 32 banks once.
+// Measured (4 layers of the 8B sizes with the output matrix, 4 tokens, one decode step): 7.3 -> 1.9 ms, of which the weights
 // alone take 0.85 ms at the measured copy rate.
 constexpr int kFewK = 512;                           // k of a stage: a block of 16 for every lane
 constexpr int kFewPitch = 20;                        // floats from one block of 16 to the next in shared memory
@@ -395,13 +396,15 @@ static int launch_few(const float* A, const float* W, const float* bias, void* o
 // The same sums for many tokens.  Bound: the 32-bit pipes (per output and block of 16 k: 16 multiply-adds and 7 operations of the
 // compensated sum).  A warp has a 32 x 32 tile and a lane 8 x 4 of it, rows in fours: three 16-byte reads of shared memory for 32
 // products.  Two rows go through one packed instruction (fma.rn.f32x2: each half rounds as fmaf does; a - b is fma(b, -1, a), one
-// rounding like __fsub_rn), at the same rate of the pipes and half the instructions to issue.  Operands come in 16-byte pieces, 32 k
-// ahead in registers, 16 rows x 2 pieces a warp and request (whole sectors; rows of k lie 4 floats beyond a multiple of 32, so
-// the transposed stores take different banks).  Row tiles of the same columns are neighbours in the grid: a weight tile comes from
-// memory once.  One layer's products of the 8B sizes, against 128 x 128 tiles of 8 x 8 (256 threads, the chains as separate
-// instructions, 64 to 128 CTAs for 4,096 columns): 64 tokens 5.03 -> 1.64 ms, 128: 5.15 -> 2.72, 200: 5.86 -> 3.98, 512: 8.74 ->
-// 8.00, 1,024: 15.9 -> 15.1.  Measured and dropped: separate instructions here (200 tokens 4.77), three blocks an SM at 168
-// registers (4.58: the reads are no longer a step ahead), 8 x 8 a lane with 4-byte cp.async (4.59; 512 tokens 6.87).
+// rounding like __fsub_rn), at the same rate of the pipes and half the instructions to issue.  Operands come in pieces of four k
+// (16 bytes, of bfloat16 8), 32 k ahead in registers, 16 rows x 2 pieces a warp and request (whole sectors of 32-bit operands, half
+// ones of bfloat16; rows of k lie 4 floats beyond a multiple of 32, so the transposed stores take different banks).  Row tiles of
+// the same columns are neighbours in the grid: a weight tile comes from memory once.  One layer's products of the 8B sizes in 32
+// bits, against 128 x 128 tiles of 8 x 8 (256 threads, the chains as separate instructions; for 4,096 columns 32 CTAs up to 128
+// tokens, 64 at 200, 128 at 512, 256 at 1,024): 64 tokens 5.03 -> 1.64 ms, 128: 5.15 -> 2.72, 200: 5.86 -> 3.98, 512: 8.74 -> 8.00,
+// 1,024: 15.9 -> 15.1; bfloat16, 4,096 x 4,096: 64 tokens 0.696 -> 0.313 ms, 200: 0.721 -> 0.386, 1,024: 1.43 -> 1.33 (where the
+// large tiles stay ahead: `big_tiles`).  Measured and dropped: separate instructions here (200 tokens 4.77), three blocks an SM at
+// 168 registers (4.58: the reads are no longer a step ahead), 8 x 8 a lane with 4-byte cp.async (4.59; 512 tokens 6.87).
 __device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
 __device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
@@ -479,32 +482,32 @@ gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const 
       for (int h = 0; h < BK; h += 16) {
         uint64_t part[4][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) part[i][j] = 0;
+          for (int j = 0; j < 4; ++j) part[i][j] = 0;
 #pragma unroll
-      for (int kk = 0; kk < 16; ++kk) {
-        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[buf][h + kk][r0]);
-        const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[buf][h + kk][r0 + 16]);
-        const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][h + kk][c0]);
-        const uint64_t a[4] = {a0.x, a0.y, a1.x, a1.y};
-        const uint64_t w[4] = {pack2(w4.x, w4.x), pack2(w4.y, w4.y), pack2(w4.z, w4.z), pack2(w4.w, w4.w)};
+        for (int kk = 0; kk < 16; ++kk) {
+          const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[buf][h + kk][r0]);
+          const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[buf][h + kk][r0 + 16]);
+          const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][h + kk][c0]);
+          const uint64_t a[4] = {a0.x, a0.y, a1.x, a1.y};
+          const uint64_t w[4] = {pack2(w4.x, w4.x), pack2(w4.y, w4.y), pack2(w4.z, w4.z), pack2(w4.w, w4.w)};
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[i][j] = fma2(a[i], w[j], part[i][j]);
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) part[i][j] = fma2(a[i], w[j], part[i][j]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint64_t s = add2(acc[i][j], part[i][j]);
-          const uint64_t bp = fma2(acc[i][j], minus, s);           // s - acc
-          const uint64_t ea = fma2(fma2(bp, minus, s), minus, acc[i][j]);
-          const uint64_t eb = fma2(bp, minus, part[i][j]);
-          lost[i][j] = add2(lost[i][j], add2(ea, eb));
-          acc[i][j] = s;
-        }
+          for (int j = 0; j < 4; ++j) {
+            const uint64_t s = add2(acc[i][j], part[i][j]);
+            const uint64_t bp = fma2(acc[i][j], minus, s);           // s - acc
+            const uint64_t ea = fma2(fma2(bp, minus, s), minus, acc[i][j]);
+            const uint64_t eb = fma2(bp, minus, part[i][j]);
+            lost[i][j] = add2(lost[i][j], add2(ea, eb));
+            acc[i][j] = s;
+          }
       }
     }
     if (b + 1 < blocks) stash(buf ^ 1);                            // (read last before the barrier at the end of block b - 1)
@@ -573,7 +576,8 @@ static int launch(const void* A, const void* W, const float* bias, void* out, in
   if constexpr (std::is_same<TA, float>::value) {
     // 16-byte pieces for cp.async; a lane adds up one output, so rows a warp x tokens <= 32.  The arithmetic grows with every
     // group of 8 tokens: one layer of the 8B sizes, this kernel against the tiles below: 24 tokens 0.86 / 1.31 ms, 40 tokens
-    // 1.42 / 1.56, 64 tokens 2.27 / 1.64.
+    // 1.42 / 1.56, 64 tokens 2.27 / 1.64.  That is the line at layers of that width; the wider an output, the earlier the tiles
+    // win (40 tokens here / 41 there, us: 24,576 x 4,096 663 / 522, 6,144 x 4,096 169 / 313, 1,024 x 4,096 39 / 199, 8 x 4,096 11 / 174).
     if (pieces && !grouped && M <= 40) {
       const float* a = (const float*)A;
       const float* w = (const float*)W;
