@@ -314,9 +314,9 @@ gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, c
   auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
   const int rounds = (K + kFewK - 1) / kFewK, blocks = (K + 15) / 16;
   ilb::pdl_launch_dependents();
-  if (settled) fetch_w(0);
-  ilb::pdl_wait();
-  if (!settled) fetch_w(0);
+  if (!settled) ilb::pdl_wait();
+  fetch_w(0);
+  ilb::pdl_wait();                                   // (returns at once the second time)
   fetch_a(0);
   commit();
   float acc = 0.f, lost = 0.f;                       // of output `lane` = r * T + t
@@ -468,9 +468,10 @@ gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const 
     for (int j = 0; j < 4; ++j) acc[i][j] = lost[i][j] = 0;
   const uint64_t minus = pack2(-1.f, -1.f);
   ilb::pdl_launch_dependents();
-  if (settled) fetch(0, true, false);
-  ilb::pdl_wait();
-  fetch(0, !settled, true);
+  if (!settled) ilb::pdl_wait();
+  fetch(0, true, false);
+  ilb::pdl_wait();                                                 // (returns at once the second time)
+  fetch(0, false, true);
   stash(0);
   __syncthreads();
   const int blocks = (K + BK - 1) / BK;
