@@ -109,16 +109,23 @@ gemm_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W,
 // bit for bit the same result (a zero-padded tail adds +0 to a chain).  Needs K and the leading
 // dimensions multiples of 4 and 16-byte (bfloat16: 8-byte) aligned bases; rows of A beyond M
 // are not multiplied by warps that hold none (a warp is one ty when BN / TN = 32).
+// The loads are ordinary ones that stay where they are written: a kernel here is resident while the launch before still writes A
+// (and a W that is not settled), so these are no read-only data in the sense of __ldg, and the compiler, which may move a read of
+// such data across the dependency wait, did so once in the 64 x 64 kernel.
 template <typename T> struct Vec4;
 template <> struct Vec4<float> {
   float4 v;
-  __device__ __forceinline__ void load(const float* p) { v = __ldg(reinterpret_cast<const float4*>(p)); }
+  __device__ __forceinline__ void load(const float* p) {
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  }
   __device__ __forceinline__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
   __device__ __forceinline__ void get(float (&f)[4]) const { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }
 };
 template <> struct Vec4<__nv_bfloat16> {
   uint2 v;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = __ldg(reinterpret_cast<const uint2*>(p)); }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) {
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  }
   __device__ __forceinline__ void zero() { v = make_uint2(0u, 0u); }
   __device__ __forceinline__ void get(float (&f)[4]) const {
     f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xFFFF0000u);
@@ -272,10 +279,10 @@ constexpr size_t few_smem(int T, int R) {
   return sizeof(float) * ((size_t)2 * (T + kFewWarps * R) * kFewRow + (size_t)kFewWarps * 32 * (R * T + 1));
 }
 
-template <typename TO, int T, int R>
+template <typename TO, int T, int R, bool kSettled>
 __global__ void __launch_bounds__(kFewWarps * 32)
 gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                     TO* __restrict__ out, int M, int N, int K, int lda, int ldw, int ldo, int accumulate, int settled) {
+                     TO* __restrict__ out, int M, int N, int K, int lda, int ldw, int ldo, int accumulate) {
   static_assert(T * R <= 32, "one lane adds up one output");
   extern __shared__ __align__(16) float few[];
   float* As = few;                                   // [2][T][kFewRow]
@@ -314,9 +321,9 @@ gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, c
   auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
   const int rounds = (K + kFewK - 1) / kFewK, blocks = (K + 15) / 16;
   ilb::pdl_launch_dependents();
-  if (!settled) ilb::pdl_wait();
+  if constexpr (!kSettled) ilb::pdl_wait();
   fetch_w(0);
-  ilb::pdl_wait();                                   // (returns at once the second time)
+  if constexpr (kSettled) ilb::pdl_wait();
   fetch_a(0);
   commit();
   float acc = 0.f, lost = 0.f;                       // of output `lane` = r * T + t
@@ -381,16 +388,23 @@ gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, c
   }
 }
 
+template <typename TO, int T, int R, bool kSettled>
+static int launch_few_tiles(const float* A, const float* W, const float* bias, void* out, int M, int N, int K, int lda, int ldw,
+                      int ldo, int accumulate, cudaStream_t stream) {
+  static ilb::OncePerDevice once;
+  constexpr size_t smem = few_smem(T, R);
+  if (once.run([] { return cudaFuncSetAttribute(gemm_simt_few_kernel<TO, T, R, kSettled>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
+    return fail("gemm_simt: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(cudaGetLastError()));
+  ilb::launch(gemm_simt_few_kernel<TO, T, R, kSettled>, dim3((unsigned)((N + kFewWarps * R - 1) / (kFewWarps * R) * ((M + T - 1) / T))), dim3(kFewWarps * 32), smem, stream,
+              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate);
+  return check_launch("gemm_simt");
+}
+
 template <typename TO, int T, int R>
 static int launch_few(const float* A, const float* W, const float* bias, void* out, int M, int N, int K, int lda, int ldw,
                       int ldo, int accumulate, int settled, cudaStream_t stream) {
-  static ilb::OncePerDevice once;
-  constexpr size_t smem = few_smem(T, R);
-  if (once.run([] { return cudaFuncSetAttribute(gemm_simt_few_kernel<TO, T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }) != cudaSuccess)
-    return fail("gemm_simt: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(cudaGetLastError()));
-  ilb::launch(gemm_simt_few_kernel<TO, T, R>, dim3((unsigned)((N + kFewWarps * R - 1) / (kFewWarps * R) * ((M + T - 1) / T))), dim3(kFewWarps * 32), smem, stream,
-              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, settled);
-  return check_launch("gemm_simt");
+  return settled ? launch_few_tiles<TO, T, R, true>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream)
+                 : launch_few_tiles<TO, T, R, false>(A, W, bias, out, M, N, K, lda, ldw, ldo, accumulate, stream);
 }
 
 // The same sums for many tokens.  Bound: the 32-bit pipes (per output and block of 16 k: 16 multiply-adds and 7 operations of the
@@ -412,10 +426,10 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; a
 
 constexpr int kWideM = 64, kWideN = 64, kWideK = 32;
 
-template <typename TA, typename TO>
+template <typename TA, typename TO, bool kSettled>
 __global__ void __launch_bounds__(kWideM * kWideN / 32, 2)
 gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias, TO* __restrict__ out,
-                      int M, int N, int K, int lda, int ldw, int ldo, int accumulate, int settled) {
+                      int M, int N, int K, int lda, int ldw, int ldo, int accumulate) {
   constexpr int BM = kWideM, BN = kWideN, BK = kWideK;
   constexpr int WARPS = (BM / 32) * (BN / 32);
   constexpr int HALVES = BK / 8;                                   // pairs of pieces of a row
@@ -468,9 +482,9 @@ gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const 
     for (int j = 0; j < 4; ++j) acc[i][j] = lost[i][j] = 0;
   const uint64_t minus = pack2(-1.f, -1.f);
   ilb::pdl_launch_dependents();
-  if (!settled) ilb::pdl_wait();
+  if constexpr (!kSettled) ilb::pdl_wait();
   fetch(0, true, false);
-  ilb::pdl_wait();                                                 // (returns at once the second time)
+  if constexpr (kSettled) ilb::pdl_wait();
   fetch(0, false, true);
   stash(0);
   __syncthreads();
@@ -546,8 +560,8 @@ static int launch_wide(const TA* A, const TA* W, const float* bias, void* out, i
                        int accumulate, int settled, cudaStream_t stream) {
   const long long tiles = (long long)((M + kWideM - 1) / kWideM) * ((N + kWideN - 1) / kWideN);
   ILB_REQUIRE(tiles <= 2147483647LL, "gemm_simt: grid too large for M=%d N=%d", M, N);
-  ilb::launch(gemm_simt_wide_kernel<TA, TO>, dim3((unsigned)tiles), dim3(kWideM * kWideN / 32), 0, stream,
-              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate, settled);
+  ilb::launch(settled ? gemm_simt_wide_kernel<TA, TO, true> : gemm_simt_wide_kernel<TA, TO, false>, dim3((unsigned)tiles), dim3(kWideM * kWideN / 32), 0, stream,
+              A, W, bias, (TO*)out, M, N, K, lda, ldw, ldo, accumulate);
   return check_launch("gemm_simt");
 }
 

@@ -211,6 +211,27 @@ def test_gemm_simt_takes_a_matrix_of_the_launch_before(M, in_dtype):
         assert torch.equal(out, want)
 
 
+@pytest.mark.parametrize("M,N,in_dtype", [(1, 40, torch.float32), (4, 40, torch.float32), (40, 40, torch.float32), (45, 64, torch.float32),
+                                          (45, 64, torch.bfloat16), (16, 40, torch.bfloat16), (500, 4001, torch.bfloat16), (300, 40, torch.float32)])
+def test_gemm_simt_takes_rows_of_the_launch_before(M, N, in_dtype):
+    """The rows are the result of the launch right before (a long product), the matrix is settled: the product is that of the rows
+    it leaves, whatever their buffer held."""
+    K, inner = 36, 12288
+    torch.manual_seed(M + N)
+    w = torch.randn(N, K).to(in_dtype).cuda()
+    x, y = torch.randn(M, inner).to(in_dtype).cuda(), (torch.randn(K, inner) / inner ** 0.5).to(in_dtype).cuda()
+    a, out, want = torch.empty(M, K, dtype=in_dtype, device="cuda"), torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    ops().gemm_simt(x, y, a)
+    torch.cuda.synchronize()
+    ops().gemm_simt(a.clone(), w, want)
+    for _ in range(3):
+        a.zero_()
+        torch.cuda.synchronize()
+        ops().gemm_simt(x, y, a)
+        ops().gemm_simt(a, w, out, settled=True)
+        assert torch.equal(out, want)
+
+
 # ------------------------------------------------------------------ attention pieces
 def build_cache(seqs_kv, nkv, d, page_size, num_pages, dtype, seed=0, page_order="shuffled"):
     """Scatter each sequence's keys/values into pages; returns cache tensors and the block
