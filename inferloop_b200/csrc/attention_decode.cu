@@ -213,6 +213,19 @@ __device__ __forceinline__ void touch_row(const float* row, int lane) {
   }
 }
 
+// A value that the launch before may write (an angle, a norm weight that is not settled).  No read-only data in the sense of __ldg,
+// which the compiler may move across the dependency wait, but an ordinary load that stays behind it.
+__device__ __forceinline__ float after_wait(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 after_wait(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+
 // Rows g and g + 8 of the warp's query heads from the fused projection output, as A
 // fragments: per-head RMSNorm in 32-bit (sum over the row's four threads), then the rotation
 // of pairs (i, i + D/2), which a thread holds both members of; rounded to bfloat16 once.
@@ -257,8 +270,8 @@ __device__ __forceinline__ void load_q_fused(uint32_t (&q)[D / 16][4], const __n
 #pragma unroll
       for (int kk = 0; kk < D / 16; ++kk) {
         const int c = kk * 16 + 2 * t;
-        x[kk][0] = x[kk][0] * inv * __ldg(weight + c);     x[kk][1] = x[kk][1] * inv * __ldg(weight + c + 1);
-        x[kk][2] = x[kk][2] * inv * __ldg(weight + c + 8); x[kk][3] = x[kk][3] * inv * __ldg(weight + c + 9);
+        x[kk][0] = x[kk][0] * inv * after_wait(weight + c);     x[kk][1] = x[kk][1] * inv * after_wait(weight + c + 1);
+        x[kk][2] = x[kk][2] * inv * after_wait(weight + c + 8); x[kk][3] = x[kk][3] * inv * after_wait(weight + c + 9);
       }
     }
     if (cs != nullptr) {
@@ -266,7 +279,7 @@ __device__ __forceinline__ void load_q_fused(uint32_t (&q)[D / 16][4], const __n
       for (int kk = 0; kk < D / 32; ++kk) {                // column i < D/2 pairs with i + D/2 = block kk + D/32
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 w = __ldg(cs + kk * 16 + 2 * t + (e & 1) + (e >> 1) * 8);
+          const float2 w = after_wait(cs + kk * 16 + 2 * t + (e & 1) + (e >> 1) * 8);
           const float a = x[kk][e], b = x[kk + D / 32][e];
           // products and sums rounded separately, as the reference's scalar code does
           x[kk][e] = __fsub_rn(__fmul_rn(a, w.x), __fmul_rn(b, w.y));
@@ -316,8 +329,8 @@ __device__ __forceinline__ void load_q_variant(uint32_t (&q)[D / 16][4], const _
       for (int kk = 0; kk < D / 16; ++kk) {
         const int c = kk * 16 + 2 * t;
         if (weight != nullptr) {
-          x[kk][0] = x[kk][0] * inv * __ldg(weight + c);     x[kk][1] = x[kk][1] * inv * __ldg(weight + c + 1);
-          x[kk][2] = x[kk][2] * inv * __ldg(weight + c + 8); x[kk][3] = x[kk][3] * inv * __ldg(weight + c + 9);
+          x[kk][0] = x[kk][0] * inv * after_wait(weight + c);     x[kk][1] = x[kk][1] * inv * after_wait(weight + c + 1);
+          x[kk][2] = x[kk][2] * inv * after_wait(weight + c + 8); x[kk][3] = x[kk][3] * inv * after_wait(weight + c + 9);
         } else {
 #pragma unroll
           for (int e = 0; e < 4; ++e) x[kk][e] = x[kk][e] * inv;
@@ -332,7 +345,7 @@ __device__ __forceinline__ void load_q_variant(uint32_t (&q)[D / 16][4], const _
         for (int h = 0; h < 2; ++h) {
           const int c = kk * 16 + 2 * t + 8 * h;
           if (c + 1 < rd) {
-            const float2 w = __ldg(cs + c / 2);
+            const float2 w = after_wait(cs + c / 2);
             const float a = x[kk][2 * h], b = x[kk][2 * h + 1];
             x[kk][2 * h] = __fsub_rn(__fmul_rn(a, w.x), __fmul_rn(b, w.y));
             x[kk][2 * h + 1] = __fadd_rn(__fmul_rn(a, w.y), __fmul_rn(b, w.x));
@@ -346,7 +359,7 @@ __device__ __forceinline__ void load_q_variant(uint32_t (&q)[D / 16][4], const _
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int i = c + (e & 1) + (e >> 1) * 8;
-          const float2 w = __ldg(cs + i);
+          const float2 w = after_wait(cs + i);
           const float a = x[kk][e], b = x[kk + D / 32][e];
           // products and sums rounded separately, as the reference's scalar code does
           x[kk][e] = __fsub_rn(__fmul_rn(a, w.x), __fmul_rn(b, w.y));
@@ -379,7 +392,7 @@ struct NewKey {
 #pragma unroll
       for (int i = 0; i < E; ++i) { k[h][i] = k_src[element(h, i, lane)]; v[h][i] = v_src[element(h, i, lane)]; }
 #pragma unroll
-    for (int i = 0; i < E; ++i) angle[i] = cs != nullptr ? __ldg(cs + E * lane + i) : make_float2(1.f, 0.f);
+    for (int i = 0; i < E; ++i) angle[i] = cs != nullptr ? after_wait(cs + E * lane + i) : make_float2(1.f, 0.f);
   }
   __device__ __forceinline__ void make(const float* k_weight, float eps, bool rotate, __nv_bfloat16* k_dst, __nv_bfloat16* v_dst,
                                        __nv_bfloat16* row, int lane) {
@@ -396,7 +409,7 @@ struct NewKey {
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int i = 0; i < E; ++i) x[h][i] = x[h][i] * inv * __ldg(k_weight + element(h, i, lane));
+        for (int i = 0; i < E; ++i) x[h][i] = x[h][i] * inv * after_wait(k_weight + element(h, i, lane));
     }
     if (rotate) {
 #pragma unroll
@@ -465,7 +478,7 @@ __device__ __forceinline__ void patch_new_key_variant(uint32_t ks, uint32_t vs, 
     for (int h = 0; h < 2; ++h)
 #pragma unroll
       for (int i = 0; i < E; ++i)
-        k[h][i] = k_weight != nullptr ? k[h][i] * inv * __ldg(k_weight + h * (D / 2) + E * lane + i) : k[h][i] * inv;
+        k[h][i] = k_weight != nullptr ? k[h][i] * inv * after_wait(k_weight + h * (D / 2) + E * lane + i) : k[h][i] * inv;
   };
   if (normed && !(mode & kNormAfterRotation)) norm();
   if (cs != nullptr && (mode & kPairsInterleaved)) {
@@ -474,7 +487,7 @@ __device__ __forceinline__ void patch_new_key_variant(uint32_t ks, uint32_t vs, 
       if constexpr (E == 2) {                               // the lane's two elements of this half are a pair
         const int e = h * (D / 2) + 2 * lane;
         if (e + 1 < rd) {
-          const float2 w = __ldg(cs + e / 2);
+          const float2 w = after_wait(cs + e / 2);
           const float a = k[h][0], b = k[h][1];
           k[h][0] = __fsub_rn(__fmul_rn(a, w.x), __fmul_rn(b, w.y));
           k[h][1] = __fadd_rn(__fmul_rn(a, w.y), __fmul_rn(b, w.x));
@@ -483,7 +496,7 @@ __device__ __forceinline__ void patch_new_key_variant(uint32_t ks, uint32_t vs, 
         const int e = h * (D / 2) + lane;
         const float mine = k[h][0], other = __shfl_xor_sync(0xffffffffu, mine, 1);
         if ((e | 1) < rd) {
-          const float2 w = __ldg(cs + e / 2);
+          const float2 w = after_wait(cs + e / 2);
           k[h][0] = (lane & 1) ? __fadd_rn(__fmul_rn(other, w.y), __fmul_rn(mine, w.x))
                                : __fsub_rn(__fmul_rn(mine, w.x), __fmul_rn(other, w.y));
         }
@@ -492,7 +505,7 @@ __device__ __forceinline__ void patch_new_key_variant(uint32_t ks, uint32_t vs, 
   } else if (cs != nullptr) {
 #pragma unroll
     for (int i = 0; i < E; ++i) {
-      const float2 w = __ldg(cs + E * lane + i);
+      const float2 w = after_wait(cs + E * lane + i);
       const float a = k[0][i], b = k[1][i];
       k[0][i] = __fsub_rn(__fmul_rn(a, w.x), __fmul_rn(b, w.y));
       k[1][i] = __fadd_rn(__fmul_rn(a, w.y), __fmul_rn(b, w.x));
@@ -500,7 +513,7 @@ __device__ __forceinline__ void patch_new_key_variant(uint32_t ks, uint32_t vs, 
   }
   if (normed && (mode & kNormAfterRotation)) norm();
   if (v_mode != 0) {
-    const float lam = v_mode == 2 ? __ldg(v_lambda) : 0.f;
+    const float lam = v_mode == 2 ? after_wait(v_lambda) : 0.f;
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -629,7 +642,7 @@ decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   auto emit_pair = [&](int head, int m, auto&& value) {
     float a = value(m), b = value(m + DV / 2);
     if (turn != nullptr) {
-      const float2 w = __ldg(turn + m);
+      const float2 w = after_wait(turn + m);
       const float t = fmaf(b, w.y, a * w.x);
       b = fmaf(-a, w.y, b * w.x);
       a = t;
