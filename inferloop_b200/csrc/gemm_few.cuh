@@ -1,0 +1,570 @@
+// bfloat16 products of up to 128 tokens, included by gemm_tcgen05.cu (whose helpers it uses):
+//     out[T, N] (+)= A[T, K] * W[N, K]^T (+ bias), or the gated unit over interleaved gate and up rows,
+// where A is given, or is the RMS norm of 32-bit rows that the kernel reads itself.
+//
+// What bounds it: the weight is read once, so the floor is its bytes at the copy rate.  Three things kept the
+// former deal (128 weight rows on the MMA's rows, one or two tiles to an SM) away from it: tiles of one height
+// leave a quarter to a half of the SMs with half the work of the others (24,576 rows are 192 tiles of 128 for
+// 148 SMs), the tokens' operand is fetched again for every tile, and many tokens leave a shallow ring.  Here the
+// tokens are the MMA's rows (64 of them, or 128; a tile's operand A block holds the real tokens only, the MMA
+// reads on into the weight block behind it and the rows that come of it are nobody's) and the weight rows its
+// columns, so that a tile may be any multiple of 16 rows up to 256.  `few_plan` picks the height and the number of
+// K ranges for which the CTAs, two to an SM, come out even.  Launch after launch on rotating weights (us; before ->
+// after, the floor in brackets): 24,576 x 4,096 gated, 8 tokens 36.1 -> 33.0 (30.8), 64 tokens 45.6 -> 36.5, 128
+// tokens 55.8 -> 41.7; 51,200 x 5,120 gated, 24 tokens 95.2 -> 79.1 (80.2); 5,120 x 17,408 adding, 8 tokens 29.9 ->
+// 27.9 (27.3), 24 tokens 35.8 -> 30.6, 96 tokens 37.7 -> 32.5; 6,144 x 4,096, 8 tokens 12.0 -> 11.1 (7.7), 96
+// tokens 22.2 -> 16.7; 10,240 x 5,120, 64 tokens 27.8 -> 22.8 (16.0).
+//
+// Per CTA (320 threads):
+//   warp 0     requests the weight blocks by TMA (128-byte swizzle; one box a block, or for gated weights a box of
+//              eight gate rows and their eight up rows for every 16 rows of the tile, so that a tile need not be
+//              whole blocks of 64) into a ring of `stages` buffers, the first ring before the kernel waits for its
+//              predecessor; one lane requests the token blocks behind the wait;
+//   warp 1     tensor memory; one lane issues tcgen05.mma, four to a K block of 64;
+//   warps 2-9  the write-out.  With one K range, or ranges that meet in memory (red.add), the tile goes through the
+//              idle ring so that a thread holds four neighbouring outputs; the ranges of a tile that must be added
+//              in K order are the CTAs of a cluster, which send each other their shares (st.async on the owner's
+//              mbarrier), chunk j of 16 columns belonging to CTA j % split.
+// Norm inside (TT > 0): out = (x * w) W^T / rms(x), and the root mean square is a factor of the row that can be
+// applied to the 32-bit result.  So warps 2-9 read the 32-bit rows, multiply by the norm's weight, round to
+// bfloat16 (one rounding, as the norm's own kernel has) and lay them out as the MMA wants them, a block at a
+// time ahead of the weight stream, with the sums of squares beside.  A launch and its wait fall away (1.7 us) for
+// 0.3 to 0.8 us in the product.  Every CTA reads the rows again: at 16 tokens of 4,096 x 24,576 33.7 -> 34.3 us,
+// at 24 tokens of 5,120 x 34,816 54.8 -> 58.3 us, more than the norm's launch; so up to 16 tokens.
+// All mbarrier waits are bounded, as in the other kernels.
+
+constexpr int kFewTokens = 128, kFewNormTokens = 16;
+constexpr int kFewWarps = 8, kFewEpi = 32 * kFewWarps, kFewThreads = 64 + kFewEpi;
+constexpr int kFewStages = 12;
+// Two CTAs to an SM: 228 KB less 1 KB each that the system keeps, halved.
+constexpr int kFewSmem = 112 * 1024;
+
+struct FewParams {
+  void* out;
+  const float* bias;
+  int* error_flag;
+  const float* x;            // NORM: the 32-bit rows [T, K] the product takes normed, and the norm's weight
+  const float* norm_w;
+  float eps;
+  int T, N, K, ldo, ldx;
+  int rows, tp, k_blocks, split, cluster, stages, tmem_cols, red;
+  int stage_bytes, ring_bytes, recv_bytes;
+  int epilogue, out_f32, relu2, gate_relu;
+  float act_limit, act_sharp, act_offset;
+};
+
+// TT: tokens the norm's threads may have to look after (0: the product reads its rows as they are).
+template <int MM, int TT>
+__global__ void __launch_bounds__(kFewThreads, 2)
+gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_y, const FewParams p) {
+  constexpr bool NORM = TT > 0;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - smem_u32(smem_raw));
+  float* recv = reinterpret_cast<float*>(smem + p.ring_bytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.ring_bytes + p.recv_bytes);
+  const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kFewStages, tfull = empty0 + 8 * kFewStages, rbar = tfull + 8;
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * kFewStages + 2);
+  volatile int* failed = reinterpret_cast<volatile int*>(bars + 2 * kFewStages + 3);
+  float* ssq = reinterpret_cast<float*>(bars + 2 * kFewStages + 4);      // NORM: [warps][tokens] partial sums; then [tokens]
+
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x / p.split, part = blockIdx.x - tile * p.split;
+  const int kb0 = (int)((long long)p.k_blocks * part / p.split), cnt = (int)((long long)p.k_blocks * (part + 1) / p.split) - kb0;
+  const bool gated = p.epilogue == kSwiGLU;
+  const int row0 = tile * p.rows;
+  const int n_early = cnt < p.stages ? cnt : p.stages;
+  const uint32_t w_off = (uint32_t)p.tp * 128u;
+  const uint32_t tx = (uint32_t)(p.rows + (NORM ? 0 : p.tp)) * 128u;
+  const int boxes = gated ? p.rows / 16 : 1;
+  auto load_w = [&](uint32_t dst, uint32_t bar, int kcol) {
+    if (gated) {
+      if (lane < boxes) {
+        const int g = row0 / 16 + lane;
+        tma_load_5d(dst + w_off + (uint32_t)lane * 2048u, &map_w, bar, kcol, 0, g & 7, 0, g >> 3);
+      }
+    } else if (lane == 0) {
+      tma_load_2d(dst + w_off, &map_w, bar, kcol, row0);
+    }
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int s = 0; s < p.stages; ++s) { mbar_init(full0 + 8 * s, NORM ? 2 : 1); mbar_init(empty0 + 8 * s, 1); }
+      mbar_init(tfull, 1);
+      if (p.cluster > 1) mbar_init(rbar, 1);
+      *failed = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      if (p.cluster > 1) {
+        const int nch = p.rows / 16, me = part;
+        const int nloc = (nch - me + p.split - 1) / p.split;
+        mbar_expect_tx(rbar, (uint32_t)(p.split * nloc * p.T * 64 + (NORM ? p.split * ((p.T + 3) / 4) * 16 : 0)));
+      }
+      for (int it = 0; it < n_early; ++it) mbar_expect_tx(full0 + 8 * it, tx);
+    }
+    __syncwarp();
+    for (int it = 0; it < n_early; ++it) load_w(base + it * p.stage_bytes, full0 + 8 * it, (kb0 + it) * kBlockK);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(p.tmem_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  if (p.cluster > 1) cluster_sync_all(); else __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    bool ok = true;
+    if (!NORM) {
+      pdl_wait();
+      if (lane == 0)
+        for (int it = 0; it < n_early; ++it) tma_load_2d(base + it * p.stage_bytes, &map_y, full0 + 8 * it, (kb0 + it) * kBlockK, 0);
+    }
+    int s = n_early == p.stages ? 0 : n_early;
+    uint32_t ph = 0;
+    int armed = n_early;
+    for (int it = n_early; it < cnt; ++it) {
+      ok = mbar_wait(empty0 + 8 * s, ph);
+      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      const uint32_t dst = base + s * p.stage_bytes;
+      if (lane == 0) {
+        mbar_expect_tx(full0 + 8 * s, tx);
+        if (!NORM) tma_load_2d(dst, &map_y, full0 + 8 * s, (kb0 + it) * kBlockK, 0);
+      }
+      __syncwarp();
+      load_w(dst, full0 + 8 * s, (kb0 + it) * kBlockK);
+      armed = it + 1;
+      if (++s == p.stages) { s = 0; ph ^= 1; }
+    }
+    if (!ok && lane == 0) {
+      *failed = 1; if (p.error_flag) *p.error_flag = 1;
+      for (int it = armed > p.stages ? armed - p.stages : 0; it < armed; ++it) mbar_wait(full0 + 8 * (it % p.stages), (it / p.stages) & 1);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.rows >> 3) << 17) | ((uint32_t)(MM >> 4) << 24);
+      bool ok = true;
+      int s = 0;
+      uint32_t ph = 0;
+      for (int it = 0; it < cnt; ++it) {
+        ok = mbar_wait(full0 + 8 * s, ph);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint32_t a = base + s * p.stage_bytes;
+        const uint64_t da = smem_desc(a), db = smem_desc(a + w_off);
+#pragma unroll
+        for (int k = 0; k < kBlockK / 16; ++k) mma_bf16(tmem, da + 2 * k, db + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
+        tcgen05_commit(empty0 + 8 * s);
+        if (++s == p.stages) { s = 0; ph ^= 1; }
+      }
+      if (!ok) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
+      tcgen05_commit(tfull);
+    }
+  } else {
+    const int et = threadIdx.x - 64, ew = warp - 2;
+    pdl_wait();
+    if (NORM) {
+      // ---- the rows: norm weight applied, rounded to bfloat16 and laid out as the MMA reads them, sums of squares beside
+      constexpr int kPer = TT > 0 ? TT / 2 : 1;              // tokens of a lane
+      float sq[kPer];
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) sq[i] = 0.f;
+      const int half = lane >> 4, c = lane & 15;
+      bool ok = true;
+      // A stage belongs to one warp: it sees every phase of the stage's barrier (a parity tells two neighbouring phases apart, no more).
+      int s = ew, round = 0;
+      for (int it = ew; ok; ) {
+        if (s >= p.stages) { s = ew; ++round; if (s >= p.stages) break; }
+        it = round * p.stages + s;
+        if (it >= cnt) break;
+        const int k = (kb0 + it) * kBlockK + c * 4;
+        const bool in_k = k < p.K;                            // (K is a multiple of 8)
+        const float4 w = in_k ? *reinterpret_cast<const float4*>(p.norm_w + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 v[kPer];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          const int t = 2 * i + half;
+          v[i] = (t < p.T && in_k) ? __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)t * p.ldx + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (round > 0) ok = mbar_wait(empty0 + 8 * s, (round - 1) & 1);
+        const uint32_t dst = base + s * p.stage_bytes;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          const int t = 2 * i + half;
+          if (t < p.T) {
+            sq[i] = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, sq[i]))));
+            const uint32_t lo = pack_bf16(v[i].x * w.x, v[i].y * w.y), hi = pack_bf16(v[i].z * w.z, v[i].w * w.w);
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + (uint32_t)t * 128u + (uint32_t)((((c >> 1) ^ (t & 7)) << 4) | ((c & 1) << 3))), "r"(lo), "r"(hi) : "memory");
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0 && ok) mbar_arrive(full0 + 8 * s);
+        s += kFewWarps;
+      }
+      if (!ok) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
+        if (c == 0) ssq[ew * TT + 2 * i + half] = sq[i];
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(kFewEpi) : "memory");
+      float total = 0.f;
+      if (et < TT) {
+#pragma unroll
+        for (int w = 0; w < kFewWarps; ++w) total += ssq[w * TT + et];
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(kFewEpi) : "memory");
+      if (et < TT) ssq[et] = p.cluster > 1 ? total : rsqrtf(total / (float)p.K + p.eps);
+      asm volatile("bar.sync 1, %0;" ::"n"(kFewEpi) : "memory");
+    }
+    const int quad = warp & 3, hf = ew >> 2;
+    const int t = MM == 128 ? quad * 32 + lane : quad * 16 + lane;
+    const bool warp_on = (MM == 128 ? quad * 32 : quad * 16) < p.T;
+    const bool mine = t < p.T && (MM == 128 || lane < 16);
+    const int nch = p.rows / 16;
+    if (!mbar_wait(tfull, 0)) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
+    tcgen05_fence_after();
+    const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
+    const bool bad = *failed != 0;
+    if (p.cluster > 1) {
+      // ---- the K ranges of a tile are the CTAs of a cluster: chunk j of 16 columns belongs to CTA j % split
+      const int nmax = (nch + p.split - 1) / p.split;
+      const uint32_t recv_addr = smem_u32(recv);
+      const uint32_t sums_off = (uint32_t)(p.split * nmax * p.T) * 64u;
+      if (NORM && et < (p.T + 3) / 4) {
+        const float4 v = *reinterpret_cast<const float4*>(ssq + 4 * et);
+        for (int q = 0; q < p.split; ++q)
+          st_peer_v4(peer_addr(recv_addr + sums_off + (uint32_t)(part * ((p.T + 3) / 4) + et) * 16u, q), peer_addr(rbar, q), v.x, v.y, v.z, v.w);
+      }
+      if (warp_on) {
+        for (int j = hf; j < nch; j += 2) {
+          float v[32];
+          tmem_load_16(taddr + j * 16, v);
+          if (mine) {
+            const uint32_t owner = (uint32_t)(j % p.split);
+            const uint32_t nl = (uint32_t)((nch - (int)owner + p.split - 1) / p.split);
+            const uint32_t dst = peer_addr(recv_addr + (((uint32_t)part * nl + (uint32_t)(j / p.split)) * (uint32_t)p.T + (uint32_t)t) * 64u, owner);
+            const uint32_t bar = peer_addr(rbar, owner);
+#pragma unroll
+            for (int c4 = 0; c4 < 4; ++c4)
+              st_peer_v4(dst + (uint32_t)((c4 ^ ((t >> 1) & 3)) << 4), bar, v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
+          }
+        }
+      }
+      const int nl = (nch - part + p.split - 1) / p.split;
+      const bool vec = p.ldo % 4 == 0 && (uintptr_t)p.out % 16 == 0;
+      bool arrived = false;
+      const int per_shift = gated ? 1 : 2, n_end = gated ? p.N / 2 : p.N;       // units of four outputs: two or four a chunk
+      for (int u0 = et; u0 < (nl * p.T) << per_shift; u0 += 2 * kFewEpi) {
+        float old[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int u = u0 + i * kFewEpi;
+          const int c4 = u & ((1 << per_shift) - 1), q = u >> per_shift, jl = q / p.T, tt = q - jl * p.T;
+          const int n = row0 + (jl * p.split + part) * 16 + c4 * 4;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) old[i][e] = 0.f;
+          if (p.epilogue == kAccumulate && jl < nl) {
+            const float* src = (const float*)p.out + (size_t)tt * p.ldo + n;
+            if (vec && n + 4 <= p.N) {
+              const float4 o = __ldcg(reinterpret_cast<const float4*>(src));
+              old[i][0] = o.x; old[i][1] = o.y; old[i][2] = o.z; old[i][3] = o.w;
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) if (n + e < p.N) old[i][e] = __ldcg(src + e);
+            }
+          }
+        }
+        if (!arrived) {
+          if (!mbar_wait(rbar, 0)) { *failed = 1; if (p.error_flag) *p.error_flag = 1; break; }
+          arrived = true;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int u = u0 + i * kFewEpi;
+          const int c4 = u & ((1 << per_shift) - 1), q = u >> per_shift, jl = q / p.T, tt = q - jl * p.T;
+          if (jl >= nl) continue;
+          const int chunk = jl * p.split + part;
+          const int n = gated ? row0 / 2 + chunk * 8 + c4 * 4 : row0 + chunk * 16 + c4 * 4;
+          float a[4] = {0.f, 0.f, 0.f, 0.f}, up[4] = {0.f, 0.f, 0.f, 0.f}, total = 0.f;
+          for (int z = 0; z < p.split; ++z) {
+            const float* src = recv + (size_t)((z * nl + jl) * p.T + tt) * 16;
+            const float4 s4 = *reinterpret_cast<const float4*>(src + ((c4 ^ ((tt >> 1) & 3)) << 2));
+            a[0] += s4.x; a[1] += s4.y; a[2] += s4.z; a[3] += s4.w;
+            if (gated) {
+              const float4 u4 = *reinterpret_cast<const float4*>(src + (((c4 + 2) ^ ((tt >> 1) & 3)) << 2));
+              up[0] += u4.x; up[1] += u4.y; up[2] += u4.z; up[3] += u4.w;
+            }
+            if (NORM) total += recv[sums_off / 4 + z * ((p.T + 3) / 4) * 4 + tt];
+          }
+          if (NORM) {
+            const float r = rsqrtf(total / (float)p.K + p.eps);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { a[e] *= r; up[e] *= r; }
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float b = (p.bias && n + e < n_end) ? p.bias[n + e] : 0.f;
+            a[e] = gated ? gate_mul(p, a[e], up[e]) : relu2_if(p.relu2, a[e] + b + old[i][e]);
+          }
+          const size_t o = (size_t)tt * p.ldo + n;
+          if (vec && n + 4 <= n_end) {
+            if (p.out_f32) *reinterpret_cast<float4*>((float*)p.out + o) = make_float4(a[0], a[1], a[2], a[3]);
+            else *reinterpret_cast<uint2*>((__nv_bfloat16*)p.out + o) = make_uint2(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]));
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (n + e < n_end) { if (p.out_f32) ((float*)p.out)[o + e] = a[e]; else ((__nv_bfloat16*)p.out)[o + e] = __float2bfloat16_rn(a[e]); }
+          }
+        }
+      }
+      if (!arrived && !mbar_wait(rbar, 0)) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
+    } else if (!bad) {
+      // ---- the tile (or its K range) through shared memory: the ring is idle, everything in it has been consumed
+      float* st = reinterpret_cast<float*>(smem);
+      const int pitch = p.rows + 4;
+      if (warp_on) {
+        for (int j = hf; j < nch; j += 2) {
+          float v[32];
+          tmem_load_16(taddr + j * 16, v);
+          if (mine) {
+#pragma unroll
+            for (int c4 = 0; c4 < 4; ++c4)
+              *reinterpret_cast<float4*>(st + (size_t)t * pitch + j * 16 + c4 * 4) = make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
+          }
+        }
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(kFewEpi) : "memory");
+      const bool vec = p.ldo % 4 == 0 && (uintptr_t)p.out % 16 == 0;
+      const int per = gated ? p.rows / 8 : p.rows / 4;       // units of four outputs a token
+      const int n_end = gated ? p.N / 2 : p.N;
+      for (int u = et; u < per * p.T; u += kFewEpi) {
+        const int tt = u / per, f = u - tt * per;
+        float a[4];
+        int n;
+        const float r = NORM ? ssq[tt] : 1.f;
+        if (gated) {
+          const float* src = st + (size_t)tt * pitch + (f >> 1) * 16 + (f & 1) * 4;
+          const float4 g = *reinterpret_cast<const float4*>(src), up = *reinterpret_cast<const float4*>(src + 8);
+          a[0] = gate_mul(p, g.x * r, up.x * r); a[1] = gate_mul(p, g.y * r, up.y * r);
+          a[2] = gate_mul(p, g.z * r, up.z * r); a[3] = gate_mul(p, g.w * r, up.w * r);
+          n = row0 / 2 + f * 4;
+        } else {
+          const float4 g = *reinterpret_cast<const float4*>(st + (size_t)tt * pitch + f * 4);
+          a[0] = g.x * r; a[1] = g.y * r; a[2] = g.z * r; a[3] = g.w * r;
+          n = row0 + f * 4;
+          if (p.bias && (!p.red || part == 0)) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[e] += n + e < n_end ? p.bias[n + e] : 0.f;
+          }
+        }
+        const size_t o = (size_t)tt * p.ldo + n;
+        if (p.red) {
+          float* dst = (float*)p.out + o;
+          if (vec && n + 4 <= n_end) {
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a[0]), "f"(a[1]), "f"(a[2]), "f"(a[3]) : "memory");
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) if (n + e < n_end) atomicAdd(dst + e, a[e]);
+          }
+          continue;
+        }
+        if (p.epilogue == kAccumulate) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) if (n + e < n_end) a[e] += __ldcg((const float*)p.out + o + e);
+        }
+        if (p.relu2) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] = relu2_if(1, a[e]);
+        }
+        if (vec && n + 4 <= n_end) {
+          if (p.out_f32) *reinterpret_cast<float4*>((float*)p.out + o) = make_float4(a[0], a[1], a[2], a[3]);
+          else *reinterpret_cast<uint2*>((__nv_bfloat16*)p.out + o) = make_uint2(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (n + e < n_end) { if (p.out_f32) ((float*)p.out)[o + e] = a[e]; else ((__nv_bfloat16*)p.out)[o + e] = __float2bfloat16_rn(a[e]); }
+        }
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ host side
+constexpr int kFewTail = (2 * kFewStages + 4) * 8 + kFewWarps * kFewNormTokens * 4;     // barriers, flags, sums of squares
+
+// The interleaved weight [rows, cols]: boxes of eight gate rows and their eight up rows, 64 deep.
+int make_gated_map(CUtensorMap* out, const void* ptr, int rows, int cols, int ld) {
+  static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
+  static std::mutex mu;
+  const MapKey key{ptr, rows, cols, ld, 0};
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(key);
+  if (it != cache.end()) { *out = it->second; return 0; }
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail("gemm_tc: cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t ldb = (cuuint64_t)ld * 2;
+  const cuuint64_t dims[5] = {(cuuint64_t)cols, 8, 8, 2, (cuuint64_t)(rows / 128)}, strides[4] = {ldb, 8 * ldb, 64 * ldb, 128 * ldb};
+  const cuuint32_t box[5] = {(cuuint32_t)kBlockK, 8, 1, 2, 1}, estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail("gemm_tc: cuTensorMapEncodeTiled failed with code %d (gated rows %d cols %d ld %d)", (int)r, rows, cols, ld);
+  if (cache.size() > 4096) cache.clear();
+  cache.emplace(key, *out);
+  return 0;
+}
+
+template <int MM, int TT>
+cudaError_t configure_few() {
+  static OncePerDevice once;
+  return once.run([] {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MM, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
+    if (e == cudaSuccess)      // two CTAs share an SM only with the largest shared-memory carve-out
+      cudaFuncSetAttribute(gemm_few_kernel<MM, TT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e;
+  });
+}
+
+// How a product of few tokens is dealt out.
+struct FewPlan { int rows, split, stages, cluster, red, tiles, grid, ring, recv, smem; };
+
+// The shared memory of a plan, with as many stages as two CTAs to an SM leave room for; false when two do not fit.
+bool few_memory(int T, int k_range, FewPlan& f) {
+  const int tp = (T + 7) / 8 * 8, stage = (tp + f.rows) * 128, mm = T <= 64 ? 64 : 128;
+  f.recv = f.cluster > 1 ? f.split * ((f.rows / 16 + f.split - 1) / f.split) * T * 64 + f.split * ((T + 3) / 4) * 16 : 0;
+  const int room = kFewSmem - 1024 - kFewTail - f.recv;
+  f.stages = room / stage;
+  if (f.stages > kFewStages) f.stages = kFewStages;
+  if (f.stages > k_range) f.stages = k_range;
+  if (f.stages < (k_range < 2 ? k_range : 2)) return false;
+  f.ring = f.stages * stage;
+  const int reach = (f.stages - 1) * stage + mm * 128;             // the MMA reads mm rows from the last stage's first
+  if (reach > f.ring) f.ring = reach;
+  const int staged = (T * (f.rows + 4) * 4 + 15) / 16 * 16;        // the tile on its way out
+  if (f.cluster == 1 && staged > f.ring) f.ring = staged;
+  f.smem = 1024 + f.ring + f.recv + kFewTail;
+  return f.smem <= kFewSmem;
+}
+
+// Clusters of so many CTAs, two CTAs to an SM, that the device holds at once.  The occupancy query counts one CTA to an
+// SM for any kernel that allocates tensor memory, so an empty kernel of the same shape is asked about: it answers 148, 71 and
+// 33 clusters of 2, 4 and 8, and 72 clusters of four did take a second round (18 -> 26 us), 64 and 66 did not.
+__global__ void __launch_bounds__(kFewThreads, 2) few_shape_kernel() {}
+
+int few_clusters(int cluster) {
+  static int cache[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  if (cluster < 1 || cluster > 8) return 0;
+  if (cache[cluster] != 0) return cache[cluster] < 0 ? 0 : cache[cluster];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster * 256);
+  cfg.blockDim = dim3(kFewThreads);
+  cfg.dynamicSmemBytes = kFewSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  int n = 0;
+  cudaError_t e = cudaFuncSetAttribute(few_shape_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(few_shape_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, few_shape_kernel, &cfg);
+  if (e != cudaSuccess) { cudaGetLastError(); n = 0; }
+  cache[cluster] = n > 0 ? n : -1;
+  return n > 0 ? n : 0;
+}
+
+// What a plan costs, near enough to its time in us to rank plans: a fit to 9,600 timed plans of 20 weights (1,024 to 51,200 rows,
+// 1,024 to 25,600 deep) at 1 to 128 tokens; the plan it picks is on average 1.4 % slower than the best one.  What decides is not
+// an SM's share of the bytes but how long a CTA's stream is against its ring (a round trip of 3.4 us for `stages` blocks of
+// 64) and how many MMAs are issued (four a block, each as long as 118 columns at least); a second CTA on some SMs leaves
+// less room to the next kernel's first blocks; and the shares that meet cost by the value.
+double few_cost(int T, int N, int K, const FewPlan& f) {
+  const int kb = (K + kBlockK - 1) / kBlockK, range = (kb + f.split - 1) / f.split, sms = sm_count();
+  const int per_sm = f.grid <= sms ? 1 : 2;
+  const double bytes = (double)N * K * 2 / 7.0e6, ring = 3.38 * range / f.stages, tile = 1e-3 * T * f.rows;
+  double t = (bytes > ring ? bytes : ring) + 0.317 * range + 0.107 * per_sm * range * (f.rows > 118 ? f.rows / 128.0 : 0.92);
+  if (per_sm == 2) t += 0.476 + 2.44 * (f.grid - sms) / sms;
+  if (f.red) t += 0.965 * f.split * 4e-6 * T * N;
+  else if (f.cluster > 1) t += (0.78 + 1.04 * per_sm) * tile + 0.02 * f.split;
+  else t += 0.966 * tile;
+  return t;
+}
+
+// `in_memory` > 1: the K ranges of a tile, up to that many, may be separate CTAs that add into the output in memory (the sum's order
+// is then not fixed).  False where the kernel does not serve: more tokens, or a weight of more tiles than two CTAs to an SM.
+bool few_plan(int T, int N, int K, int in_memory, FewPlan& best) {
+  if (T > kFewTokens || (N + 255) / 256 > 2 * sm_count()) return false;
+  struct Key { long long a, b; bool operator==(const Key& o) const { return a == o.a && b == o.b; } };
+  struct Hash { size_t operator()(const Key& k) const { return std::hash<long long>()(k.a * 1000003ll ^ k.b); } };
+  static std::unordered_map<Key, FewPlan, Hash> cache;
+  static std::mutex mu;
+  const Key key{((long long)T << 32) | (unsigned)N, ((long long)K << 8) | in_memory};
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(key);
+  if (it != cache.end()) { best = it->second; return best.rows > 0; }
+  const int kb = (K + kBlockK - 1) / kBlockK;
+  const bool may_add = in_memory > 1;
+  // Clusters are not placed in the last slots while the kernel before still holds some: 280 and 292 CTAs lost 5 to 6 % to 256.
+  // More than 64 tokens that add in memory: one CTA to an SM (two take 0.5 to 1 us less of 10 to 45, but a product of many tokens
+  // has never had more).
+  const int most = !may_add ? 2 * sm_count() * 15 / 16 : T > 64 ? sm_count() : 2 * sm_count();
+  double least = 1e30;
+  best = FewPlan{};
+  auto consider = [&](int split) {
+    for (int rows = 16; rows <= 256; rows += 16) {
+      FewPlan f{};
+      f.rows = rows; f.split = split; f.red = may_add && split > 1 ? 1 : 0; f.cluster = f.red ? 1 : split;
+      f.tiles = (N + rows - 1) / rows; f.grid = f.tiles * split;
+      if (f.grid > (split > 1 ? most : 2 * sm_count()) || !few_memory(T, kb / split, f)) continue;
+      const double t = few_cost(T, N, K, f);
+      if (t >= least) continue;
+      if (f.cluster > 1 && f.tiles > few_clusters(f.cluster)) continue;       // all clusters at once, or the last ones cost a second round
+      least = t;
+      best = f;
+    }
+  };
+  if (may_add) {
+    for (int split = 1; split <= in_memory && split <= kb; ++split) consider(split);
+  } else {
+    // Sums of fewer than eight blocks: as many ranges as there are powers of two, whatever the tokens, as products of more tokens
+    // have them: the same partial sums, and a row's bits rarely depend on what it is computed beside.  (At 16 tokens the
+    // fastest too, 768 x 256 3.04 -> 2.71 us; at 40 tokens it takes up to 0.6 us more, 1,536 x 256 2.96 -> 3.56.)
+    if (kb < 8) consider(kb >= 4 ? 4 : kb >= 2 ? 2 : 1);
+    // (tiles of 64 rows that fill the device twice over: an exchange could only cost)
+    if (best.rows == 0)
+      for (int split = 1; split <= 8 && split <= kb && (split == 1 || (long long)N <= 64ll * 2 * sm_count()); split *= 2) consider(split);
+  }
+  if (cache.size() > 4096) cache.clear();
+  cache.emplace(key, best);
+  return best.rows > 0;
+}
+
+template <int MM, int TT>
+int launch_few(const CUtensorMap& mw, const CUtensorMap& my, const FewParams& p, const FewPlan& f, cudaStream_t stream) {
+  const cudaError_t e = configure_few<MM, TT>();
+  if (e != cudaSuccess) return fail("gemm_tc: cannot reserve %d bytes of shared memory: %s", kFewSmem, cudaGetErrorString(e));
+  ilb::launch_cluster(gemm_few_kernel<MM, TT>, dim3(f.grid), dim3(kFewThreads), (size_t)f.smem, stream, p.cluster, mw, my, p);
+  return check_launch("gemm_tc");
+}
+
+// Fills in the deal and launches; `p` holds everything else.
+int run_few(FewParams& p, const FewPlan& f, const void* A, int lda, const void* W, int ldw, cudaStream_t stream) {
+  p.rows = f.rows; p.tp = (p.T + 7) / 8 * 8; p.k_blocks = (p.K + kBlockK - 1) / kBlockK; p.split = f.split; p.cluster = f.cluster;
+  p.stages = f.stages; p.red = f.red; p.stage_bytes = (p.tp + p.rows) * 128; p.ring_bytes = f.ring; p.recv_bytes = f.recv;
+  p.tmem_cols = p.rows <= 32 ? 32 : p.rows <= 64 ? 64 : p.rows <= 128 ? 128 : 256;
+  CUtensorMap mw, my;
+  if (p.epilogue == kSwiGLU ? make_gated_map(&mw, W, p.N, p.K, ldw) : make_map(&mw, W, p.N, p.K, ldw, p.rows)) return -1;
+  my = mw;
+  if (A != nullptr && make_map(&my, A, p.T, p.K, lda, p.tp)) return -1;
+  if (p.x != nullptr) return p.T <= 8 ? launch_few<64, 8>(mw, my, p, f, stream) : launch_few<64, 16>(mw, my, p, f, stream);
+  return p.T <= 64 ? launch_few<64, 0>(mw, my, p, f, stream) : launch_few<128, 0>(mw, my, p, f, stream);
+}

@@ -3,7 +3,8 @@
 // or, for a weight whose rows interleave 64 gate rows with their 64 up rows,
 //     out[M,N/2] = silu(gate) * up   (the SwiGLU product in the epilogue).
 //
-// One kernel serves decode-shaped (few tokens) and prefill-shaped (many tokens) products.
+// Up to 128 tokens run on `gemm_few_kernel` (gemm_few.cuh), unless the weight has more tiles than two CTAs to an SM
+// (the output matrix); those, and products of more tokens, on the kernels of this file.
 // tcgen05.mma computes D[128 x BN] = X[128 x K] * Y[BN x K]^T with both operands K-major in
 // shared memory.  With few tokens the operands are swapped: X is a 128-row tile of the
 // WEIGHT and Y the (padded) tokens, so every tensor-core row does useful work and the
@@ -21,14 +22,6 @@
 //   warps 2-5   read an accumulator with tcgen05.ld and write the result while the next
 //               tile accumulates in the other one.
 // How the work is dealt out (host side, end of this file):
-//   few tokens, tiles <= 2 CTAs per SM: every tile's K range is cut into 1, 2, 4 or 8 equal
-//     parts, one per CTA of a thread-block cluster.  Each CTA SENDS the rows of its share to
-//     the CTA that owns them (st.async, counted by the owner's mbarrier); the owner adds the
-//     shares in K order from its own shared memory and writes out (token tiles up to 64; the
-//     128-token tile keeps the older form in which owners read their peers' shares between
-//     two cluster barriers).  One cluster barrier, at the start.
-//     Accumulating products of up to eight tokens with a large weight skip the cluster: the K
-//     ranges are separate CTAs that add their shares into the 32-bit output (red.add.v4).
 //   few tokens, many tiles (the output matrix): a persistent grid takes equal, contiguous runs
 //     of (tile, K block) units ("stream-K"); a tile shared by two CTAs goes through a 32-bit
 //     workspace slot and a ticket: the CTA that takes the tile's last ticket adds the shares in
@@ -116,7 +109,6 @@ struct Params {
   int out_f32;               // element type of out
   int cluster;               // > 1: a tile's K ranges belong to the CTAs of one cluster, added through their shared memory
   int tma_out;               // many tokens: the result leaves through shared memory and TMA stores (adds, when accumulating)
-  int red_out;               // few tokens, accumulating: the K ranges of a tile are separate CTAs whose shares meet in memory (red.add)
   int relu2;                 // a plain bfloat16 result leaves as relu(result)^2
   int gate_relu;             // the gated epilogue's activation: 0 silu, 1 relu, 2 the clamped unit with the constants below, 3 gelu (tanh form)
   float act_limit, act_sharp, act_offset;
@@ -181,11 +173,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   constexpr int kTileFloats = BN * kTileX;                     // one 128-row block of a tile
   constexpr int kBufs = MS == 1 ? 2 : 1;                       // tiles that tensor memory holds
   constexpr int kEpiThreads = 128 * MS;
-  // Few tokens and a cluster: every CTA SENDS the rows of its share to the CTA that owns them
-  // (asynchronous stores that count on the owner's mbarrier), so the owner waits for bytes,
-  // not for the whole cluster, and nobody reads a peer's memory.  Wider token tiles keep the
-  // form in which the owner fetches the shares.
-  constexpr bool kPush = SWAP && BN <= 64;
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // dynamic shared memory is only 16-byte aligned by contract; align by hand
@@ -199,11 +186,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const uint32_t tfull0 = empty0 + 8 * STAGES, tempty0 = tfull0 + 16;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* flags = reinterpret_cast<volatile int*>(bars + 2 * STAGES + 5);   // [0] = failed, [1] = last ticket
-  const uint32_t red_bar = smem_u32(bars + 2 * STAGES + 6);                        // counts the bytes of the shares sent here
-  // [32][64] SwiGLU exchange of whole tiles (swap mode), or the shares sent by the cluster:
-  // [source CTA][gate, up][BN / 4][rows of this CTA][4]
-  float* xch = reinterpret_cast<float*>(bars + 2 * STAGES + 8);
-  const bool push = kPush && p.cluster > 1;
+  float* xch = reinterpret_cast<float*>(bars + 2 * STAGES + 8);     // [32][64] SwiGLU exchange of whole tiles (swap mode)
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -242,10 +225,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, kEpiThreads); }
-    if (push) mbar_init(red_bar, 1);
     flags[0] = 0; flags[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (push) mbar_expect_tx(red_bar, (uint32_t)(kTileX * BN * 4));   // one whole tile's worth of rows arrives here
     // The weight operand depends on no earlier kernel and on no other thread of this CTA:
     // the first ring of weight tiles is requested right here, before tensor memory is
     // allocated and before this kernel waits for its predecessor; the activation tiles of
@@ -270,8 +251,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tcgen05_fence_before();
-  if (push) cluster_sync_all();          // every peer's mbarrier is ready before anything is sent to it
-  else __syncthreads();
+  __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -372,119 +352,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       const bool with_bias = p.bias != nullptr && (kb0 == 0 || !additive);   // once per output: of the ranges that meet in memory, the first adds it
       bool last = whole;
       int c_first = 0, c_last = 0;
-      if (SWAP && !whole && p.red_out) {
-        // Few tokens, accumulating into the 32-bit output: this CTA's K range is added in
-        // memory, where the other ranges of the tile meet it (a 32-bit sum of the same terms
-        // in whatever order they arrive); no cluster, nothing exchanged, nothing waited for.
-        // The share goes through shared memory ([token][row]; the stage ring is idle, every load
-        // into it has been consumed) so that a thread adds four neighbouring features at once.
-        float* red = reinterpret_cast<float*>(smem);
-        const float bv = (p.bias && kb0 == 0 && xr < p.N) ? p.bias[xr] : 0.f;
-        for (int c0 = 0; c0 < BN; c0 += CH) {
-          float v[32];
-          if (CH == 32) tmem_load_32(taddr + c0, v); else tmem_load_16(taddr + c0, v);
-#pragma unroll
-          for (int c = 0; c < CH; ++c) red[(c0 + c) * kTileX + row] = v[c] + bv;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        const bool vec = (p.ldo % 4 == 0) && ((uintptr_t)p.out % 16 == 0) && (x0 + kTileX <= p.N);
-        for (int q = (int)threadIdx.x - 64; q < BN * (kTileX / 4); q += 128) {
-          const int c = q / (kTileX / 4), r4 = (q % (kTileX / 4)) * 4;
-          const int m = y0 + c;
-          if (m >= p.M) break;
-          const float4 val = *reinterpret_cast<const float4*>(red + c * kTileX + r4);
-          float* dst = (float*)p.out + (size_t)m * p.ldo + x0 + r4;
-          if (vec) {
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(val.x), "f"(val.y), "f"(val.z), "f"(val.w) : "memory");
-          } else {
-            const float e[4] = {val.x, val.y, val.z, val.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (x0 + r4 + j < p.N) atomicAdd(dst + j, e[j]);
-          }
-        }
-        break;
-      }
-      if (kPush && !whole && p.cluster > 1) {
-        // The S CTAs of a cluster hold the S consecutive K ranges of one tile.  CTA r owns 1/S
-        // of the tile's rows (of its gate rows and their up rows): every CTA sends the rows of
-        // its share to their owners, [source][gate, up][column / 4][row][4].
-        const int S = p.cluster;
-        const bool sw = p.epilogue == kSwiGLU;
-        const int parts = sw ? 2 : 1;
-        const int rows_per = (sw ? 64 : kTileX) / S;
-        const int rr = sw ? (row & 63) : row;
-        const uint32_t owner = (uint32_t)(rr / rows_per);
-        const int rl = rr % rows_per, part = sw ? (row >> 6) : 0;
-        const uint32_t me = cluster_rank();
-        const uint32_t dst0 = peer_addr(smem_u32(xch) + 16u * (uint32_t)(((int)me * parts + part) * (BN / 4) * rows_per + rl), owner);
-        const uint32_t bar = peer_addr(red_bar, owner);
-        for (int c0 = 0; c0 < BN; c0 += CH) {
-          float v[32];
-          if (CH == 32) tmem_load_32(taddr + c0, v); else tmem_load_16(taddr + c0, v);
-#pragma unroll
-          for (int g = 0; g < CH / 4; ++g)
-            st_peer_v4(dst0 + 16u * (uint32_t)((c0 / 4 + g) * rows_per), bar, v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-        }
-        // ... and adds, in the order of increasing K, the shares of the rows it owns.
-        const int r = (int)me;
-        const int t = (int)threadIdx.x - 64;
-        const int my_rl = t % rows_per;
-        const int my_row = r * rows_per + my_rl;
-        const int n = sw ? (x0 / kTileX) * 64 + my_row : x0 + my_row;       // output feature
-        const int n_end = sw ? p.N / 2 : p.N;
-        const float bv = (p.bias && n < n_end) ? p.bias[n] : 0.f;
-        bool arrived = false;
-        for (int cg = t / rows_per; cg < BN / 4; cg += 128 / rows_per) {
-          float old[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int m = y0 + cg * 4 + j;
-            old[j] = (p.epilogue == kAccumulate && m < p.M && n < n_end) ? __ldcg((const float*)p.out + (size_t)m * p.ldo + n) : 0.f;
-          }
-          if (!arrived) {
-            if (!mbar_wait(red_bar, 0)) { flags[0] = 1; if (p.error_flag) *p.error_flag = 1; break; }
-            arrived = true;
-          }
-          float acc[4] = {0.f, 0.f, 0.f, 0.f}, up[4] = {0.f, 0.f, 0.f, 0.f};
-          const float4* slots = reinterpret_cast<const float4*>(xch);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            if (q < S) {
-              const float4 a = slots[((q * parts) * (BN / 4) + cg) * rows_per + my_rl];
-              acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-              if (sw) {
-                const float4 u = slots[((q * parts + 1) * (BN / 4) + cg) * rows_per + my_rl];
-                up[0] += u.x; up[1] += u.y; up[2] += u.z; up[3] += u.w;
-              }
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int m = y0 + cg * 4 + j;
-            if (m < p.M && n < n_end) {
-              const float val = sw ? gate_mul(p, acc[j], up[j]) : relu2_if(p.relu2, acc[j] + bv + old[j]);
-              const size_t o = (size_t)m * p.ldo + n;
-              if (p.out_f32) ((float*)p.out)[o] = val; else ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(val);
-            }
-          }
-        }
-        // a thread without rows of its own still stays until the shares sent here have landed
-        if (!arrived && !mbar_wait(red_bar, 0)) { flags[0] = 1; if (p.error_flag) *p.error_flag = 1; }
-        break;
-      }
-      if (SWAP && !whole && p.cluster > 1) {
-        // This CTA's share goes to its own shared memory ([col][row]; the stage ring is idle,
-        // every load into it has been consumed); the cluster adds the shares after the roles.
-        float* red = reinterpret_cast<float*>(smem);
-        for (int c0 = 0; c0 < BN; c0 += CH) {
-          float v[32];
-          if (CH == 32) tmem_load_32(taddr + c0, v); else tmem_load_16(taddr + c0, v);
-#pragma unroll
-          for (int c = 0; c < CH; ++c) red[(c0 + c) * kTileX + row] = v[c];
-        }
-        break;
-      }
       const bool peers = !SWAP && !whole && p.cluster > 1;     // many tokens, a tile's K ranges over a cluster
       if (peers) {
         // The sharers of this tile are the CTAs of this cluster.  Each parks its share in its
@@ -829,65 +696,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       cluster_sync_all();                              // nobody leaves while a peer may still read its share
     }
     if (!SWAP && p.tma_out) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // the staging block is read, the stores are done
-  }
-  if (SWAP && p.cluster > 1 && !push) {
-    // The S CTAs of a cluster hold the S consecutive K ranges of one tile.  CTA r adds, in the
-    // order of increasing K, the shares of its 1/S of the tile's rows and writes them out.
-    cluster_sync_all();
-    if (warp >= 2 && flags[0] == 0) {
-      const int S = p.cluster;
-      const int r = (int)cluster_rank();
-      const long long tile = blockIdx.x / S;
-      const int x0 = (int)(tile % p.tiles_x) * kTileX, y0 = (int)(tile / p.tiles_x) * BN;
-      const bool sw = p.epilogue == kSwiGLU;
-      const int rows_per = (sw ? 64 : kTileX) / S;          // rows (gate rows) of this CTA
-      const int t = threadIdx.x - 64;
-      const int row = r * rows_per + t % rows_per;
-      const int cstep = 128 / rows_per;
-      const int n = sw ? (x0 / kTileX) * 64 + row : x0 + row;   // output feature
-      const int n_end = sw ? p.N / 2 : p.N;
-      const float bv = (p.bias && n < n_end) ? p.bias[n] : 0.f;
-      constexpr int kCols = 4;                                  // columns a thread has in flight
-      for (int cb = t / rows_per; cb < BN; cb += cstep * kCols) {
-        float acc[kCols], up[kCols], old[kCols];
-#pragma unroll
-        for (int j = 0; j < kCols; ++j) {
-          const int m = y0 + cb + j * cstep;
-          acc[j] = 0.f; up[j] = 0.f;
-          old[j] = (p.epilogue == kAccumulate && cb + j * cstep < BN && m < p.M && n < n_end)
-                       ? __ldcg((const float*)p.out + (size_t)m * p.ldo + n) : 0.f;
-        }
-        // every peer's share is requested before the first is used; the sums run in K order
-        for (int part = 0; part < (sw ? 2 : 1); ++part) {
-          float share[8][kCols];
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-#pragma unroll
-            for (int j = 0; j < kCols; ++j) {
-              const int c = cb + j * cstep;
-              share[q][j] = (q < S && c < BN)
-                                ? ld_peer_f32(base + (uint32_t)(c * kTileX + part * 64 + row) * 4u, (uint32_t)q) : 0.f;
-            }
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-#pragma unroll
-            for (int j = 0; j < kCols; ++j) {
-              if (part == 0) acc[j] += share[q][j]; else up[j] += share[q][j];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kCols; ++j) {
-          const int c = cb + j * cstep, m = y0 + c;
-          if (c < BN && m < p.M && n < n_end) {
-            const float g = acc[j];
-            const float v = sw ? gate_mul(p, g, up[j]) : relu2_if(p.relu2, g + bv + old[j]);
-            const size_t o = (size_t)m * p.ldo + n;
-            if (p.out_f32) ((float*)p.out)[o] = v; else ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(v);
-          }
-        }
-      }
-    }
-    cluster_sync_all();                  // nobody leaves while a peer may still read its shares
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -1236,13 +1044,14 @@ int sm_count() {
   return n;
 }
 
-// Ring, alignment slack, barriers and flags, then the exchange area: the whole-tile SwiGLU
-// exchange, or (`sent`) the shares that the CTAs of a cluster send here.
+#include "gemm_few.cuh"
+
+// Ring, alignment slack, barriers and flags, then (few tokens) the whole-tile SwiGLU exchange.
 template <int BN, int STAGES, bool SWAP, int MS = 1>
-constexpr size_t smem_bytes(bool sent = true) {
+constexpr size_t smem_bytes() {
   return (size_t)STAGES * (MS * kTileX * kBlockK * 2 + BN * kBlockK * 2) + 1024 + (2 * STAGES + 8) * 8 +
          (SWAP ? 0 : MS * kTileX * 128) +       // many tokens: the staging block of each row block
-         (SWAP ? (sent && BN <= 64 && kTileX * BN * 4 > 32 * 64 * 4 ? kTileX * BN * 4 : 32 * 64 * 4) : 0);
+         (SWAP ? 32 * 64 * 4 : 0);
 }
 
 template <int BN, int STAGES, bool SWAP, int MS = 1>
@@ -1282,18 +1091,9 @@ int active_clusters(int split) {
   return n > 0 ? n : 0;
 }
 
-int active_clusters_for(int bn, int split) {
-  switch (bn) {
-    case 16: return active_clusters<16, 5, true>(split);
-    case 32: return active_clusters<32, 4, true>(split);
-    case 64: return active_clusters<64, 3, true>(split);
-    default: return active_clusters<128, 3, true>(split);
-  }
-}
-
 template <int BN, int STAGES, bool SWAP, int MS = 1>
 int launch(const CUtensorMap& mx, const CUtensorMap& my, const CUtensorMap& mo, const Params& p, int grid, cudaStream_t stream) {
-  const size_t smem = smem_bytes<BN, STAGES, SWAP, MS>(p.cluster > 1);
+  const size_t smem = smem_bytes<BN, STAGES, SWAP, MS>();
   if (configure<BN, STAGES, SWAP, MS>()) return -1;
   ilb::launch_cluster(gemm_tc_kernel<BN, STAGES, SWAP, MS>, dim3(grid), dim3(threads_for(MS)), smem, stream, p.cluster, mx, my, mo, p);
   return check_launch("gemm_tc");
@@ -1310,8 +1110,6 @@ ILB_EXPORT long long ilb_gemm_tc_workspace_floats() {
 }
 ILB_EXPORT int ilb_gemm_tc_max_tickets() { return 1 << 16; }
 
-// Clusters of `split` CTAs of the decode kernel for token tiles of `bn` that fit the device at once.
-ILB_EXPORT int ilb_gemm_tc_active_clusters(int bn, int split) { return active_clusters_for(bn, split); }
 // What the kernel can take: bf16 operands, K and the leading dimensions multiples of 8
 // (16-byte rows for TMA), 16-byte aligned bases.
 ILB_EXPORT int ilb_gemm_tc_supported(int M, int N, int K, int lda, int ldw) {
@@ -1326,12 +1124,10 @@ struct Plan { bool swap, tail, additive; int bn, ms, x_rows, y_rows; long long g
 // Whether the K ranges of a tile may meet in memory (the sum's order is then not fixed: runs
 // agree beyond rounding, not bit for bit).  `ilb_gemm_tc_sums_in_memory(0)` turns it off.
 bool g_sums_in_memory = true;
-// Accumulating products of up to this many tokens, with a weight of at least 2,048 x 2,048, add
-// the K ranges of a tile in memory (separate CTAs, red.add) instead of inside a cluster.  In a
-// decode step of Qwen3-8B sizes, one 32-bit value per add: batch 1 3.41 -> 3.31 ms, batch 2
-// 3.44 -> 3.36, batch 4 3.51 -> 3.47, but batch 8 3.62 -> 3.70 and batch 16 3.92 -> 4.26 (the
-// adds are paid per lane); four neighbouring features per add (the share transposed through
-// shared memory): batch 1 3.29, batch 4 3.43, batch 8 3.52 ms.
+// Accumulating products of up to this many tokens, with a weight of at least 2,048 x 2,048, add the K ranges of a tile in
+// memory (separate CTAs, red.add) instead of inside a cluster, which fixes the order (4,096 x 4,096 at 8 tokens 7.2 against
+// 8.6 us, 4,096 x 12,288 16.9 against 18.5); so do 65 to 128 tokens into a wide output (9.6 against 12.9, 20.1 against 24.6).
+// In between the order stays fixed.
 int g_red_few_tokens = 8;
 int g_red_few_split = 8;
 
@@ -1346,26 +1142,10 @@ long long add_split(long long rest, long long k_blocks) {
 // `can_add`: the product accumulates into a 32-bit output that the TMA write-out can reach,
 // so that the K ranges of a tile may be added in memory.
 int make_plan(Params& p, int M, int N, int K, int accumulate, int n_tickets, int max_ctas, bool can_add, Plan& plan) {
-  // 65 to 128 tokens of a product that accumulates into a wide 32-bit output: tokens on the
-  // MMA's rows after all, 128 x 256 tiles cut into equal K ranges that meet in memory.  With
-  // the weight on the rows the K ranges of a tile are a cluster that exchanges 32-bit shares;
-  // here nothing is exchanged (4,096 x 4,096 at 128 tokens 16.4 -> 12.7 us, 5,120 x 25,600 at
-  // 64 tokens 56.0 -> 46.3 us alone; but inside a decode step, between its neighbours, the
-  // weight on the rows stays ahead up to 64 tokens: 5.86 against 5.90 ms at batch 64, and
-  // 8.35 against 7.86 ms at batch 96).
-  bool few_in_memory = false;
-  if (M > 64 && M <= 128 && can_add && accumulate == 1 && g_sums_in_memory && max_ctas <= 0 && N >= 3072) {
-    const long long t = (N + 255) / 256, kb = (K + kBlockK - 1) / kBlockK;
-    const long long rest = t % sm_count();
-    few_in_memory = rest != 0 && t * 12 >= sm_count() && add_split(rest, kb) >= 2;
-  }
-  const bool swap = M <= 128 && !few_in_memory;
+  const bool swap = M <= 128;
   bool tail = false;
   int bn, ms = 1;                                    // ms: 128-row blocks of X per tile
-  if (few_in_memory) {
-    bn = 256;
-    tail = true;
-  } else if (swap) {
+  if (swap) {
     bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   } else {
     // Many tokens: the tile shape that keeps the most SMs busy in whole rounds, larger tiles
@@ -1431,34 +1211,12 @@ int make_plan(Params& p, int M, int N, int K, int accumulate, int n_tickets, int
   const long long tiles = (long long)p.tiles_x * p.tiles_y;
   ILB_REQUIRE(tiles <= n_tickets, "gemm_tc: %lld output tiles exceed the %d tickets", tiles, n_tickets);
 
-  // Decode shapes (swap): two CTAs per SM (the rings are sized for it), one streams while
-  // the other is in its prologue or epilogue.  When the tiles are fewer than the CTAs that
-  // fit, every tile is cut into the same number of K ranges (at most 8), so that no CTA
-  // straddles two tiles; otherwise the persistent grid takes contiguous runs of units.
+  // Decode shapes (swap; a weight too wide for one round of `gemm_few_kernel`, the output matrix): two CTAs per SM (the rings
+  // are sized for it), one streams while the other is in its prologue or epilogue; the persistent grid takes contiguous
+  // runs of units.
   const long long cap = swap ? 2ll * sm_count() : sm_count();
   long long grid = cap;
   p.cluster = 1;
-  if (swap && tiles <= cap && max_ctas <= 0) {
-    // every tile is cut into 1, 2, 4 or 8 K ranges, one per CTA of a cluster that adds them
-    // through shared memory: no workspace round trip and no tickets
-    long long split = 1;
-    while (split < 8 && tiles * split * 2 <= cap && split * 2 <= p.k_blocks) split *= 2;
-    // All clusters resident at once, or the stragglers cost a second round.  The occupancy
-    // query counts one CTA of this kernel per SM; the small rings run two per SM, and then a
-    // cluster of `split` CTAs takes the SMs of a cluster of split / 2.
-    const bool two_per_sm = true;
-    while (split > 1 && active_clusters_for(bn, (int)(two_per_sm ? split / 2 : split)) < tiles) split /= 2;
-    grid = tiles * split;
-    p.cluster = (int)split;
-    if (can_add && g_sums_in_memory && accumulate == 1 && M <= g_red_few_tokens && split > 1 && N >= 2048 && K >= 2048) {
-      // the ranges as separate CTAs that add into the output (as many as the cluster would have held, or more)
-      long long s = split;
-      while (s < g_red_few_split && tiles * s * 2 <= cap && s * 2 <= p.k_blocks) s *= 2;
-      grid = tiles * s;
-      p.cluster = 1;
-      p.red_out = 1;
-    }
-  }
   if (!swap && max_ctas <= 0) {
     // Many tokens.  Tiles that share an operand block must want it at the same time, or every
     // CTA streams its own copy from memory: whole tiles in rounds of equal size, all CTAs
@@ -1588,6 +1346,43 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const CUtensorMap&
   return check_launch("gemm_tc");
 }
 
+// Whether (and into how many ranges at most) a product of few tokens may add the K ranges of a tile in memory.
+int few_ranges_in_memory(int M, int N, int K, bool can_add) {
+  if (!can_add || !g_sums_in_memory) return 1;
+  if (M <= g_red_few_tokens) return N >= 2048 && K >= 2048 ? g_red_few_split : 1;
+  return M > 64 && N >= 3072 && K >= 512 ? 8 : 1;
+}
+
+int epilogue_of(int mode, Params& p) {
+  // 3 from the caller: the gated epilogue with relu as the gate's activation (else silu); 4: the clamped gated unit
+  // 5: a plain product whose bfloat16 result leaves as relu(result)^2; 6: the gated epilogue with gelu's tanh form
+  p.relu2 = mode == 5 ? 1 : 0;
+  p.gate_relu = mode == 3 ? 1 : (mode == 4 ? 2 : (mode == 6 ? 3 : 0));
+  return mode == 5 ? kStore : (mode >= 3 ? kSwiGLU : mode);
+}
+
+int check_epilogue(int mode, const void* out, int out_f32, int N, int ldo, const float* bias, float act_limit) {
+  ILB_REQUIRE(out != nullptr && mode >= 0 && mode <= 6, "gemm_tc: unknown epilogue %d", mode);
+  ILB_REQUIRE(mode != 5 || !out_f32, "gemm_tc: relu squared belongs to a bfloat16 result");
+  ILB_REQUIRE(mode != 4 || act_limit > 0.f, "gemm_tc: the clamped unit needs a positive limit");
+  ILB_REQUIRE(mode != 1 || out_f32, "gemm_tc: accumulation needs a 32-bit output");
+  if (mode >= 2 && mode != 5) {
+    ILB_REQUIRE(N % 128 == 0 && bias == nullptr, "gemm_tc: the SwiGLU epilogue needs N (%d) a multiple of 128 and no bias", N);
+    ILB_REQUIRE(ldo >= N / 2, "gemm_tc: output leading dimension too small");
+  } else {
+    ILB_REQUIRE(ldo >= N, "gemm_tc: output leading dimension too small");
+  }
+  return 0;
+}
+
+FewParams few_params(const Params& p) {
+  FewParams q{};
+  q.out = p.out; q.bias = p.bias; q.error_flag = p.error_flag; q.T = p.M; q.N = p.N; q.K = p.K; q.ldo = p.ldo;
+  q.epilogue = p.epilogue; q.out_f32 = p.out_f32; q.relu2 = p.relu2; q.gate_relu = p.gate_relu;
+  q.act_limit = p.act_limit; q.act_sharp = p.act_sharp; q.act_offset = p.act_offset;
+  return q;
+}
+
 }  // namespace
 
 // max_ctas > 0 sets the grid (tests use it to force many shared tiles).
@@ -1599,37 +1394,28 @@ ILB_EXPORT int ilb_gemm_tc(const void* A, const void* W, const float* bias, void
   ILB_REQUIRE(K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0,
               "gemm_tc: K (%d) and the leading dimensions (%d, %d) must be multiples of 8", K, lda, ldw);
   ILB_REQUIRE(((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0), "gemm_tc: operands must be 16-byte aligned");
-  // 3 from the caller: the gated epilogue with relu as the gate's activation (else silu); 4: the clamped gated unit
-  // 5: a plain product whose bfloat16 result leaves as relu(result)^2; 6: the gated epilogue with gelu's tanh form
-  const int relu2 = accumulate == 5 ? 1 : 0;
-  if (relu2) accumulate = kStore;
-  ILB_REQUIRE(!relu2 || !out_f32, "gemm_tc: relu squared belongs to a bfloat16 result");
-  const int gate_relu = accumulate == 3 ? 1 : (accumulate == 4 ? 2 : (accumulate == 6 ? 3 : 0));
-  if (gate_relu) accumulate = kSwiGLU;
-  ILB_REQUIRE(gate_relu != 2 || act_limit > 0.f, "gemm_tc: the clamped unit needs a positive limit");
-  ILB_REQUIRE(accumulate >= 0 && accumulate <= 2, "gemm_tc: unknown epilogue %d", accumulate);
-  ILB_REQUIRE(accumulate != 1 || out_f32, "gemm_tc: accumulation needs a 32-bit output");
-  if (accumulate == 2) {
-    ILB_REQUIRE(N % 128 == 0 && bias == nullptr, "gemm_tc: the SwiGLU epilogue needs N (%d) a multiple of 128 and no bias", N);
-    ILB_REQUIRE(ldo >= N / 2, "gemm_tc: output leading dimension too small");
-  } else {
-    ILB_REQUIRE(ldo >= N, "gemm_tc: output leading dimension too small");
-  }
+  if (check_epilogue(accumulate, out, out_f32, N, ldo, bias, act_limit)) return -1;
   ILB_REQUIRE(workspace != nullptr && tickets != nullptr, "gemm_tc: workspace and tickets are required");
 
   Params p{};
   p.out = out; p.bias = bias; p.partial = workspace; p.tickets = tickets; p.error_flag = error_flag;
   p.M = M; p.N = N; p.K = K; p.ldo = ldo;
   p.k_blocks = (K + kBlockK - 1) / kBlockK;
-  p.epilogue = accumulate;
+  p.epilogue = accumulate = epilogue_of(accumulate, p);
   p.out_f32 = out_f32;
-  p.relu2 = relu2;
-  p.gate_relu = gate_relu; p.act_limit = act_limit; p.act_sharp = act_sharp; p.act_offset = act_offset;
+  const int relu2 = p.relu2, gate_relu = p.gate_relu;
+  p.act_limit = act_limit; p.act_sharp = act_sharp; p.act_offset = act_offset;
 
   Plan plan{};
   const int es = out_f32 ? 4 : 2, out_cols = accumulate == 2 ? N / 2 : N;
   const bool tma_reach = ((uintptr_t)out % 16 == 0) && ((long long)ldo * es) % 16 == 0;   // rows of 16-byte multiples from a 16-byte base
-  if (make_plan(p, M, N, K, accumulate, n_tickets, max_ctas, tma_reach && out_f32 && accumulate == 1, plan)) return -1;
+  const bool can_add = tma_reach && out_f32 && accumulate == 1;
+  FewPlan few;
+  if (max_ctas <= 0 && few_plan(M, N, K, few_ranges_in_memory(M, N, K, can_add), few)) {
+    FewParams q = few_params(p);
+    return run_few(q, few, A, lda, W, ldw, stream);
+  }
+  if (make_plan(p, M, N, K, accumulate, n_tickets, max_ctas, can_add, plan)) return -1;
   const bool swap = plan.swap;
   // Many tokens: a pair of CTAs per 256 x 256 tile where the result can leave by TMA.
   if (!swap && g_pairs != 0 && max_ctas <= 0 && tma_reach && !(accumulate == 2 && out_f32)) {
@@ -1672,8 +1458,7 @@ ILB_EXPORT int ilb_gemm_tc(const void* A, const void* W, const float* bias, void
     switch (bn) {
       case 16: return launch<16, 5, true>(mx, my, mo, p, (int)grid, stream);
       case 32: return launch<32, 4, true>(mx, my, mo, p, (int)grid, stream);
-      // the shares sent to a CTA take the room of a stage: a shallower ring for clusters only
-      case 64: return p.cluster > 1 ? launch<64, 3, true>(mx, my, mo, p, (int)grid, stream) : launch<64, 4, true>(mx, my, mo, p, (int)grid, stream);
+      case 64: return launch<64, 4, true>(mx, my, mo, p, (int)grid, stream);
       default: return launch<128, 3, true>(mx, my, mo, p, (int)grid, stream);
     }
   }
@@ -1685,6 +1470,29 @@ ILB_EXPORT int ilb_gemm_tc(const void* A, const void* W, const float* bias, void
   if (bn == 256) return launch<256, 4, false>(mx, my, mo, p, (int)grid, stream);
   return launch<128, 6, false>(mx, my, mo, p, (int)grid, stream);
 }
+
+// The same product with A = the RMS norm (weight norm_w, 32-bit) of the 32-bit rows x [M, K], up to 16 of them, in one launch.
+ILB_EXPORT int ilb_gemm_tc_normed(const float* x, const float* norm_w, float eps, const void* W, const float* bias, void* out, int out_f32,
+                                  int M, int N, int K, int ldx, int ldw, int ldo, int mode, int* error_flag, float act_limit,
+                                  float act_sharp, float act_offset, cudaStream_t stream) {
+  ILB_REQUIRE(M > 0 && M <= kFewNormTokens && N > 0 && K > 0, "gemm_tc_normed: bad sizes M=%d N=%d K=%d", M, N, K);
+  ILB_REQUIRE(K % 8 == 0 && ldw % 8 == 0 && ldx % 4 == 0 && ldx >= K && ldw >= K, "gemm_tc_normed: K (%d) and the weight's leading dimension (%d) must be multiples of 8, the rows' (%d) of 4", K, ldw, ldx);
+  ILB_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)norm_w % 16 == 0) && ((uintptr_t)W % 16 == 0), "gemm_tc_normed: operands must be 16-byte aligned");
+  ILB_REQUIRE(x != nullptr && norm_w != nullptr && W != nullptr && eps > 0.f && mode != 1, "gemm_tc_normed: missing operands, or an accumulating product");
+  if (check_epilogue(mode, out, out_f32, N, ldo, bias, act_limit)) return -1;
+  Params p{};
+  p.out = out; p.bias = bias; p.error_flag = error_flag; p.M = M; p.N = N; p.K = K; p.ldo = ldo; p.out_f32 = out_f32;
+  p.epilogue = epilogue_of(mode, p);
+  p.act_limit = act_limit; p.act_sharp = act_sharp; p.act_offset = act_offset;
+  FewPlan few;
+  ILB_REQUIRE(few_plan(M, N, K, 1, few), "gemm_tc_normed: a weight of %d rows is not served", N);
+  FewParams q = few_params(p);
+  q.x = x; q.ldx = ldx; q.norm_w = norm_w; q.eps = eps;
+  return run_few(q, few, nullptr, 0, W, ldw, stream);
+}
+ILB_EXPORT int ilb_gemm_tc_normed_tokens() { return kFewNormTokens; }
+// Weights of more rows than this are not served by the kernel of few tokens.
+ILB_EXPORT int ilb_gemm_tc_few_rows() { return 256 * 2 * sm_count(); }
 
 // Products of many tokens on pairs of CTAs: 0 never, 1 where the sizes favour it, 2 wherever possible.
 ILB_EXPORT int ilb_gemm_tc_pairs(int mode) {
@@ -1724,11 +1532,18 @@ ILB_EXPORT int ilb_gemm_tc_plan(int M, int N, int K, int epilogue, int* out) {
   ILB_REQUIRE(M > 0 && N > 0 && K > 0 && out != nullptr && epilogue >= 0 && epilogue <= 2, "gemm_tc: bad sizes for a plan");
   Params p{};
   p.M = M; p.N = N; p.K = K; p.k_blocks = (K + kBlockK - 1) / kBlockK; p.epilogue = epilogue;
+  FewPlan few;
+  if (few_plan(M, N, K, few_ranges_in_memory(M, N, K, epilogue == 1), few)) {
+    // (65 to 128 tokens whose ranges meet in memory are reported as a product of many tokens, which also let them meet there)
+    out[0] = M <= 64 || !few.red; out[1] = (M + 7) / 8 * 8; out[2] = 1; out[3] = few.grid; out[4] = few.cluster;
+    out[5] = 0; out[6] = few.tiles; out[7] = few.red ? few.tiles : 0; out[8] = few.red; out[9] = 0; out[10] = 0;
+    return 0;
+  }
   Plan plan{};
   if (make_plan(p, M, N, K, epilogue, 1 << 30, 0, epilogue == 1, plan)) return -1;
   out[0] = plan.swap ? 1 : 0; out[1] = plan.bn; out[2] = plan.ms; out[3] = (int)plan.grid; out[4] = p.cluster;
   out[5] = p.dp_waves; out[6] = p.tiles_x * p.tiles_y; out[7] = (int)(p.tiles_x * (long long)p.tiles_y - p.sk_tile0);
-  out[8] = (plan.additive || p.red_out) ? 1 : 0;
+  out[8] = plan.additive ? 1 : 0;
   out[9] = 0; out[10] = 0;
   PairPlan pp{};
   if (!plan.swap && g_pairs != 0 && pair_plan(M, N, K, epilogue == 1 && g_sums_in_memory, pair_capacity(), pp) &&

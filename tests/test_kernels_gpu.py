@@ -578,6 +578,39 @@ def test_gemm_tcgen05_few_tokens_add_their_ranges_in_memory(M, N, K, bias):
     o.check_device_errors()
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 40, 64, 65, 128])
+@pytest.mark.parametrize("N,K,form", [(6144, 512, "bias"), (1000, 264, "bias"), (72, 8, "bias"), (3072, 2048, "accumulate"), (515, 1096, "accumulate"),
+                                      (1280, 4096, "accumulate"), (2304, 136, "swiglu"), (1408, 2048, "swiglu"), (24576, 192, "swiglu"),
+                                      (328, 320, "relu2")])
+def test_gemm_tcgen05_few_tokens_over_tiles_and_ranges(M, N, K, form):
+    """Up to 128 tokens: tiles of any multiple of 16 rows, so that a tile of gated weights begins and ends inside a block of 64
+    and the last tile of every width is ragged; whole tiles, ranges in a cluster and ranges that meet in memory; a depth
+    that ends inside a block of 64; outputs whose rows are no multiple of 16 bytes, or whose base is not (what lies around
+    them stays)."""
+    o = ops()
+    torch.manual_seed(M + N + K)
+    a = torch.randn(M, K).to(torch.bfloat16)
+    w = (torch.randn(N, K) * 0.05).to(torch.bfloat16)
+    b = torch.randn(N) if form in ("bias", "accumulate") else None
+    ref = a.double() @ w.double().T + (b.double() if b is not None else 0)
+    cols = N
+    if form == "swiglu":
+        g = ref.view(M, N // 128, 2, 64)
+        ref, cols = (torch.nn.functional.silu(g[:, :, 0]) * g[:, :, 1]).reshape(M, N // 2), N // 2
+    elif form == "relu2":
+        ref = torch.relu(ref) ** 2
+    for offset in (0, 3):
+        dtype = torch.float32 if form == "accumulate" else torch.bfloat16
+        whole = torch.randn(M * cols + 8).to(dtype).cuda()
+        out = whole[offset:offset + M * cols].view(M, cols)
+        before = whole.clone()
+        want = ref + out.double().cpu() if form == "accumulate" else ref
+        o.gemm_tc(a.cuda(), w.cuda(), out, None if b is None else b.cuda(), accumulate=form == "accumulate", swiglu=form == "swiglu", relu2=form == "relu2")
+        o.check_device_errors()
+        close(out, want, "float32" if dtype == torch.float32 else "bfloat16", scale=float(ref.abs().max()), what=f"few tokens {M}x{N}x{K} {form} +{offset}")
+        assert torch.equal(whole[:offset], before[:offset]) and torch.equal(whole[offset + M * cols:], before[offset + M * cols:])
+
+
 def test_gemm_tuning_knobs_move_the_plan():
     """The knobs behind the measured defaults: how many tokens send their K ranges to memory,
     and how many ranges a tile of a pair may be cut into."""
