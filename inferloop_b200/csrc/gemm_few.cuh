@@ -1,6 +1,5 @@
 // bfloat16 products of up to 128 tokens, included by gemm_tcgen05.cu (whose helpers it uses):
-//     out[T, N] (+)= A[T, K] * W[N, K]^T (+ bias), or the gated unit over interleaved gate and up rows,
-// where A is given, or is the RMS norm of 32-bit rows that the kernel reads itself.
+//     out[T, N] (+)= A[T, K] * W[N, K]^T (+ bias), or the gated unit over interleaved gate and up rows.
 //
 // What bounds it: the weight is read once, so the floor is its bytes at the copy rate.  Three things kept the
 // former deal (128 weight rows on the MMA's rows, one or two tiles to an SM) away from it: tiles of one height
@@ -25,15 +24,12 @@
 //              idle ring so that a thread holds four neighbouring outputs; the ranges of a tile that must be added
 //              in K order are the CTAs of a cluster, which send each other their shares (st.async on the owner's
 //              mbarrier), chunk j of 16 columns belonging to CTA j % split.
-// Norm inside (TT > 0): out = (x * w) W^T / rms(x), and the root mean square is a factor of the row that can be
-// applied to the 32-bit result.  So warps 2-9 read the 32-bit rows, multiply by the norm's weight, round to
-// bfloat16 (one rounding, as the norm's own kernel has) and lay them out as the MMA wants them, a block at a
-// time ahead of the weight stream, with the sums of squares beside.  A launch and its wait fall away (1.7 us) for
-// 0.3 to 0.8 us in the product.  Every CTA reads the rows again: at 16 tokens of 4,096 x 24,576 33.7 -> 34.3 us,
-// at 24 tokens of 5,120 x 34,816 54.8 -> 58.3 us, more than the norm's launch; so up to 16 tokens.
+// (Tried and taken back: the RMS norm in front of a product of up to 16 tokens inside it, warps 2-9 reading the 32-bit rows, laying
+// them out ahead of the stream and leaving the root mean square to the result.  Launch after launch it took 0.3 to 0.8 us where the
+// norm's launch takes 1.7; in a step, where that launch hides behind its neighbours, 8B sizes lost 3 % at one token.)
 // All mbarrier waits are bounded, as in the other kernels.
 
-constexpr int kFewTokens = 128, kFewNormTokens = 16;
+constexpr int kFewTokens = 128;
 constexpr int kFewWarps = 8, kFewEpi = 32 * kFewWarps, kFewThreads = 64 + kFewEpi;
 constexpr int kFewStages = 12;
 // Two CTAs to an SM: 228 KB less 1 KB each that the system keeps, halved.
@@ -43,21 +39,17 @@ struct FewParams {
   void* out;
   const float* bias;
   int* error_flag;
-  const float* x;            // NORM: the 32-bit rows [T, K] the product takes normed, and the norm's weight
-  const float* norm_w;
-  float eps;
-  int T, N, K, ldo, ldx;
+  int T, N, K, ldo;
   int rows, tp, k_blocks, split, cluster, stages, tmem_cols, red;
   int stage_bytes, ring_bytes, recv_bytes;
   int epilogue, out_f32, relu2, gate_relu;
   float act_limit, act_sharp, act_offset;
 };
 
-// TT: tokens the norm's threads may have to look after (0: the product reads its rows as they are).
-template <int MM, int TT>
+// MM: rows of the MMA, 64 or 128.
+template <int MM>
 __global__ void __launch_bounds__(kFewThreads, 2)
 gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_y, const FewParams p) {
-  constexpr bool NORM = TT > 0;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - smem_u32(smem_raw));
@@ -66,7 +58,6 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kFewStages, tfull = empty0 + 8 * kFewStages, rbar = tfull + 8;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * kFewStages + 2);
   volatile int* failed = reinterpret_cast<volatile int*>(bars + 2 * kFewStages + 3);
-  float* ssq = reinterpret_cast<float*>(bars + 2 * kFewStages + 4);      // NORM: [warps][tokens] partial sums; then [tokens]
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -76,7 +67,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   const int row0 = tile * p.rows;
   const int n_early = cnt < p.stages ? cnt : p.stages;
   const uint32_t w_off = (uint32_t)p.tp * 128u;
-  const uint32_t tx = (uint32_t)(p.rows + (NORM ? 0 : p.tp)) * 128u;
+  const uint32_t tx = (uint32_t)(p.rows + p.tp) * 128u;
   const int boxes = gated ? p.rows / 16 : 1;
   auto load_w = [&](uint32_t dst, uint32_t bar, int kcol) {
     if (gated) {
@@ -91,7 +82,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int s = 0; s < p.stages; ++s) { mbar_init(full0 + 8 * s, NORM ? 2 : 1); mbar_init(empty0 + 8 * s, 1); }
+      for (int s = 0; s < p.stages; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
       mbar_init(tfull, 1);
       if (p.cluster > 1) mbar_init(rbar, 1);
       *failed = 0;
@@ -99,7 +90,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       if (p.cluster > 1) {
         const int nch = p.rows / 16, me = part;
         const int nloc = (nch - me + p.split - 1) / p.split;
-        mbar_expect_tx(rbar, (uint32_t)(p.split * nloc * p.T * 64 + (NORM ? p.split * ((p.T + 3) / 4) * 16 : 0)));
+        mbar_expect_tx(rbar, (uint32_t)(p.split * nloc * p.T * 64));
       }
       for (int it = 0; it < n_early; ++it) mbar_expect_tx(full0 + 8 * it, tx);
     }
@@ -117,11 +108,9 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
   if (warp == 0) {
     bool ok = true;
-    if (!NORM) {
-      pdl_wait();
-      if (lane == 0)
-        for (int it = 0; it < n_early; ++it) tma_load_2d(base + it * p.stage_bytes, &map_y, full0 + 8 * it, (kb0 + it) * kBlockK, 0);
-    }
+    pdl_wait();
+    if (lane == 0)
+      for (int it = 0; it < n_early; ++it) tma_load_2d(base + it * p.stage_bytes, &map_y, full0 + 8 * it, (kb0 + it) * kBlockK, 0);
     int s = n_early == p.stages ? 0 : n_early;
     uint32_t ph = 0;
     int armed = n_early;
@@ -131,7 +120,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       const uint32_t dst = base + s * p.stage_bytes;
       if (lane == 0) {
         mbar_expect_tx(full0 + 8 * s, tx);
-        if (!NORM) tma_load_2d(dst, &map_y, full0 + 8 * s, (kb0 + it) * kBlockK, 0);
+        tma_load_2d(dst, &map_y, full0 + 8 * s, (kb0 + it) * kBlockK, 0);
       }
       __syncwarp();
       load_w(dst, full0 + 8 * s, (kb0 + it) * kBlockK);
@@ -165,62 +154,6 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   } else {
     const int et = threadIdx.x - 64, ew = warp - 2;
     pdl_wait();
-    if (NORM) {
-      // ---- the rows: norm weight applied, rounded to bfloat16 and laid out as the MMA reads them, sums of squares beside
-      constexpr int kPer = TT > 0 ? TT / 2 : 1;              // tokens of a lane
-      float sq[kPer];
-#pragma unroll
-      for (int i = 0; i < kPer; ++i) sq[i] = 0.f;
-      const int half = lane >> 4, c = lane & 15;
-      bool ok = true;
-      // A stage belongs to one warp: it sees every phase of the stage's barrier (a parity tells two neighbouring phases apart, no more).
-      int s = ew, round = 0;
-      for (int it = ew; ok; ) {
-        if (s >= p.stages) { s = ew; ++round; if (s >= p.stages) break; }
-        it = round * p.stages + s;
-        if (it >= cnt) break;
-        const int k = (kb0 + it) * kBlockK + c * 4;
-        const bool in_k = k < p.K;                            // (K is a multiple of 8)
-        const float4 w = in_k ? *reinterpret_cast<const float4*>(p.norm_w + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 v[kPer];
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-          const int t = 2 * i + half;
-          v[i] = (t < p.T && in_k) ? __ldcg(reinterpret_cast<const float4*>(p.x + (size_t)t * p.ldx + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        if (round > 0) ok = mbar_wait(empty0 + 8 * s, (round - 1) & 1);
-        const uint32_t dst = base + s * p.stage_bytes;
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-          const int t = 2 * i + half;
-          if (t < p.T) {
-            sq[i] = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, sq[i]))));
-            const uint32_t lo = pack_bf16(v[i].x * w.x, v[i].y * w.y), hi = pack_bf16(v[i].z * w.z, v[i].w * w.w);
-            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + (uint32_t)t * 128u + (uint32_t)((((c >> 1) ^ (t & 7)) << 4) | ((c & 1) << 3))), "r"(lo), "r"(hi) : "memory");
-          }
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(full0 + 8 * s);
-        s += kFewWarps;
-      }
-      if (!ok) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
-#pragma unroll
-      for (int i = 0; i < kPer; ++i) {
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
-        if (c == 0) ssq[ew * TT + 2 * i + half] = sq[i];
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(kFewEpi) : "memory");
-      float total = 0.f;
-      if (et < TT) {
-#pragma unroll
-        for (int w = 0; w < kFewWarps; ++w) total += ssq[w * TT + et];
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(kFewEpi) : "memory");
-      if (et < TT) ssq[et] = p.cluster > 1 ? total : rsqrtf(total / (float)p.K + p.eps);
-      asm volatile("bar.sync 1, %0;" ::"n"(kFewEpi) : "memory");
-    }
     const int quad = warp & 3, hf = ew >> 2;
     const int t = MM == 128 ? quad * 32 + lane : quad * 16 + lane;
     const bool warp_on = (MM == 128 ? quad * 32 : quad * 16) < p.T;
@@ -232,14 +165,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const bool bad = *failed != 0;
     if (p.cluster > 1) {
       // ---- the K ranges of a tile are the CTAs of a cluster: chunk j of 16 columns belongs to CTA j % split
-      const int nmax = (nch + p.split - 1) / p.split;
       const uint32_t recv_addr = smem_u32(recv);
-      const uint32_t sums_off = (uint32_t)(p.split * nmax * p.T) * 64u;
-      if (NORM && et < (p.T + 3) / 4) {
-        const float4 v = *reinterpret_cast<const float4*>(ssq + 4 * et);
-        for (int q = 0; q < p.split; ++q)
-          st_peer_v4(peer_addr(recv_addr + sums_off + (uint32_t)(part * ((p.T + 3) / 4) + et) * 16u, q), peer_addr(rbar, q), v.x, v.y, v.z, v.w);
-      }
       if (warp_on) {
         for (int j = hf; j < nch; j += 2) {
           float v[32];
@@ -290,7 +216,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           if (jl >= nl) continue;
           const int chunk = jl * p.split + part;
           const int n = gated ? row0 / 2 + chunk * 8 + c4 * 4 : row0 + chunk * 16 + c4 * 4;
-          float a[4] = {0.f, 0.f, 0.f, 0.f}, up[4] = {0.f, 0.f, 0.f, 0.f}, total = 0.f;
+          float a[4] = {0.f, 0.f, 0.f, 0.f}, up[4] = {0.f, 0.f, 0.f, 0.f};
           for (int z = 0; z < p.split; ++z) {
             const float* src = recv + (size_t)((z * nl + jl) * p.T + tt) * 16;
             const float4 s4 = *reinterpret_cast<const float4*>(src + ((c4 ^ ((tt >> 1) & 3)) << 2));
@@ -299,12 +225,6 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
               const float4 u4 = *reinterpret_cast<const float4*>(src + (((c4 + 2) ^ ((tt >> 1) & 3)) << 2));
               up[0] += u4.x; up[1] += u4.y; up[2] += u4.z; up[3] += u4.w;
             }
-            if (NORM) total += recv[sums_off / 4 + z * ((p.T + 3) / 4) * 4 + tt];
-          }
-          if (NORM) {
-            const float r = rsqrtf(total / (float)p.K + p.eps);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { a[e] *= r; up[e] *= r; }
           }
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -346,16 +266,15 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const int tt = u / per, f = u - tt * per;
         float a[4];
         int n;
-        const float r = NORM ? ssq[tt] : 1.f;
         if (gated) {
           const float* src = st + (size_t)tt * pitch + (f >> 1) * 16 + (f & 1) * 4;
           const float4 g = *reinterpret_cast<const float4*>(src), up = *reinterpret_cast<const float4*>(src + 8);
-          a[0] = gate_mul(p, g.x * r, up.x * r); a[1] = gate_mul(p, g.y * r, up.y * r);
-          a[2] = gate_mul(p, g.z * r, up.z * r); a[3] = gate_mul(p, g.w * r, up.w * r);
+          a[0] = gate_mul(p, g.x, up.x); a[1] = gate_mul(p, g.y, up.y);
+          a[2] = gate_mul(p, g.z, up.z); a[3] = gate_mul(p, g.w, up.w);
           n = row0 / 2 + f * 4;
         } else {
           const float4 g = *reinterpret_cast<const float4*>(st + (size_t)tt * pitch + f * 4);
-          a[0] = g.x * r; a[1] = g.y * r; a[2] = g.z * r; a[3] = g.w * r;
+          a[0] = g.x; a[1] = g.y; a[2] = g.z; a[3] = g.w;
           n = row0 + f * 4;
           if (p.bias && (!p.red || part == 0)) {
 #pragma unroll
@@ -401,7 +320,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 }
 
 // ------------------------------------------------------------------ host side
-constexpr int kFewTail = (2 * kFewStages + 4) * 8 + kFewWarps * kFewNormTokens * 4;     // barriers, flags, sums of squares
+constexpr int kFewTail = (2 * kFewStages + 4) * 8;     // barriers, flags
 
 // The interleaved weight [rows, cols]: boxes of eight gate rows and their eight up rows, 64 deep.
 int make_gated_map(CUtensorMap* out, const void* ptr, int rows, int cols, int ld) {
@@ -424,13 +343,13 @@ int make_gated_map(CUtensorMap* out, const void* ptr, int rows, int cols, int ld
   return 0;
 }
 
-template <int MM, int TT>
+template <int MM>
 cudaError_t configure_few() {
   static OncePerDevice once;
   return once.run([] {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MM, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
     if (e == cudaSuccess)      // two CTAs share an SM only with the largest shared-memory carve-out
-      cudaFuncSetAttribute(gemm_few_kernel<MM, TT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      cudaFuncSetAttribute(gemm_few_kernel<MM>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     return e;
   });
 }
@@ -441,7 +360,7 @@ struct FewPlan { int rows, split, stages, cluster, red, tiles, grid, ring, recv,
 // The shared memory of a plan, with as many stages as two CTAs to an SM leave room for; false when two do not fit.
 bool few_memory(int T, int k_range, FewPlan& f) {
   const int tp = (T + 7) / 8 * 8, stage = (tp + f.rows) * 128, mm = T <= 64 ? 64 : 128;
-  f.recv = f.cluster > 1 ? f.split * ((f.rows / 16 + f.split - 1) / f.split) * T * 64 + f.split * ((T + 3) / 4) * 16 : 0;
+  f.recv = f.cluster > 1 ? f.split * ((f.rows / 16 + f.split - 1) / f.split) * T * 64 : 0;
   const int room = kFewSmem - 1024 - kFewTail - f.recv;
   f.stages = room / stage;
   if (f.stages > kFewStages) f.stages = kFewStages;
@@ -548,11 +467,11 @@ bool few_plan(int T, int N, int K, int in_memory, FewPlan& best) {
   return best.rows > 0;
 }
 
-template <int MM, int TT>
+template <int MM>
 int launch_few(const CUtensorMap& mw, const CUtensorMap& my, const FewParams& p, const FewPlan& f, cudaStream_t stream) {
-  const cudaError_t e = configure_few<MM, TT>();
+  const cudaError_t e = configure_few<MM>();
   if (e != cudaSuccess) return fail("gemm_tc: cannot reserve %d bytes of shared memory: %s", kFewSmem, cudaGetErrorString(e));
-  ilb::launch_cluster(gemm_few_kernel<MM, TT>, dim3(f.grid), dim3(kFewThreads), (size_t)f.smem, stream, p.cluster, mw, my, p);
+  ilb::launch_cluster(gemm_few_kernel<MM>, dim3(f.grid), dim3(kFewThreads), (size_t)f.smem, stream, p.cluster, mw, my, p);
   return check_launch("gemm_tc");
 }
 
@@ -563,8 +482,6 @@ int run_few(FewParams& p, const FewPlan& f, const void* A, int lda, const void* 
   p.tmem_cols = p.rows <= 32 ? 32 : p.rows <= 64 ? 64 : p.rows <= 128 ? 128 : 256;
   CUtensorMap mw, my;
   if (p.epilogue == kSwiGLU ? make_gated_map(&mw, W, p.N, p.K, ldw) : make_map(&mw, W, p.N, p.K, ldw, p.rows)) return -1;
-  my = mw;
-  if (A != nullptr && make_map(&my, A, p.T, p.K, lda, p.tp)) return -1;
-  if (p.x != nullptr) return p.T <= 8 ? launch_few<64, 8>(mw, my, p, f, stream) : launch_few<64, 16>(mw, my, p, f, stream);
-  return p.T <= 64 ? launch_few<64, 0>(mw, my, p, f, stream) : launch_few<128, 0>(mw, my, p, f, stream);
+  if (make_map(&my, A, p.T, p.K, lda, p.tp)) return -1;
+  return p.T <= 64 ? launch_few<64>(mw, my, p, f, stream) : launch_few<128>(mw, my, p, f, stream);
 }

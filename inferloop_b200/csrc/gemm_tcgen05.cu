@@ -1471,29 +1471,6 @@ ILB_EXPORT int ilb_gemm_tc(const void* A, const void* W, const float* bias, void
   return launch<128, 6, false>(mx, my, mo, p, (int)grid, stream);
 }
 
-// The same product with A = the RMS norm (weight norm_w, 32-bit) of the 32-bit rows x [M, K], up to 16 of them, in one launch.
-ILB_EXPORT int ilb_gemm_tc_normed(const float* x, const float* norm_w, float eps, const void* W, const float* bias, void* out, int out_f32,
-                                  int M, int N, int K, int ldx, int ldw, int ldo, int mode, int* error_flag, float act_limit,
-                                  float act_sharp, float act_offset, cudaStream_t stream) {
-  ILB_REQUIRE(M > 0 && M <= kFewNormTokens && N > 0 && K > 0, "gemm_tc_normed: bad sizes M=%d N=%d K=%d", M, N, K);
-  ILB_REQUIRE(K % 8 == 0 && ldw % 8 == 0 && ldx % 4 == 0 && ldx >= K && ldw >= K, "gemm_tc_normed: K (%d) and the weight's leading dimension (%d) must be multiples of 8, the rows' (%d) of 4", K, ldw, ldx);
-  ILB_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)norm_w % 16 == 0) && ((uintptr_t)W % 16 == 0), "gemm_tc_normed: operands must be 16-byte aligned");
-  ILB_REQUIRE(x != nullptr && norm_w != nullptr && W != nullptr && eps > 0.f && mode != 1, "gemm_tc_normed: missing operands, or an accumulating product");
-  if (check_epilogue(mode, out, out_f32, N, ldo, bias, act_limit)) return -1;
-  Params p{};
-  p.out = out; p.bias = bias; p.error_flag = error_flag; p.M = M; p.N = N; p.K = K; p.ldo = ldo; p.out_f32 = out_f32;
-  p.epilogue = epilogue_of(mode, p);
-  p.act_limit = act_limit; p.act_sharp = act_sharp; p.act_offset = act_offset;
-  FewPlan few;
-  ILB_REQUIRE(few_plan(M, N, K, 1, few), "gemm_tc_normed: a weight of %d rows is not served", N);
-  FewParams q = few_params(p);
-  q.x = x; q.ldx = ldx; q.norm_w = norm_w; q.eps = eps;
-  return run_few(q, few, nullptr, 0, W, ldw, stream);
-}
-ILB_EXPORT int ilb_gemm_tc_normed_tokens() { return kFewNormTokens; }
-// Weights of more rows than this are not served by the kernel of few tokens.
-ILB_EXPORT int ilb_gemm_tc_few_rows() { return 256 * 2 * sm_count(); }
-
 // Products of many tokens on pairs of CTAs: 0 never, 1 where the sizes favour it, 2 wherever possible.
 ILB_EXPORT int ilb_gemm_tc_pairs(int mode) {
   g_pairs = mode < 0 ? 0 : mode > 2 ? 2 : mode;

@@ -1280,8 +1280,9 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[
 def gemm_sums_in_memory(on: bool) -> None:
     """Whether products that accumulate into a 32-bit output may let the K ranges of a tile meet
     in memory: the tiles of the last round of many tokens (on single CTAs or on pairs), and every
-    tile of up to eight tokens when the weight is large (faster; the order of that 32-bit sum
-    is not fixed, so two runs agree beyond rounding but not bit for bit).  On by default;
+    tile of up to eight tokens when the weight is large, or of 65 to 128 when the output is wide
+    (faster; the order of that 32-bit sum is not fixed, so two runs agree beyond rounding but not
+    bit for bit).  On by default;
     off gives sums whose bits do not change from run to run."""
     load_module("gemm_tcgen05").ilb_gemm_tc_sums_in_memory(_i(1 if on else 0))
 
@@ -1311,7 +1312,9 @@ def gemm_tuning(few_tokens_in_memory: Optional[int] = None, few_tokens_ranges: i
 
 def gemm_tc_plan(M: int, N: int, K: int, accumulate: bool = False, swiglu: bool = False) -> dict:
     """How `gemm_tc` deals out a product of these sizes (needs a device: the answer depends
-    on how many CTAs fit it).  `pairs` > 0: the product runs on that many pairs of CTAs, each
+    on how many CTAs fit it).  Up to 128 tokens on the kernel of few tokens (gemm_few.cuh): `tile_n` is the token
+    block's height, `tiles` and `grid` its deal, `cluster` the ranges of a tile that meet in K order; `swap` is 0
+    there for 65 to 128 tokens whose ranges meet in memory.  `pairs` > 0: the product runs on that many pairs of CTAs, each
     tile left over after the whole rounds (or every tile) cut into `pair_split` K ranges, and
     `sums_meet_in_memory` speaks of those; the other fields then describe the single-CTA deal
     that `gemm_pairs(0)` would use."""
