@@ -7,12 +7,13 @@
 // 148 SMs), the tokens' operand is fetched again for every tile, and many tokens leave a shallow ring.  Here the
 // tokens are the MMA's rows (64 of them, or 128; a tile's operand A block holds the real tokens only, the MMA
 // reads on into the weight block behind it and the rows that come of it are nobody's) and the weight rows its
-// columns, so that a tile may be any multiple of 16 rows up to 256.  `few_plan` picks the height and the number of
-// K ranges for which the CTAs, two to an SM, come out even.  Launch after launch on rotating weights (us; before ->
-// after, the floor in brackets): 24,576 x 4,096 gated, 8 tokens 36.1 -> 33.0 (30.8), 64 tokens 45.6 -> 36.5, 128
-// tokens 55.8 -> 41.7; 51,200 x 5,120 gated, 24 tokens 95.2 -> 79.1 (80.2); 5,120 x 17,408 adding, 8 tokens 29.9 ->
-// 27.9 (27.3), 24 tokens 35.8 -> 30.6, 96 tokens 37.7 -> 32.5; 6,144 x 4,096, 8 tokens 12.0 -> 11.1 (7.7), 96
-// tokens 22.2 -> 16.7; 10,240 x 5,120, 64 tokens 27.8 -> 22.8 (16.0).
+// columns, so that a tile may be any multiple of 16 rows up to 256.  `few_plan` picks the height for which the CTAs, two to an
+// SM, come out even; into how many K ranges a sum is cut belongs to the weight (`few_ranges`), unless the ranges meet in
+// memory.  Launch after launch on rotating weights (us; former deal -> this one; in brackets the weight's bytes at 6.54 TB/s,
+// the rate of a copy, which reads and writes: reads alone have reached 7.1): 24,576 x 4,096 gated, 8 tokens 35.1 -> 32.2
+// (30.8), 64 tokens 43.5 -> 34.8, 128 tokens 55.7 -> 39.7; 51,200 x 5,120 gated, 1 token 84.0 -> 76.1 (80.2), 72 tokens
+// 129.7 -> 84.4; 5,120 x 17,408 adding, 8 tokens 30.1 -> 28.2 (27.3), 24 tokens 35.6 -> 30.9, 64 tokens 40.2 -> 33.5;
+// 6,144 x 4,096, 8 tokens 11.8 -> 11.6 (7.7), 96 tokens 22.0 -> 15.1; 10,240 x 5,120, 64 tokens 27.8 -> 22.6 (16.0).
 //
 // Per CTA (320 threads):
 //   warp 0     requests the weight blocks by TMA (128-byte swizzle; one box a block, or for gated weights a box of
@@ -22,8 +23,9 @@
 //   warp 1     tensor memory; one lane issues tcgen05.mma, four to a K block of 64;
 //   warps 2-9  the write-out.  With one K range, or ranges that meet in memory (red.add), the tile goes through the
 //              idle ring so that a thread holds four neighbouring outputs; the ranges of a tile that must be added
-//              in K order are the CTAs of a cluster, which send each other their shares (st.async on the owner's
-//              mbarrier), chunk j of 16 columns belonging to CTA j % split.
+//              in K order are the CTAs of a cluster, chunk j of 16 columns belonging to CTA j % split.  They send each
+//              other their shares (st.async on the owner's mbarrier); where the area for these would leave too little
+//              ring (LATE), each parks its share in its idle ring and the owners fetch, between two cluster barriers.
 // (Tried and taken back: the RMS norm in front of a product of up to 16 tokens inside it, warps 2-9 reading the 32-bit rows, laying
 // them out ahead of the stream and leaving the root mean square to the result.  Launch after launch it took 0.3 to 0.8 us where the
 // norm's launch takes 1.7; in a step, where that launch hides behind its neighbours, 8B sizes lost 3 % at one token.)
@@ -46,14 +48,14 @@ struct FewParams {
   float act_limit, act_sharp, act_offset;
 };
 
-// MM: rows of the MMA, 64 or 128.
-template <int MM>
+// MM: rows of the MMA, 64 or 128.  LATE: the shares of a cluster are parked and fetched, not sent.
+template <int MM, bool LATE>
 __global__ void __launch_bounds__(kFewThreads, 2)
 gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_y, const FewParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - smem_u32(smem_raw));
-  float* recv = reinterpret_cast<float*>(smem + p.ring_bytes);
+  float* recv = reinterpret_cast<float*>(smem + (LATE ? 0 : p.ring_bytes));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.ring_bytes + p.recv_bytes);
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kFewStages, tfull = empty0 + 8 * kFewStages, rbar = tfull + 8;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * kFewStages + 2);
@@ -84,10 +86,10 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     if (lane == 0) {
       for (int s = 0; s < p.stages; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
       mbar_init(tfull, 1);
-      if (p.cluster > 1) mbar_init(rbar, 1);
+      if (p.cluster > 1 && !LATE) mbar_init(rbar, 1);
       *failed = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      if (p.cluster > 1) {
+      if (p.cluster > 1 && !LATE) {
         const int nch = p.rows / 16, me = part;
         const int nloc = (nch - me + p.split - 1) / p.split;
         mbar_expect_tx(rbar, (uint32_t)(p.split * nloc * p.T * 64));
@@ -131,6 +133,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       *failed = 1; if (p.error_flag) *p.error_flag = 1;
       for (int it = armed > p.stages ? armed - p.stages : 0; it < armed; ++it) mbar_wait(full0 + 8 * (it % p.stages), (it / p.stages) & 1);
     }
+    __syncwarp();
+    if (LATE) { cluster_sync_all(); cluster_sync_all(); }       // with the warps of the write-out
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.rows >> 3) << 17) | ((uint32_t)(MM >> 4) << 24);
@@ -151,6 +155,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       if (!ok) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
       tcgen05_commit(tfull);
     }
+    __syncwarp();
+    if (LATE) { cluster_sync_all(); cluster_sync_all(); }       // with the warps of the write-out
   } else {
     const int et = threadIdx.x - 64, ew = warp - 2;
     pdl_wait();
@@ -163,9 +169,11 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     tcgen05_fence_after();
     const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
     const bool bad = *failed != 0;
-    if (p.cluster > 1) {
+    if (LATE || p.cluster > 1) {
       // ---- the K ranges of a tile are the CTAs of a cluster: chunk j of 16 columns belongs to CTA j % split
-      const uint32_t recv_addr = smem_u32(recv);
+      // A chunk is [four columns][token][4], tokens swizzled by the column: a warp's stores are whole lines of 128 bytes, and a quarter
+      // warp that reads four columns of two tokens meets no bank twice.
+      const uint32_t recv_addr = smem_u32(recv), plane = (uint32_t)p.tp * 16u;
       if (warp_on) {
         for (int j = hf; j < nch; j += 2) {
           float v[32];
@@ -173,17 +181,22 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           if (mine) {
             const uint32_t owner = (uint32_t)(j % p.split);
             const uint32_t nl = (uint32_t)((nch - (int)owner + p.split - 1) / p.split);
-            const uint32_t dst = peer_addr(recv_addr + (((uint32_t)part * nl + (uint32_t)(j / p.split)) * (uint32_t)p.T + (uint32_t)t) * 64u, owner);
-            const uint32_t bar = peer_addr(rbar, owner);
+            const uint32_t dst = LATE ? 0u : peer_addr(recv_addr + ((uint32_t)part * nl + (uint32_t)(j / p.split)) * 4u * plane, owner);
+            const uint32_t bar = LATE ? 0u : peer_addr(rbar, owner);
 #pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4)
-              st_peer_v4(dst + (uint32_t)((c4 ^ ((t >> 1) & 3)) << 4), bar, v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
+            for (int c4 = 0; c4 < 4; ++c4) {
+              const uint32_t off = (uint32_t)c4 * plane + (uint32_t)(t ^ (c4 << 1)) * 16u;
+              if (LATE) *reinterpret_cast<float4*>(smem + (uint32_t)j * 4u * plane + off) = make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
+              else st_peer_v4(dst + off, bar, v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
+            }
           }
         }
       }
+      __syncwarp();
+      if (LATE) cluster_sync_all();
       const int nl = (nch - part + p.split - 1) / p.split;
       const bool vec = p.ldo % 4 == 0 && (uintptr_t)p.out % 16 == 0;
-      bool arrived = false;
+      bool arrived = LATE;
       const int per_shift = gated ? 1 : 2, n_end = gated ? p.N / 2 : p.N;       // units of four outputs: two or four a chunk
       for (int u0 = et; u0 < (nl * p.T) << per_shift; u0 += 2 * kFewEpi) {
         float old[2][4];
@@ -217,13 +230,34 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           const int chunk = jl * p.split + part;
           const int n = gated ? row0 / 2 + chunk * 8 + c4 * 4 : row0 + chunk * 16 + c4 * 4;
           float a[4] = {0.f, 0.f, 0.f, 0.f}, up[4] = {0.f, 0.f, 0.f, 0.f};
-          for (int z = 0; z < p.split; ++z) {
-            const float* src = recv + (size_t)((z * nl + jl) * p.T + tt) * 16;
-            const float4 s4 = *reinterpret_cast<const float4*>(src + ((c4 ^ ((tt >> 1) & 3)) << 2));
-            a[0] += s4.x; a[1] += s4.y; a[2] += s4.z; a[3] += s4.w;
-            if (gated) {
-              const float4 u4 = *reinterpret_cast<const float4*>(src + (((c4 + 2) ^ ((tt >> 1) & 3)) << 2));
-              up[0] += u4.x; up[1] += u4.y; up[2] += u4.z; up[3] += u4.w;
+          const uint32_t at = (uint32_t)c4 * plane + (uint32_t)(tt ^ (c4 << 1)) * 16u;
+          const uint32_t at_up = (uint32_t)(c4 + 2) * plane + (uint32_t)(tt ^ ((c4 + 2) << 1)) * 16u;
+          if (LATE) {                            // four peers' loads in flight
+            for (int z0 = 0; z0 < p.split; z0 += 4) {
+              float4 s4[4], u4[4];
+#pragma unroll
+              for (int z = 0; z < 4; ++z) {
+                if (z0 + z >= p.split) break;
+                const uint32_t src = peer_addr(recv_addr + (uint32_t)chunk * 4u * plane, (uint32_t)(z0 + z));
+                s4[z] = ld_peer_v4(src + at);
+                if (gated) u4[z] = ld_peer_v4(src + at_up);
+              }
+#pragma unroll
+              for (int z = 0; z < 4; ++z) {
+                if (z0 + z >= p.split) break;
+                a[0] += s4[z].x; a[1] += s4[z].y; a[2] += s4[z].z; a[3] += s4[z].w;
+                if (gated) { up[0] += u4[z].x; up[1] += u4[z].y; up[2] += u4[z].z; up[3] += u4[z].w; }
+              }
+            }
+          } else {
+            for (int z = 0; z < p.split; ++z) {
+              const uint8_t* src = reinterpret_cast<const uint8_t*>(recv) + (uint32_t)(z * nl + jl) * 4u * plane;
+              const float4 s4 = *reinterpret_cast<const float4*>(src + at);
+              a[0] += s4.x; a[1] += s4.y; a[2] += s4.z; a[3] += s4.w;
+              if (gated) {
+                const float4 u4 = *reinterpret_cast<const float4*>(src + at_up);
+                up[0] += u4.x; up[1] += u4.y; up[2] += u4.z; up[3] += u4.w;
+              }
             }
           }
 #pragma unroll
@@ -242,7 +276,9 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           }
         }
       }
-      if (!arrived && !mbar_wait(rbar, 0)) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
+      __syncwarp();
+      if (LATE) cluster_sync_all();           // nobody leaves while a peer may still read its share
+      else if (!arrived && !mbar_wait(rbar, 0)) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
     } else if (!bad) {
       // ---- the tile (or its K range) through shared memory: the ring is idle, everything in it has been consumed
       float* st = reinterpret_cast<float*>(smem);
@@ -276,12 +312,16 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           const float4 g = *reinterpret_cast<const float4*>(st + (size_t)tt * pitch + f * 4);
           a[0] = g.x; a[1] = g.y; a[2] = g.z; a[3] = g.w;
           n = row0 + f * 4;
-          if (p.bias && (!p.red || part == 0)) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) a[e] += n + e < n_end ? p.bias[n + e] : 0.f;
-          }
         }
         const size_t o = (size_t)tt * p.ldo + n;
+        if (p.epilogue == kAccumulate && !p.red) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) if (n + e < n_end) a[e] += __ldcg((const float*)p.out + o + e);
+        }
+        if (!gated && p.bias && (!p.red || part == 0)) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] += n + e < n_end ? p.bias[n + e] : 0.f;
+        }
         if (p.red) {
           float* dst = (float*)p.out + o;
           if (vec && n + 4 <= n_end) {
@@ -291,10 +331,6 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             for (int e = 0; e < 4; ++e) if (n + e < n_end) atomicAdd(dst + e, a[e]);
           }
           continue;
-        }
-        if (p.epilogue == kAccumulate) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) if (n + e < n_end) a[e] += __ldcg((const float*)p.out + o + e);
         }
         if (p.relu2) {
 #pragma unroll
@@ -343,24 +379,85 @@ int make_gated_map(CUtensorMap* out, const void* ptr, int rows, int cols, int ld
   return 0;
 }
 
-template <int MM>
+template <int MM, bool LATE>
 cudaError_t configure_few() {
   static OncePerDevice once;
   return once.run([] {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MM, LATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
     if (e == cudaSuccess)      // two CTAs share an SM only with the largest shared-memory carve-out
-      cudaFuncSetAttribute(gemm_few_kernel<MM>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      cudaFuncSetAttribute(gemm_few_kernel<MM, LATE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     return e;
   });
 }
 
-// How a product of few tokens is dealt out.
-struct FewPlan { int rows, split, stages, cluster, red, tiles, grid, ring, recv, smem; };
+// What the deal depends on beside the sizes: SMs, and the clusters of 1 to 8 CTAs that the device holds at once with one CTA to an SM
+// and with two.
+struct FewDevice { int sms, one[9], two[9]; };
+
+// An empty kernel of the same shape is asked about: the occupancy query counts one CTA to an SM for any kernel that allocates tensor
+// memory.  A B200 answers 74, 33 and 15 clusters of 2, 4 and 8 with one CTA to an SM; 148, 71 and 33 with two (72 clusters of
+// four did take a second round, 18 -> 26 us; 64 and 66 did not).
+__global__ void __launch_bounds__(kFewThreads, 2) few_shape_kernel() {}
+
+int few_clusters(int cluster, int smem) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster * 256);
+  cfg.blockDim = dim3(kFewThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  int n = 0;
+  cudaError_t e = cudaFuncSetAttribute(few_shape_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(few_shape_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, few_shape_kernel, &cfg);
+  if (e != cudaSuccess) { cudaGetLastError(); n = 0; }
+  return n;
+}
+
+FewDevice few_device() {
+  static std::mutex mu;
+  static FewDevice known{};
+  std::lock_guard<std::mutex> g(mu);
+  if (known.sms == 0) {
+    FewDevice d{};
+    d.sms = sm_count();
+    for (int c = 1; c <= 8; c *= 2) { d.one[c] = few_clusters(c, 2 * kFewSmem); d.two[c] = few_clusters(c, kFewSmem); }
+    known = d;
+  }
+  return known;
+}
+
+// How a product of few tokens is dealt out.  late: the shares of a cluster are parked in the rings and fetched.
+struct FewPlan { int rows, split, stages, cluster, late, red, tiles, grid, ring, recv, smem; };    // recv: 0 when late
+
+// Into how many K ranges a tile's sum is cut where their order is kept.  It belongs to the weight alone, so that a row's bits are the
+// same whatever it is computed beside: what tiles of 128 rows allow, in ranges of equal length, of CTAs that the device
+// holds at once.  0: more tiles than two CTAs to an SM, which are shared out block by block (`make_plan`).
+int few_ranges(int N, int K, const FewDevice& d) {
+  const long long tiles = (N + 127) / 128, kb = (K + kBlockK - 1) / kBlockK;
+  if (tiles > 2ll * d.sms) return 0;
+  int split = 1;
+  while (split < 8 && tiles * split * 2 <= 2ll * d.sms && split * 2 <= kb) split *= 2;
+  while (split > 1 && d.one[split / 2] < tiles) split /= 2;
+  return split;
+}
+
+// Into how many ranges at most a product that adds into a 32-bit output cuts a tile's sum when the ranges may meet there (separate CTAs,
+// red.add; the order is then not fixed); 1: it keeps the order.
+int few_ranges_in_memory(int T, int N, int K, const FewDevice& d) {
+  if (!g_sums_in_memory) return 1;
+  if (T <= g_red_few_tokens) return N >= 2048 && K >= 2048 && few_ranges(N, K, d) > 1 ? g_red_few_split : 1;
+  if (T <= 64 || N < 3072) return 1;
+  const long long tiles = (N + 255) / 256, rest = tiles % d.sms;
+  return rest != 0 && tiles * 12 >= d.sms && add_split(rest, (K + kBlockK - 1) / kBlockK) >= 2 ? 8 : 1;
+}
 
 // The shared memory of a plan, with as many stages as two CTAs to an SM leave room for; false when two do not fit.
 bool few_memory(int T, int k_range, FewPlan& f) {
   const int tp = (T + 7) / 8 * 8, stage = (tp + f.rows) * 128, mm = T <= 64 ? 64 : 128;
-  f.recv = f.cluster > 1 ? f.split * ((f.rows / 16 + f.split - 1) / f.split) * T * 64 : 0;
+  f.recv = f.cluster > 1 && !f.late ? f.split * ((f.rows / 16 + f.split - 1) / f.split) * tp * 64 : 0;
   const int room = kFewSmem - 1024 - kFewTail - f.recv;
   f.stages = room / stage;
   if (f.stages > kFewStages) f.stages = kFewStages;
@@ -369,109 +466,88 @@ bool few_memory(int T, int k_range, FewPlan& f) {
   f.ring = f.stages * stage;
   const int reach = (f.stages - 1) * stage + mm * 128;             // the MMA reads mm rows from the last stage's first
   if (reach > f.ring) f.ring = reach;
-  const int staged = (T * (f.rows + 4) * 4 + 15) / 16 * 16;        // the tile on its way out
-  if (f.cluster == 1 && staged > f.ring) f.ring = staged;
-  f.smem = 1024 + f.ring + f.recv + kFewTail;
+  const int staged = f.cluster == 1 ? (T * (f.rows + 4) * 4 + 15) / 16 * 16 : f.late ? f.rows * tp * 4 : 0;       // the tile on its way out
+  if (staged > f.ring) f.ring = staged;
+  f.smem = 1024 + f.ring + f.recv + kFewTail;                      // what the kernel lays out, in this order
   return f.smem <= kFewSmem;
 }
 
-// Clusters of so many CTAs, two CTAs to an SM, that the device holds at once.  The occupancy query counts one CTA to an
-// SM for any kernel that allocates tensor memory, so an empty kernel of the same shape is asked about: it answers 148, 71 and
-// 33 clusters of 2, 4 and 8, and 72 clusters of four did take a second round (18 -> 26 us), 64 and 66 did not.
-__global__ void __launch_bounds__(kFewThreads, 2) few_shape_kernel() {}
-
-int few_clusters(int cluster) {
-  static int cache[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  if (cluster < 1 || cluster > 8) return 0;
-  if (cache[cluster] != 0) return cache[cluster] < 0 ? 0 : cache[cluster];
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cluster * 256);
-  cfg.blockDim = dim3(kFewThreads);
-  cfg.dynamicSmemBytes = kFewSmem;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  int n = 0;
-  cudaError_t e = cudaFuncSetAttribute(few_shape_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(few_shape_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, few_shape_kernel, &cfg);
-  if (e != cudaSuccess) { cudaGetLastError(); n = 0; }
-  cache[cluster] = n > 0 ? n : -1;
-  return n > 0 ? n : 0;
-}
-
-// What a plan costs, near enough to its time in us to rank plans: a fit to 9,600 timed plans of 20 weights (1,024 to 51,200 rows,
-// 1,024 to 25,600 deep) at 1 to 128 tokens; the plan it picks is on average 1.4 % slower than the best one.  What decides is not
-// an SM's share of the bytes but how long a CTA's stream is against its ring (a round trip of 3.4 us for `stages` blocks of
-// 64) and how many MMAs are issued (four a block, each as long as 118 columns at least); a second CTA on some SMs leaves
-// less room to the next kernel's first blocks; and the shares that meet cost by the value.
-double few_cost(int T, int N, int K, const FewPlan& f) {
-  const int kb = (K + kBlockK - 1) / kBlockK, range = (kb + f.split - 1) / f.split, sms = sm_count();
+// What ranks the plans of a product (it is no time): a fit to 6,313 timed plans of 253 products, 20 weights (1,024 to 51,200 rows, 1,024 to
+// 25,600 deep) at 1 to 128 tokens.  The plan it picks is on average 1.3 % slower than the fastest that was timed, 23 % at worst
+// (4,096 x 1,024 at 40 tokens, 7.5 against 6.1 us).  What decides is not an SM's share of the bytes but how long a CTA's stream is
+// against its ring (a round trip for `stages` blocks of 64) and how many MMAs are issued (four a block, each as long as 118
+// columns at least); a second CTA on some SMs leaves less room to the next kernel's first blocks; and the write-out costs by the
+// value.  Shares that are parked and fetched cost two to three us more than shares that are sent: they pay where the area
+// for the latter would leave a ring of one to three stages (6,144 x 4,096 at 96 tokens 16.9 -> 15.2 us, 12,288 x 2,048 at 128 18.8 -> 15.6).
+double few_cost(int T, int N, int K, const FewPlan& f, const FewDevice& d) {
+  const int kb = (K + kBlockK - 1) / kBlockK, range = (kb + f.split - 1) / f.split, sms = d.sms;
   const int per_sm = f.grid <= sms ? 1 : 2;
-  const double bytes = (double)N * K * 2 / 7.0e6, ring = 3.38 * range / f.stages, tile = 1e-3 * T * f.rows;
-  double t = (bytes > ring ? bytes : ring) + 0.317 * range + 0.107 * per_sm * range * (f.rows > 118 ? f.rows / 128.0 : 0.92);
-  if (per_sm == 2) t += 0.476 + 2.44 * (f.grid - sms) / sms;
-  if (f.red) t += 0.965 * f.split * 4e-6 * T * N;
-  else if (f.cluster > 1) t += (0.78 + 1.04 * per_sm) * tile + 0.02 * f.split;
-  else t += 0.966 * tile;
+  const double bytes = (double)N * K * 2 / 7.0e6, ring = 2.85 * range / f.stages, tile = 1e-3 * T * f.rows;
+  double t = (bytes > ring ? bytes : ring) + 0.204 * range + 0.147 * per_sm * range * (f.rows > 118 ? f.rows / 128.0 : 0.92);
+  if (per_sm == 2) t += 0.866 + 2.62 * (f.grid - sms) / sms;
+  if (f.red) t += 0.794 * f.split * 4e-6 * T * N;
+  else if (f.cluster > 1) t += (0.388 + 0.118 * per_sm) * tile + 0.272 * f.split + (f.late ? 2.87 + 0.186 * per_sm * tile : 0.0);
+  else t += 1.55 * tile;
   return t;
 }
 
-// `in_memory` > 1: the K ranges of a tile, up to that many, may be separate CTAs that add into the output in memory (the sum's order
-// is then not fixed).  False where the kernel does not serve: more tokens, or a weight of more tiles than two CTAs to an SM.
-bool few_plan(int T, int N, int K, int in_memory, FewPlan& best) {
-  if (T > kFewTokens || (N + 255) / 256 > 2 * sm_count()) return false;
+// `can_add`: the product adds into a 32-bit output whose rows are 16-byte multiples.  False where the kernel does not serve: more
+// tokens, or a weight of more tiles than two CTAs to an SM.
+bool few_plan(int T, int N, int K, bool can_add, const FewDevice& d, FewPlan& best) {
+  if (T > kFewTokens || (N + 255) / 256 > 2 * d.sms) return false;
+  const int meet = can_add ? few_ranges_in_memory(T, N, K, d) : 1;
+  int ranges = few_ranges(N, K, d);
+  // A weight of more 128-row tiles than two CTAs to an SM: whole tiles here, but only where the adding products of its width let their
+  // ranges meet in memory, so that the rows it reads differ from run to run as it is (51,200 x 5,120 gated, 8 tokens 76.9 us
+  // here and 85.9 in `make_plan`'s form, 96 tokens 84.8 and 139.2).  Elsewhere it keeps that form, and so its bits, although 24
+  // tokens take 91.2 us where whole tiles took 77.5.
+  if (ranges == 0 && meet == 1) {
+    if (few_ranges_in_memory(T, K, K, d) == 1) return false;
+    ranges = 1;
+  }
   struct Key { long long a, b; bool operator==(const Key& o) const { return a == o.a && b == o.b; } };
   struct Hash { size_t operator()(const Key& k) const { return std::hash<long long>()(k.a * 1000003ll ^ k.b); } };
   static std::unordered_map<Key, FewPlan, Hash> cache;
   static std::mutex mu;
-  const Key key{((long long)T << 32) | (unsigned)N, ((long long)K << 8) | in_memory};
+  const Key key{((long long)T << 32) | (unsigned)N, ((long long)K << 16) | (meet << 8) | ranges};
   std::lock_guard<std::mutex> g(mu);
   auto it = cache.find(key);
   if (it != cache.end()) { best = it->second; return best.rows > 0; }
   const int kb = (K + kBlockK - 1) / kBlockK;
-  const bool may_add = in_memory > 1;
   // Clusters are not placed in the last slots while the kernel before still holds some: 280 and 292 CTAs lost 5 to 6 % to 256.
   // More than 64 tokens that add in memory: one CTA to an SM (two take 0.5 to 1 us less of 10 to 45, but a product of many tokens
   // has never had more).
-  const int most = !may_add ? 2 * sm_count() * 15 / 16 : T > 64 ? sm_count() : 2 * sm_count();
+  const int most = meet == 1 ? 2 * d.sms * 15 / 16 : T > 64 ? d.sms : 2 * d.sms;
   double least = 1e30;
   best = FewPlan{};
-  auto consider = [&](int split) {
-    for (int rows = 16; rows <= 256; rows += 16) {
-      FewPlan f{};
-      f.rows = rows; f.split = split; f.red = may_add && split > 1 ? 1 : 0; f.cluster = f.red ? 1 : split;
-      f.tiles = (N + rows - 1) / rows; f.grid = f.tiles * split;
-      if (f.grid > (split > 1 ? most : 2 * sm_count()) || !few_memory(T, kb / split, f)) continue;
-      const double t = few_cost(T, N, K, f);
-      if (t >= least) continue;
-      if (f.cluster > 1 && f.tiles > few_clusters(f.cluster)) continue;       // all clusters at once, or the last ones cost a second round
-      least = t;
-      best = f;
-    }
+  auto consider = [&](int split, bool at_once) {
+    for (int rows = 16; rows <= 256; rows += 16)
+      for (int late = 0; late <= (meet == 1 && split > 1 ? 1 : 0); ++late) {
+        FewPlan f{};
+        f.rows = rows; f.split = split; f.red = meet > 1 && split > 1 ? 1 : 0; f.cluster = f.red ? 1 : split; f.late = late;
+        f.tiles = (N + rows - 1) / rows; f.grid = f.tiles * split;
+        if (f.grid > (split > 1 ? most : 2 * d.sms) && at_once) continue;
+        if (f.cluster > 1 && f.tiles > d.two[f.cluster] && at_once) continue;       // or the last ones cost a second round
+        if (!few_memory(T, kb / split, f)) continue;
+        const double t = few_cost(T, N, K, f, d);
+        if (t < least) { least = t; best = f; }
+      }
   };
-  if (may_add) {
-    for (int split = 1; split <= in_memory && split <= kb; ++split) consider(split);
-  } else {
-    // Sums of fewer than eight blocks: as many ranges as there are powers of two, whatever the tokens, as products of more tokens
-    // have them: the same partial sums, and a row's bits rarely depend on what it is computed beside.  (At 16 tokens the
-    // fastest too, 768 x 256 3.04 -> 2.71 us; at 40 tokens it takes up to 0.6 us more, 1,536 x 256 2.96 -> 3.56.)
-    if (kb < 8) consider(kb >= 4 ? 4 : kb >= 2 ? 2 : 1);
-    // (tiles of 64 rows that fill the device twice over: an exchange could only cost)
-    if (best.rows == 0)
-      for (int split = 1; split <= 8 && split <= kb && (split == 1 || (long long)N <= 64ll * 2 * sm_count()); split *= 2) consider(split);
-  }
+  if (meet > 1)
+    for (int split = 1; split <= meet && split <= kb; ++split) consider(split, true);
+  else
+    consider(ranges, true);
+  if (best.rows == 0 && meet == 1 && ranges > 1) consider(ranges, false);
   if (cache.size() > 4096) cache.clear();
   cache.emplace(key, best);
   return best.rows > 0;
 }
 
-template <int MM>
+template <int MM, bool LATE>
 int launch_few(const CUtensorMap& mw, const CUtensorMap& my, const FewParams& p, const FewPlan& f, cudaStream_t stream) {
-  const cudaError_t e = configure_few<MM>();
+  const cudaError_t e = configure_few<MM, LATE>();
   if (e != cudaSuccess) return fail("gemm_tc: cannot reserve %d bytes of shared memory: %s", kFewSmem, cudaGetErrorString(e));
-  ilb::launch_cluster(gemm_few_kernel<MM>, dim3(f.grid), dim3(kFewThreads), (size_t)f.smem, stream, p.cluster, mw, my, p);
+  ilb::launch_cluster(gemm_few_kernel<MM, LATE>, dim3(f.grid), dim3(kFewThreads), (size_t)f.smem, stream, p.cluster, mw, my, p);
   return check_launch("gemm_tc");
 }
 
@@ -483,5 +559,6 @@ int run_few(FewParams& p, const FewPlan& f, const void* A, int lda, const void* 
   CUtensorMap mw, my;
   if (p.epilogue == kSwiGLU ? make_gated_map(&mw, W, p.N, p.K, ldw) : make_map(&mw, W, p.N, p.K, ldw, p.rows)) return -1;
   if (make_map(&my, A, p.T, p.K, lda, p.tp)) return -1;
-  return p.T <= 64 ? launch_few<64>(mw, my, p, f, stream) : launch_few<128>(mw, my, p, f, stream);
+  if (f.late) return p.T <= 64 ? launch_few<64, true>(mw, my, p, f, stream) : launch_few<128, true>(mw, my, p, f, stream);
+  return p.T <= 64 ? launch_few<64, false>(mw, my, p, f, stream) : launch_few<128, false>(mw, my, p, f, stream);
 }

@@ -3,8 +3,8 @@
 // or, for a weight whose rows interleave 64 gate rows with their 64 up rows,
 //     out[M,N/2] = silu(gate) * up   (the SwiGLU product in the epilogue).
 //
-// Up to 128 tokens run on `gemm_few_kernel` (gemm_few.cuh), unless the weight has more tiles than two CTAs to an SM
-// (the output matrix); those, and products of more tokens, on the kernels of this file.
+// Up to 128 tokens run on `gemm_few_kernel` (gemm_few.cuh), unless the weight has more tiles of 128 rows than two CTAs to an SM (the
+// output matrix; and some wide gated weights, by `few_plan`'s rule); those, and products of more tokens, on the kernels of this file.
 // tcgen05.mma computes D[128 x BN] = X[128 x K] * Y[BN x K]^T with both operands K-major in
 // shared memory.  With few tokens the operands are swapped: X is a 128-row tile of the
 // WEIGHT and Y the (padded) tokens, so every tensor-core row does useful work and the
@@ -1044,6 +1044,24 @@ int sm_count() {
   return n;
 }
 
+// Whether the K ranges of a tile may meet in memory (the sum's order is then not fixed: runs
+// agree beyond rounding, not bit for bit).  `ilb_gemm_tc_sums_in_memory(0)` turns it off.
+bool g_sums_in_memory = true;
+// Accumulating products of up to this many tokens, with a weight of at least 2,048 x 2,048, add the K ranges of a tile in
+// memory (separate CTAs, red.add) instead of inside a cluster, which fixes the order (4,096 x 4,096 at 8 tokens 7.2 against
+// 8.6 us, 4,096 x 12,288 16.9 against 18.5); so do 65 to 128 tokens into a wide output (9.6 against 12.9, 20.1 against 24.6).
+// In between the order stays fixed.
+int g_red_few_tokens = 8;
+int g_red_few_split = 8;
+
+// Equal K ranges per tile when `rest` tiles share the SMs: as many as fit, none shorter than
+// four K blocks.
+long long add_split(long long rest, long long k_blocks) {
+  long long split = sm_count() / rest;
+  if (split > k_blocks / 4) split = k_blocks / 4;
+  return split < 1 ? 1 : split;
+}
+
 #include "gemm_few.cuh"
 
 // Ring, alignment slack, barriers and flags, then (few tokens) the whole-tile SwiGLU exchange.
@@ -1120,24 +1138,6 @@ namespace {
 // How a product is dealt out: orientation, tile shape, grid, cluster, rounds (fills the
 // scheduling fields of `p`, which must hold M, N, K, k_blocks and the epilogue already).
 struct Plan { bool swap, tail, additive; int bn, ms, x_rows, y_rows; long long grid; };
-
-// Whether the K ranges of a tile may meet in memory (the sum's order is then not fixed: runs
-// agree beyond rounding, not bit for bit).  `ilb_gemm_tc_sums_in_memory(0)` turns it off.
-bool g_sums_in_memory = true;
-// Accumulating products of up to this many tokens, with a weight of at least 2,048 x 2,048, add the K ranges of a tile in
-// memory (separate CTAs, red.add) instead of inside a cluster, which fixes the order (4,096 x 4,096 at 8 tokens 7.2 against
-// 8.6 us, 4,096 x 12,288 16.9 against 18.5); so do 65 to 128 tokens into a wide output (9.6 against 12.9, 20.1 against 24.6).
-// In between the order stays fixed.
-int g_red_few_tokens = 8;
-int g_red_few_split = 8;
-
-// Equal K ranges per tile when `rest` tiles share the SMs: as many as fit, none shorter than
-// four K blocks.
-long long add_split(long long rest, long long k_blocks) {
-  long long split = sm_count() / rest;
-  if (split > k_blocks / 4) split = k_blocks / 4;
-  return split < 1 ? 1 : split;
-}
 
 // `can_add`: the product accumulates into a 32-bit output that the TMA write-out can reach,
 // so that the K ranges of a tile may be added in memory.
@@ -1346,13 +1346,6 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const CUtensorMap&
   return check_launch("gemm_tc");
 }
 
-// Whether (and into how many ranges at most) a product of few tokens may add the K ranges of a tile in memory.
-int few_ranges_in_memory(int M, int N, int K, bool can_add) {
-  if (!can_add || !g_sums_in_memory) return 1;
-  if (M <= g_red_few_tokens) return N >= 2048 && K >= 2048 ? g_red_few_split : 1;
-  return M > 64 && N >= 3072 && K >= 512 ? 8 : 1;
-}
-
 int epilogue_of(int mode, Params& p) {
   // 3 from the caller: the gated epilogue with relu as the gate's activation (else silu); 4: the clamped gated unit
   // 5: a plain product whose bfloat16 result leaves as relu(result)^2; 6: the gated epilogue with gelu's tanh form
@@ -1411,7 +1404,7 @@ ILB_EXPORT int ilb_gemm_tc(const void* A, const void* W, const float* bias, void
   const bool tma_reach = ((uintptr_t)out % 16 == 0) && ((long long)ldo * es) % 16 == 0;   // rows of 16-byte multiples from a 16-byte base
   const bool can_add = tma_reach && out_f32 && accumulate == 1;
   FewPlan few;
-  if (max_ctas <= 0 && few_plan(M, N, K, few_ranges_in_memory(M, N, K, can_add), few)) {
+  if (max_ctas <= 0 && few_plan(M, N, K, can_add, few_device(), few)) {
     FewParams q = few_params(p);
     return run_few(q, few, A, lda, W, ldw, stream);
   }
@@ -1510,7 +1503,7 @@ ILB_EXPORT int ilb_gemm_tc_plan(int M, int N, int K, int epilogue, int* out) {
   Params p{};
   p.M = M; p.N = N; p.K = K; p.k_blocks = (K + kBlockK - 1) / kBlockK; p.epilogue = epilogue;
   FewPlan few;
-  if (few_plan(M, N, K, few_ranges_in_memory(M, N, K, epilogue == 1), few)) {
+  if (few_plan(M, N, K, epilogue == 1, few_device(), few)) {
     // (65 to 128 tokens whose ranges meet in memory are reported as a product of many tokens, which also let them meet there)
     out[0] = M <= 64 || !few.red; out[1] = (M + 7) / 8 * 8; out[2] = 1; out[3] = few.grid; out[4] = few.cluster;
     out[5] = 0; out[6] = few.tiles; out[7] = few.red ? few.tiles : 0; out[8] = few.red; out[9] = 0; out[10] = 0;
@@ -1528,6 +1521,22 @@ ILB_EXPORT int ilb_gemm_tc_plan(int M, int N, int K, int epilogue, int* out) {
     out[9] = pp.n_pairs; out[10] = pp.split;
     out[8] = pp.split > 1 ? 1 : 0;
   }
+  return 0;
+}
+
+// The plan of a product of few tokens on a device with these facts (for tests; needs no GPU): SMs, then the clusters of 2, 4 and 8 CTAs
+// that it holds at once with one CTA to an SM and with two.  out[0..10] = served, rows of a tile, K ranges, stages, cluster, shares that
+// are fetched from the rings, ranges that meet in memory, tiles, bytes of the ring, of the area for shares, of all shared memory.
+ILB_EXPORT int ilb_gemm_few_plan(int T, int N, int K, int can_add, const int* facts, int* out) {
+  ILB_REQUIRE(T > 0 && N > 0 && K > 0 && facts != nullptr && out != nullptr && facts[0] > 0, "gemm_tc: bad sizes for a plan");
+  FewDevice d{};
+  d.sms = facts[0];
+  d.one[1] = d.sms; d.two[1] = 2 * d.sms;
+  for (int i = 0; i < 3; ++i) { d.one[2 << i] = facts[1 + i]; d.two[2 << i] = facts[4 + i]; }
+  FewPlan f{};
+  const bool served = few_plan(T, N, K, can_add != 0, d, f);
+  const int v[11] = {served ? 1 : 0, f.rows, f.split, f.stages, f.cluster, f.late, f.red, f.tiles, f.ring, f.recv, f.smem};
+  for (int i = 0; i < 11; ++i) out[i] = v[i];
   return 0;
 }
 

@@ -160,6 +160,11 @@ __device__ __forceinline__ float ld_peer_f32(uint32_t local_addr, uint32_t rank)
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
   return v;
 }
+__device__ __forceinline__ float4 ld_peer_v4(uint32_t remote_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote_addr) : "memory");
+  return v;
+}
 // Four floats into a peer's shared memory; the bytes count towards the peer's mbarrier.
 __device__ __forceinline__ void st_peer_v4(uint32_t remote_addr, uint32_t remote_bar, float a, float b, float c, float d) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"

@@ -33,3 +33,96 @@ def test_tiles_of_an_exact_product_of_many_tokens():
     assert tile(2048, 24576, 0) == 128
     for M, N in ((41, 8), (200, 4096), (512, 4096), (512, 6144), (1024, 4096), (2048, 4096), (2048, 6144), (512, 24576), (1024, 24576)):
         assert tile(M, N, 0) == 64
+
+
+# ------------------------------------------------------------------ products of few tokens (gemm_few.cuh)
+FEW_KEYS = ("served", "rows", "ranges", "stages", "cluster", "fetched", "in_memory", "tiles", "ring", "shares", "smem")
+FEW_TOKENS = (1, 2, 7, 8, 9, 16, 17, 24, 33, 40, 48, 64, 65, 72, 96, 104, 128)
+
+
+def few_plan(T, N, K, adds=False, in_memory=True):
+    """The plan on a device of 148 SMs that holds 74, 33 and 15 clusters of 2, 4 and 8 CTAs with one CTA to an SM and 148, 71 and 33
+    with two."""
+    import ctypes
+
+    from inferloop_b200.csrc.build import load_module
+    lib = load_module("gemm_tcgen05")
+    lib.ilb_gemm_tc_sums_in_memory(1 if in_memory else 0)
+    try:
+        out = (ctypes.c_int * len(FEW_KEYS))()
+        assert lib.ilb_gemm_few_plan(T, N, K, 1 if adds else 0, (ctypes.c_int * 7)(SMS, 74, 33, 15, 148, 71, 33), out) == 0
+        return dict(zip(FEW_KEYS, out))
+    finally:
+        lib.ilb_gemm_tc_sums_in_memory(1)
+
+
+def test_ranges_whose_order_is_kept_belong_to_the_weight():
+    """A row's sum is cut alike whatever it is computed beside: as many equal K ranges as tiles of 128 rows allow (two CTAs to an SM,
+    clusters that fit the device at once), for every token count, and for adding products too once sums in memory are off."""
+    for (N, K), ranges in {(6144, 4096): 4, (4096, 4096): 8, (24576, 4096): 1, (4096, 12288): 8, (7168, 5120): 4, (5120, 5120): 4,
+                           (34816, 5120): 1, (5120, 17408): 4, (10240, 5120): 2, (5120, 25600): 4, (4096, 2048): 8, (2048, 6144): 8,
+                           (4224, 4096): 8, (4352, 4096): 4, (9472, 1024): 4, (9600, 1024): 2, (18944, 512): 2, (19072, 512): 1,
+                           (37888, 320): 1, (768, 256): 4, (512, 384): 4, (256, 64): 1, (256, 72): 2, (72, 8): 1}.items():
+        for T in FEW_TOKENS:
+            for adds in (False, True):
+                plan = few_plan(T, N, K, adds, in_memory=False)
+                assert plan["served"] and plan["ranges"] == ranges and not plan["in_memory"], (T, N, K, plan)
+                assert plan["cluster"] == ranges, (T, N, K, plan)
+            assert few_plan(T, N, K)["ranges"] == ranges                       # a product that adds nothing never asks
+            if 8 < T <= 64:
+                assert few_plan(T, N, K, adds=True)["ranges"] == ranges        # and between 9 and 64 tokens nor does one that does
+
+
+def test_ranges_that_meet_in_memory():
+    """Up to 8 tokens with a weight of 2,048 x 2,048 or more, or 65 to 128 with a wide output; never when switched off."""
+    for T in FEW_TOKENS:
+        for (N, K), few, many in (((4096, 4096), True, True), ((2048, 2048), True, False), ((2047, 4096), False, False), ((4096, 512), False, True),
+                                  ((4096, 448), False, False), ((3072, 1024), False, False), ((3328, 1024), False, True), ((18944, 2048), True, True),
+                                  ((19200, 2048), False, False)):
+            may = (T <= 8 and few) or (T > 64 and many)
+            plan = few_plan(T, N, K, adds=True)
+            assert not plan["in_memory"] or may, (T, N, K, plan)
+            assert not may or plan["in_memory"] or plan["ranges"] == 1, (T, N, K, plan)
+    assert few_plan(1, 4096, 4096, adds=True)["in_memory"] and few_plan(128, 4096, 4096, adds=True)["in_memory"]
+
+
+def test_weights_of_more_tiles_than_ctas():
+    """They keep the form that shares tiles out block by block, unless the rows they read differ from run to run as it is."""
+    for T in FEW_TOKENS:
+        free = T <= 8 or T > 64
+        plan = few_plan(T, 51200, 5120)
+        assert plan["served"] == free and (not free or plan["ranges"] == 1), (T, plan)
+        assert not few_plan(T, 51200, 5120, in_memory=False)["served"]
+        assert few_plan(T, 50000, 1024)["served"] == 0                         # rows of 1,024 never meet in memory
+        assert few_plan(T, 151936, 4096)["served"] == 0
+    assert few_plan(129, 4096, 4096)["served"] == 0
+
+
+def test_shared_memory_of_a_plan_holds_what_the_kernel_lays_out():
+    """1,024 bytes of alignment, the ring, the area for shares, barriers and flags; what the MMA reads beyond the tokens, the tile on its
+    way out and the shares of a cluster, sent or parked, all inside."""
+    forms = set()
+    for N in (1, 16, 72, 515, 768, 1000, 2048, 3072, 4096, 5120, 6144, 7168, 9472, 10240, 12288, 18944, 24576, 34816, 37888, 51200, 75776):
+        for K in (8, 64, 72, 320, 512, 1024, 4096, 12288, 25600):
+            for T in FEW_TOKENS:
+                for adds in (False, True):
+                    p = few_plan(T, N, K, adds)
+                    if not p["served"]:
+                        continue
+                    what = (T, N, K, adds, p)
+                    padded, chunks, blocks = -(-T // 8) * 8, p["rows"] // 16, -(-K // 64)
+                    stage = (padded + p["rows"]) * 128
+                    assert p["rows"] % 16 == 0 and 16 <= p["rows"] <= 256 and (p["tiles"] - 1) * p["rows"] < N <= p["tiles"] * p["rows"], what
+                    assert 1 <= p["ranges"] <= blocks and 1 <= p["stages"] <= 12, what
+                    assert 1023 + p["ring"] + p["shares"] + (2 * 12 + 4) * 8 <= p["smem"] <= 112 * 1024, what
+                    assert p["ring"] >= max(p["stages"] * stage, (p["stages"] - 1) * stage + (64 if T <= 64 else 128) * 128), what
+                    if p["cluster"] == 1:
+                        assert p["ring"] >= T * (p["rows"] + 4) * 4 and p["shares"] == 0 and not p["fetched"], what
+                    else:
+                        assert p["cluster"] == p["ranges"] and p["ranges"] in (2, 4, 8) and not p["in_memory"], what
+                        if p["fetched"]:
+                            assert p["ring"] >= chunks * padded * 64 and p["shares"] == 0, what
+                        else:
+                            assert p["shares"] >= p["ranges"] * -(-chunks // p["ranges"]) * padded * 64, what
+                    forms.add((p["cluster"] > 1, p["fetched"], p["in_memory"]))
+    assert forms == {(False, 0, 0), (False, 0, 1), (True, 0, 0), (True, 1, 0)}

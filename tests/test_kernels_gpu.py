@@ -611,6 +611,39 @@ def test_gemm_tcgen05_few_tokens_over_tiles_and_ranges(M, N, K, form):
         assert torch.equal(whole[:offset], before[:offset]) and torch.equal(whole[offset + M * cols:], before[offset + M * cols:])
 
 
+@pytest.mark.parametrize("N,K,form", [(4096, 4096, "accumulate"), (5120, 17408, "accumulate"), (6144, 4096, "bias"), (10240, 5120, "bias"),
+                                      (24576, 4096, "swiglu"), (51200, 5120, "swiglu"), (768, 256, "swiglu"), (512, 384, "accumulate")])
+def test_gemm_tcgen05_a_row_of_few_tokens_has_the_same_bits_whatever_it_is_beside(N, K, form):
+    """With sums in memory off, one row gives the same bits alone and among up to 128: its sum is cut into the same K ranges, added in
+    the same order, on 64 rows of the MMA or 128, the shares of a cluster sent or fetched.  Once against the 64-bit product."""
+    o = ops()
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a = torch.randn(128, K, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    b = torch.randn(N, device="cuda", generator=g) if form in ("bias", "accumulate") else None
+    cols = N // 2 if form == "swiglu" else N
+    base = torch.randn(128, cols, device="cuda", generator=g)
+    outs = {}
+    o.gemm_sums_in_memory(False)
+    try:
+        for M in (128, 1, 8, 9, 24, 40, 60, 65, 96):
+            out = base[:M].clone()
+            o.gemm_tc(a[:M], w, out, b, accumulate=form == "accumulate", swiglu=form == "swiglu")
+            outs[M] = out
+    finally:
+        o.gemm_sums_in_memory(True)
+    o.check_device_errors()
+    for M, out in outs.items():
+        assert torch.equal(out, outs[128][:M]), (M, N, K, form)
+    ref = a[:9].double() @ w.double().T + (b.double() if b is not None else 0)
+    if form == "accumulate":
+        ref += base[:9].double()
+    elif form == "swiglu":
+        z = ref.view(9, N // 128, 2, 64)
+        ref = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(9, N // 2)
+    close(outs[9], ref.cpu(), "float32", scale=float(ref.abs().max()), what=f"few tokens in order {N}x{K} {form}")
+
+
 def test_gemm_tuning_knobs_move_the_plan():
     """The knobs behind the measured defaults: how many tokens send their K ranges to memory,
     and how many ranges a tile of a pair may be cut into."""
