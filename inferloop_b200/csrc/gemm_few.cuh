@@ -36,6 +36,11 @@ constexpr int kFewWarps = 8, kFewEpi = 32 * kFewWarps, kFewThreads = 64 + kFewEp
 constexpr int kFewStages = 12;
 // Two CTAs to an SM: 228 KB less 1 KB each that the system keeps, halved.
 constexpr int kFewSmem = 112 * 1024;
+// ... and never a third, however short the ring: a CTA holds up to 256 of an SM's 512 columns of tensor memory while it waits for the
+// others of its cluster, and tcgen05.alloc waits without a limit, so two clusters could each hold what the other one needs.
+// (Their registers, 78 to 93 of 320 threads, leave no room for a third either; that is the compiler's choice.)
+constexpr int kFewLeast = 77 * 1024;
+static_assert(3 * (kFewLeast + 1024) > 228 * 1024 && 2 * (kFewSmem + 1024) <= 228 * 1024, "two CTAs to an SM");
 
 struct FewParams {
   void* out;
@@ -469,6 +474,7 @@ bool few_memory(int T, int k_range, FewPlan& f) {
   const int staged = f.cluster == 1 ? (T * (f.rows + 4) * 4 + 15) / 16 * 16 : f.late ? f.rows * tp * 4 : 0;       // the tile on its way out
   if (staged > f.ring) f.ring = staged;
   f.smem = 1024 + f.ring + f.recv + kFewTail;                      // what the kernel lays out, in this order
+  if (f.smem < kFewLeast) f.smem = kFewLeast;
   return f.smem <= kFewSmem;
 }
 

@@ -126,3 +126,13 @@ def test_shared_memory_of_a_plan_holds_what_the_kernel_lays_out():
                             assert p["shares"] >= p["ranges"] * -(-chunks // p["ranges"]) * padded * 64, what
                     forms.add((p["cluster"] > 1, p["fetched"], p["in_memory"]))
     assert forms == {(False, 0, 0), (False, 0, 1), (True, 0, 0), (True, 1, 0)}
+
+
+def test_no_third_cta_of_a_product_of_few_tokens_fits_an_sm():
+    """Each holds up to 256 of the 512 columns of tensor memory while it waits for its cluster: three on an SM could wait for one
+    another without end.  An SM has 228 KB of shared memory, 1 KB of it kept for every CTA."""
+    for N, K in ((4096, 512), (6144, 256), (24576, 192), (72, 8), (768, 256), (2048, 2048), (1, 64), (1024, 1024), (4096, 4096)):
+        for T in FEW_TOKENS:
+            for adds in (False, True):
+                plan = few_plan(T, N, K, adds)
+                assert plan["rows"] <= 256 and 3 * (plan["smem"] + 1024) > 228 * 1024, (T, N, K, plan)
