@@ -29,7 +29,9 @@
 // (Tried and taken back: the RMS norm in front of a product of up to 16 tokens inside it, warps 2-9 reading the 32-bit rows, laying
 // them out ahead of the stream and leaving the root mean square to the result.  Launch after launch it took 0.3 to 0.8 us where the
 // norm's launch takes 1.7; in a step, where that launch hides behind its neighbours, 8B sizes lost 3 % at one token.)
-// All mbarrier waits are bounded, as in the other kernels.
+// All mbarrier waits are bounded, as in the other kernels.  One that runs out raises the error flag and nothing else: every thread goes on to
+// the end as if it had not (what it writes is flagged as invalid), so that no other one waits at a barrier that it left out and
+// every share that a peer counts is sent; warp 0 then stays until what it has requested from memory has landed.
 
 constexpr int kFewTokens = 128;
 constexpr int kFewWarps = 8, kFewEpi = 32 * kFewWarps, kFewThreads = 64 + kFewEpi;
@@ -38,7 +40,7 @@ constexpr int kFewStages = 12;
 constexpr int kFewSmem = 112 * 1024;
 // ... and never a third, however short the ring: a CTA holds up to 256 of an SM's 512 columns of tensor memory while it waits for the
 // others of its cluster, and tcgen05.alloc waits without a limit, so two clusters could each hold what the other one needs.
-// (Their registers, 78 to 93 of 320 threads, leave no room for a third either; that is the compiler's choice.)
+// (Their registers, 76 to 94 of 320 threads, leave no room for a third either; that is the compiler's choice.)
 constexpr int kFewLeast = 77 * 1024;
 static_assert(3 * (kFewLeast + 1024) > 228 * 1024 && 2 * (kFewSmem + 1024) <= 228 * 1024, "two CTAs to an SM");
 
@@ -113,6 +115,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   tcgen05_fence_after();
   const uint32_t tmem = *tmem_slot;
 
+  int armed = 0;                           // warp 0: blocks requested
   if (warp == 0) {
     bool ok = true;
     pdl_wait();
@@ -120,7 +123,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       for (int it = 0; it < n_early; ++it) tma_load_2d(base + it * p.stage_bytes, &map_y, full0 + 8 * it, (kb0 + it) * kBlockK, 0);
     int s = n_early == p.stages ? 0 : n_early;
     uint32_t ph = 0;
-    int armed = n_early;
+    armed = n_early;
     for (int it = n_early; it < cnt; ++it) {
       ok = mbar_wait(empty0 + 8 * s, ph);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
@@ -134,10 +137,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       armed = it + 1;
       if (++s == p.stages) { s = 0; ph ^= 1; }
     }
-    if (!ok && lane == 0) {
-      *failed = 1; if (p.error_flag) *p.error_flag = 1;
-      for (int it = armed > p.stages ? armed - p.stages : 0; it < armed; ++it) mbar_wait(full0 + 8 * (it % p.stages), (it / p.stages) & 1);
-    }
+    if (!ok && lane == 0) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
     __syncwarp();
     if (LATE) { cluster_sync_all(); cluster_sync_all(); }       // with the warps of the write-out
   } else if (warp == 1) {
@@ -171,9 +171,9 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const bool mine = t < p.T && (MM == 128 || lane < 16);
     const int nch = p.rows / 16;
     if (!mbar_wait(tfull, 0)) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
+    __syncwarp();
     tcgen05_fence_after();
     const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
-    const bool bad = *failed != 0;
     if (LATE || p.cluster > 1) {
       // ---- the K ranges of a tile are the CTAs of a cluster: chunk j of 16 columns belongs to CTA j % split
       // A chunk is [four columns][token][4], tokens swizzled by the column: a warp's stores are whole lines of 128 bytes, and a quarter
@@ -284,7 +284,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       __syncwarp();
       if (LATE) cluster_sync_all();           // nobody leaves while a peer may still read its share
       else if (!arrived && !mbar_wait(rbar, 0)) { *failed = 1; if (p.error_flag) *p.error_flag = 1; }
-    } else if (!bad) {
+    } else {
       // ---- the tile (or its K range) through shared memory: the ring is idle, everything in it has been consumed
       float* st = reinterpret_cast<float*>(smem);
       const int pitch = p.rows + 4;
@@ -354,6 +354,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   }
   tcgen05_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *failed)
+    for (int it = armed > p.stages ? armed - p.stages : 0; it < armed; ++it) mbar_wait(full0 + 8 * (it % p.stages), (it / p.stages) & 1);
   if (warp == 1) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols) : "memory");

@@ -136,3 +136,37 @@ def test_no_third_cta_of_a_product_of_few_tokens_fits_an_sm():
             for adds in (False, True):
                 plan = few_plan(T, N, K, adds)
                 assert plan["rows"] <= 256 and 3 * (plan["smem"] + 1024) > 228 * 1024, (T, N, K, plan)
+
+
+def test_a_wait_that_runs_out_leaves_no_thread_of_a_product_of_few_tokens_behind():
+    """Read in the kernel's source: no barrier, and no load that a whole warp has to issue, stands under a condition that threads could see
+    differently once a wait has run out; nothing returns early; and what was requested from memory is awaited at the end."""
+    import os
+    import re
+
+    import inferloop_b200.csrc as csrc
+    text = open(os.path.join(csrc.__path__[0], "gemm_few.cuh")).read()
+    body = text[text.index("gemm_few_kernel("):text.index("// ------------------------------------------------------------------ host side")]
+    body = re.sub(r'"[^"\n]*bar\.sync[^"\n]*"', "BARRIER", re.sub(r"//[^\n]*", "", body))
+    body = re.sub(r'"[^"\n]*"', "", re.sub(r"for \([^{]*?;[^{]*?;[^{]*?\)", "for ()", body))
+    together = re.compile(r"BARRIER|__syncthreads\(|__syncwarp\(|cluster_sync_all\(|tmem_load_16\(")
+    private = re.compile(r"\b(failed|bad|ok|arrived|mbar_wait)\b")
+    around, statement, found = [], "", 0
+    for piece in re.split(r"([{};])", body):
+        if piece == "{":
+            around.append(statement)
+            statement = ""
+        elif piece == "}":
+            around.pop()
+            statement = ""
+        elif piece == ";":
+            if together.search(statement):
+                found += 1
+                for condition in around + [statement]:
+                    assert not private.search(condition), (statement.strip(), condition.strip())
+            statement = ""
+        else:
+            statement += piece
+    assert found >= 12 and not around and not re.search(r"\breturn\b", body)
+    end = body[body.rindex("__syncthreads("):]
+    assert re.search(r"\*failed\)\s*for \(\)\s*mbar_wait\(full0", end), "requested blocks have to land before the block ends"
