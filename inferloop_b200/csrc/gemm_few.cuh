@@ -16,9 +16,9 @@
 // 6,144 x 4,096, 8 tokens 11.8 -> 11.6 (7.7), 96 tokens 22.0 -> 15.1; 10,240 x 5,120, 64 tokens 27.8 -> 22.6 (16.0).
 //
 // Per CTA (320 threads):
-//   warp 0     requests the weight blocks by TMA (128-byte swizzle; one box a block, or for gated weights a box of
-//              eight gate rows and their eight up rows for every 16 rows of the tile, so that a tile need not be
-//              whole blocks of 64) into a ring of `stages` buffers, the first ring before the kernel waits for its
+//   warp 0     requests the weight blocks by TMA (128-byte swizzle; one box a block, or for gated weights boxes of up to 128 rows in
+//              which eight gate rows and their eight up rows alternate, so that a tile need not be whole blocks of 64; boxes of 16
+//              rows alone took 6.6 us where these take 6.0, 6,144 x 1,024 at 16 tokens) into a ring of `stages` buffers, the first ring before the kernel waits for its
 //              predecessor; one lane requests the token blocks behind the wait;
 //   warp 1     tensor memory; one lane issues tcgen05.mma, four to a K block of 64;
 //   warps 2-9  the write-out.  With one K range, or ranges that meet in memory (red.add), the tile goes through the
@@ -49,7 +49,7 @@ struct FewParams {
   const float* bias;
   int* error_flag;
   int T, N, K, ldo;
-  int rows, tp, k_blocks, split, cluster, stages, tmem_cols, red;
+  int rows, tp, k_blocks, split, cluster, stages, tmem_cols, red, groups;
   int stage_bytes, ring_bytes, recv_bytes;
   int epilogue, out_f32, relu2, gate_relu;
   float act_limit, act_sharp, act_offset;
@@ -77,12 +77,12 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   const int n_early = cnt < p.stages ? cnt : p.stages;
   const uint32_t w_off = (uint32_t)p.tp * 128u;
   const uint32_t tx = (uint32_t)(p.rows + p.tp) * 128u;
-  const int boxes = gated ? p.rows / 16 : 1;
+  const int boxes = gated ? p.rows / (16 * p.groups) : 1;
   auto load_w = [&](uint32_t dst, uint32_t bar, int kcol) {
     if (gated) {
       if (lane < boxes) {
-        const int g = row0 / 16 + lane;
-        tma_load_5d(dst + w_off + (uint32_t)lane * 2048u, &map_w, bar, kcol, 0, g & 7, 0, g >> 3);
+        const int g = row0 / 16 + lane * p.groups;
+        tma_load_5d(dst + w_off + (uint32_t)(lane * p.groups) * 2048u, &map_w, bar, kcol, 0, 0, g & 7, g >> 3);
       }
     } else if (lane == 0) {
       tma_load_2d(dst + w_off, &map_w, bar, kcol, row0);
@@ -365,19 +365,26 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 // ------------------------------------------------------------------ host side
 constexpr int kFewTail = (2 * kFewStages + 4) * 8;     // barriers, flags
 
-// The interleaved weight [rows, cols]: boxes of eight gate rows and their eight up rows, 64 deep.
-int make_gated_map(CUtensorMap* out, const void* ptr, int rows, int cols, int ld) {
+// Groups of 16 gated rows in a box: as many as divide a tile, so that no box crosses a block of 128 rows.
+int few_groups(int rows) {
+  int n = 8;
+  while (rows % (16 * n) != 0) n /= 2;
+  return n;
+}
+
+// The interleaved weight [rows, cols]: boxes of `groups` times eight gate rows and their eight up rows, 64 deep, inside a block of 128 rows.
+int make_gated_map(CUtensorMap* out, const void* ptr, int rows, int cols, int ld, int groups) {
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   static std::mutex mu;
-  const MapKey key{ptr, rows, cols, ld, 0};
+  const MapKey key{ptr, rows, cols, ld, groups};
   std::lock_guard<std::mutex> g(mu);
   auto it = cache.find(key);
   if (it != cache.end()) { *out = it->second; return 0; }
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail("gemm_tc: cuTensorMapEncodeTiled is not available from this driver");
   const cuuint64_t ldb = (cuuint64_t)ld * 2;
-  const cuuint64_t dims[5] = {(cuuint64_t)cols, 8, 8, 2, (cuuint64_t)(rows / 128)}, strides[4] = {ldb, 8 * ldb, 64 * ldb, 128 * ldb};
-  const cuuint32_t box[5] = {(cuuint32_t)kBlockK, 8, 1, 2, 1}, estr[5] = {1, 1, 1, 1, 1};
+  const cuuint64_t dims[5] = {(cuuint64_t)cols, 8, 2, 8, (cuuint64_t)(rows / 128)}, strides[4] = {ldb, 64 * ldb, 8 * ldb, 128 * ldb};
+  const cuuint32_t box[5] = {(cuuint32_t)kBlockK, 8, 2, (cuuint32_t)groups, 1}, estr[5] = {1, 1, 1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail("gemm_tc: cuTensorMapEncodeTiled failed with code %d (gated rows %d cols %d ld %d)", (int)r, rows, cols, ld);
@@ -390,7 +397,7 @@ template <int MM, bool LATE>
 cudaError_t configure_few() {
   static OncePerDevice once;
   return once.run([] {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MM, LATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MM, LATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kFewSmem);
     if (e == cudaSuccess)      // two CTAs share an SM only with the largest shared-memory carve-out
       cudaFuncSetAttribute(gemm_few_kernel<MM, LATE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     return e;
@@ -437,7 +444,8 @@ FewDevice few_device() {
 }
 
 // How a product of few tokens is dealt out.  late: the shares of a cluster are parked in the rings and fetched.
-struct FewPlan { int rows, split, stages, cluster, late, red, tiles, grid, ring, recv, smem; };    // recv: 0 when late
+// deep: one CTA to an SM with the shared memory of two.
+struct FewPlan { int rows, split, stages, cluster, late, deep, red, tiles, grid, ring, recv, smem; };    // recv: 0 when late
 
 // Into how many K ranges a tile's sum is cut where their order is kept.  It belongs to the weight alone, so that a row's bits are the
 // same whatever it is computed beside: what tiles of 128 rows allow, in ranges of equal length, of CTAs that the device
@@ -461,11 +469,12 @@ int few_ranges_in_memory(int T, int N, int K, const FewDevice& d) {
   return rest != 0 && tiles * 12 >= d.sms && add_split(rest, (K + kBlockK - 1) / kBlockK) >= 2 ? 8 : 1;
 }
 
-// The shared memory of a plan, with as many stages as two CTAs to an SM leave room for; false when two do not fit.
+// The shared memory of a plan, with as many stages as the CTAs of an SM leave room for; false when they do not fit.
 bool few_memory(int T, int k_range, FewPlan& f) {
+  const int most = f.deep ? 2 * kFewSmem : kFewSmem;
   const int tp = (T + 7) / 8 * 8, stage = (tp + f.rows) * 128, mm = T <= 64 ? 64 : 128;
   f.recv = f.cluster > 1 && !f.late ? f.split * ((f.rows / 16 + f.split - 1) / f.split) * tp * 64 : 0;
-  const int room = kFewSmem - 1024 - kFewTail - f.recv;
+  const int room = most - 1024 - kFewTail - f.recv;
   f.stages = room / stage;
   if (f.stages > kFewStages) f.stages = kFewStages;
   if (f.stages > k_range) f.stages = k_range;
@@ -477,31 +486,35 @@ bool few_memory(int T, int k_range, FewPlan& f) {
   if (staged > f.ring) f.ring = staged;
   f.smem = 1024 + f.ring + f.recv + kFewTail;                      // what the kernel lays out, in this order
   if (f.smem < kFewLeast) f.smem = kFewLeast;
-  return f.smem <= kFewSmem;
+  return f.smem <= most;
 }
 
-// What ranks the plans of a product (it is no time): a fit to 6,313 timed plans of 253 products, 20 weights (1,024 to 51,200 rows, 1,024 to
-// 25,600 deep) at 1 to 128 tokens.  The plan it picks is on average 1.3 % slower than the fastest that was timed, 23 % at worst
-// (4,096 x 1,024 at 40 tokens, 7.5 against 6.1 us).  What decides is not an SM's share of the bytes but how long a CTA's stream is
-// against its ring (a round trip for `stages` blocks of 64) and how many MMAs are issued (four a block, each as long as 118
-// columns at least); a second CTA on some SMs leaves less room to the next kernel's first blocks; and the write-out costs by the
-// value.  Shares that are parked and fetched cost two to three us more than shares that are sent: they pay where the area
-// for the latter would leave a ring of one to three stages (6,144 x 4,096 at 96 tokens 16.9 -> 15.2 us, 12,288 x 2,048 at 128 18.8 -> 15.6).
-double few_cost(int T, int N, int K, const FewPlan& f, const FewDevice& d) {
+// What ranks the plans of a product (it is no time): a fit to 16,000 timed plans of 29 weights (256 to 51,200 rows, 256 to 25,600
+// deep) at 18 token counts from 1 to 128.  The plan it picks is on average 1.5 % slower than the fastest that
+// was timed, 22 % at worst (1,280 x 256 at 112 tokens, 5.2 against 4.3 us).  What decides is not an SM's share of the bytes
+// but how long a CTA's stream is against its ring (a round trip for `stages` blocks of 64), how many MMAs are issued (four a block,
+// each as long as 118 columns at least) and how many boxes a gated block is fetched in; a second CTA on some SMs leaves less
+// room to the next kernel's first blocks; and the write-out costs by the value, in a cluster by what its busiest CTA adds up.
+// Shares that are parked and fetched cost some us more than shares that are sent: they pay where the area for the latter would
+// leave a ring of one to three stages (6,144 x 4,096 at 96 tokens 16.9 -> 15.2 us, 12,288 x 2,048 at 128 18.8 -> 15.6).
+double few_cost(int T, int N, int K, bool gated, const FewPlan& f, const FewDevice& d) {
   const int kb = (K + kBlockK - 1) / kBlockK, range = (kb + f.split - 1) / f.split, sms = d.sms;
-  const int per_sm = f.grid <= sms ? 1 : 2;
-  const double bytes = (double)N * K * 2 / 7.0e6, ring = 2.85 * range / f.stages, tile = 1e-3 * T * f.rows;
-  double t = (bytes > ring ? bytes : ring) + 0.204 * range + 0.147 * per_sm * range * (f.rows > 118 ? f.rows / 128.0 : 0.92);
-  if (per_sm == 2) t += 0.866 + 2.62 * (f.grid - sms) / sms;
-  if (f.red) t += 0.794 * f.split * 4e-6 * T * N;
-  else if (f.cluster > 1) t += (0.388 + 0.118 * per_sm) * tile + 0.272 * f.split + (f.late ? 2.87 + 0.186 * per_sm * tile : 0.0);
-  else t += 1.55 * tile;
+  const int per_sm = f.grid <= sms ? 1 : 2, chunks = f.rows / 16;
+  const double bytes = (double)N * K * 2 / 7.0e6, ring = 2.868 * range / f.stages, tile = 1e-3 * T * f.rows;
+  double t = (bytes > ring ? bytes : ring) + 0.118 * range + 0.14 * per_sm * range * (f.rows > 118 ? f.rows / 128.0 : 0.92);
+  if (per_sm == 2) t += 0.551 + 2.02 * (f.grid - sms) / sms;
+  if (gated) t += 0.006 * per_sm * range * (chunks / few_groups(f.rows));
+  if (f.red) t += 0.952 * f.split * 4e-6 * T * N;
+  else if (f.cluster > 1) {
+    const double own = 1e-3 * T * 16 * f.split * ((chunks + f.split - 1) / f.split);
+    t += (0.35 + 0.045 * per_sm) * tile + (0.137 + 0.125 * per_sm) * own + 0.187 * f.split + (f.late ? 5.149 + 0.081 * per_sm * tile : 0.0);
+  } else t += 0.31 * tile;
   return t;
 }
 
 // `can_add`: the product adds into a 32-bit output whose rows are 16-byte multiples.  False where the kernel does not serve: more
 // tokens, or a weight of more tiles than two CTAs to an SM.
-bool few_plan(int T, int N, int K, bool can_add, const FewDevice& d, FewPlan& best) {
+bool few_plan(int T, int N, int K, bool can_add, bool gated, const FewDevice& d, FewPlan& best) {
   if (T > kFewTokens || (N + 255) / 256 > 2 * d.sms) return false;
   const int meet = can_add ? few_ranges_in_memory(T, N, K, d) : 1;
   int ranges = few_ranges(N, K, d);
@@ -517,14 +530,15 @@ bool few_plan(int T, int N, int K, bool can_add, const FewDevice& d, FewPlan& be
   struct Hash { size_t operator()(const Key& k) const { return std::hash<long long>()(k.a * 1000003ll ^ k.b); } };
   static std::unordered_map<Key, FewPlan, Hash> cache;
   static std::mutex mu;
-  const Key key{((long long)T << 32) | (unsigned)N, ((long long)K << 16) | (meet << 8) | ranges};
+  const Key key{((long long)T << 32) | (unsigned)N, ((long long)K << 16) | (gated ? 1 << 12 : 0) | (meet << 8) | ranges};
   std::lock_guard<std::mutex> g(mu);
   auto it = cache.find(key);
   if (it != cache.end()) { best = it->second; return best.rows > 0; }
   const int kb = (K + kBlockK - 1) / kBlockK;
   // Clusters are not placed in the last slots while the kernel before still holds some: 280 and 292 CTAs lost 5 to 6 % to 256.
-  // More than 64 tokens that add in memory: one CTA to an SM (two take 0.5 to 1 us less of 10 to 45, but a product of many tokens
-  // has never had more).
+  // More than 64 tokens that add in memory: one CTA to an SM, as a product of many tokens has had them, with the shared memory of
+  // two; with half of it a ring of three blocks of 144 rows was all there was room for (5,120 x 17,408 at 128 tokens 40.9 -> 34.2 us,
+  // 5,120 x 25,600 at 96 55.7 -> 46.7, 4,096 x 12,288 at 96 25.0 -> 21.4).
   const int most = meet == 1 ? 2 * d.sms * 15 / 16 : T > 64 ? d.sms : 2 * d.sms;
   double least = 1e30;
   best = FewPlan{};
@@ -534,17 +548,19 @@ bool few_plan(int T, int N, int K, bool can_add, const FewDevice& d, FewPlan& be
         FewPlan f{};
         f.rows = rows; f.split = split; f.red = meet > 1 && split > 1 ? 1 : 0; f.cluster = f.red ? 1 : split; f.late = late;
         f.tiles = (N + rows - 1) / rows; f.grid = f.tiles * split;
+        f.deep = meet > 1 && T > 64 && f.grid <= d.sms ? 1 : 0;
         if (f.grid > (split > 1 ? most : 2 * d.sms) && at_once) continue;
         if (f.cluster > 1 && f.tiles > d.two[f.cluster] && at_once) continue;       // or the last ones cost a second round
         if (!few_memory(T, kb / split, f)) continue;
-        const double t = few_cost(T, N, K, f, d);
+        const double t = few_cost(T, N, K, gated, f, d);
         if (t < least) { least = t; best = f; }
       }
   };
   if (meet > 1)
-    for (int split = 1; split <= meet && split <= kb; ++split) consider(split, true);
+    for (int split = 2; split <= meet && split <= kb; ++split) consider(split, true);
   else
     consider(ranges, true);
+  if (best.rows == 0 && meet > 1) consider(1, true);
   if (best.rows == 0 && meet == 1 && ranges > 1) consider(ranges, false);
   if (cache.size() > 4096) cache.clear();
   cache.emplace(key, best);
@@ -554,18 +570,18 @@ bool few_plan(int T, int N, int K, bool can_add, const FewDevice& d, FewPlan& be
 template <int MM, bool LATE>
 int launch_few(const CUtensorMap& mw, const CUtensorMap& my, const FewParams& p, const FewPlan& f, cudaStream_t stream) {
   const cudaError_t e = configure_few<MM, LATE>();
-  if (e != cudaSuccess) return fail("gemm_tc: cannot reserve %d bytes of shared memory: %s", kFewSmem, cudaGetErrorString(e));
+  if (e != cudaSuccess) return fail("gemm_tc: cannot reserve %d bytes of shared memory: %s", 2 * kFewSmem, cudaGetErrorString(e));
   ilb::launch_cluster(gemm_few_kernel<MM, LATE>, dim3(f.grid), dim3(kFewThreads), (size_t)f.smem, stream, p.cluster, mw, my, p);
   return check_launch("gemm_tc");
 }
 
 // Fills in the deal and launches; `p` holds everything else.
 int run_few(FewParams& p, const FewPlan& f, const void* A, int lda, const void* W, int ldw, cudaStream_t stream) {
-  p.rows = f.rows; p.tp = (p.T + 7) / 8 * 8; p.k_blocks = (p.K + kBlockK - 1) / kBlockK; p.split = f.split; p.cluster = f.cluster;
+  p.rows = f.rows; p.groups = few_groups(f.rows); p.tp = (p.T + 7) / 8 * 8; p.k_blocks = (p.K + kBlockK - 1) / kBlockK; p.split = f.split; p.cluster = f.cluster;
   p.stages = f.stages; p.red = f.red; p.stage_bytes = (p.tp + p.rows) * 128; p.ring_bytes = f.ring; p.recv_bytes = f.recv;
   p.tmem_cols = p.rows <= 32 ? 32 : p.rows <= 64 ? 64 : p.rows <= 128 ? 128 : 256;
   CUtensorMap mw, my;
-  if (p.epilogue == kSwiGLU ? make_gated_map(&mw, W, p.N, p.K, ldw) : make_map(&mw, W, p.N, p.K, ldw, p.rows)) return -1;
+  if (p.epilogue == kSwiGLU ? make_gated_map(&mw, W, p.N, p.K, ldw, p.groups) : make_map(&mw, W, p.N, p.K, ldw, p.rows)) return -1;
   if (make_map(&my, A, p.T, p.K, lda, p.tp)) return -1;
   if (f.late) return p.T <= 64 ? launch_few<64, true>(mw, my, p, f, stream) : launch_few<128, true>(mw, my, p, f, stream);
   return p.T <= 64 ? launch_few<64, false>(mw, my, p, f, stream) : launch_few<128, false>(mw, my, p, f, stream);

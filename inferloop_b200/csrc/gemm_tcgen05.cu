@@ -1404,7 +1404,7 @@ ILB_EXPORT int ilb_gemm_tc(const void* A, const void* W, const float* bias, void
   const bool tma_reach = ((uintptr_t)out % 16 == 0) && ((long long)ldo * es) % 16 == 0;   // rows of 16-byte multiples from a 16-byte base
   const bool can_add = tma_reach && out_f32 && accumulate == 1;
   FewPlan few;
-  if (max_ctas <= 0 && few_plan(M, N, K, can_add, few_device(), few)) {
+  if (max_ctas <= 0 && few_plan(M, N, K, can_add, accumulate == kSwiGLU, few_device(), few)) {
     FewParams q = few_params(p);
     return run_few(q, few, A, lda, W, ldw, stream);
   }
@@ -1503,7 +1503,7 @@ ILB_EXPORT int ilb_gemm_tc_plan(int M, int N, int K, int epilogue, int* out) {
   Params p{};
   p.M = M; p.N = N; p.K = K; p.k_blocks = (K + kBlockK - 1) / kBlockK; p.epilogue = epilogue;
   FewPlan few;
-  if (few_plan(M, N, K, epilogue == 1, few_device(), few)) {
+  if (few_plan(M, N, K, epilogue == 1, epilogue == 2, few_device(), few)) {
     // (65 to 128 tokens whose ranges meet in memory are reported as a product of many tokens, which also let them meet there)
     out[0] = M <= 64 || !few.red; out[1] = (M + 7) / 8 * 8; out[2] = 1; out[3] = few.grid; out[4] = few.cluster;
     out[5] = 0; out[6] = few.tiles; out[7] = few.red ? few.tiles : 0; out[8] = few.red; out[9] = 0; out[10] = 0;
@@ -1524,17 +1524,17 @@ ILB_EXPORT int ilb_gemm_tc_plan(int M, int N, int K, int epilogue, int* out) {
   return 0;
 }
 
-// The plan of a product of few tokens on a device with these facts (for tests; needs no GPU): SMs, then the clusters of 2, 4 and 8 CTAs
+// The plan of a product of few tokens (epilogue 0: plain, 1: adding, 2: gated) on a device with these facts (for tests; needs no GPU): SMs, then the clusters of 2, 4 and 8 CTAs
 // that it holds at once with one CTA to an SM and with two.  out[0..10] = served, rows of a tile, K ranges, stages, cluster, shares that
 // are fetched from the rings, ranges that meet in memory, tiles, bytes of the ring, of the area for shares, of all shared memory.
-ILB_EXPORT int ilb_gemm_few_plan(int T, int N, int K, int can_add, const int* facts, int* out) {
+ILB_EXPORT int ilb_gemm_few_plan(int T, int N, int K, int epilogue, const int* facts, int* out) {
   ILB_REQUIRE(T > 0 && N > 0 && K > 0 && facts != nullptr && out != nullptr && facts[0] > 0, "gemm_tc: bad sizes for a plan");
   FewDevice d{};
   d.sms = facts[0];
   d.one[1] = d.sms; d.two[1] = 2 * d.sms;
   for (int i = 0; i < 3; ++i) { d.one[2 << i] = facts[1 + i]; d.two[2 << i] = facts[4 + i]; }
   FewPlan f{};
-  const bool served = few_plan(T, N, K, can_add != 0, d, f);
+  const bool served = few_plan(T, N, K, epilogue == 1, epilogue == 2, d, f);
   const int v[11] = {served ? 1 : 0, f.rows, f.split, f.stages, f.cluster, f.late, f.red, f.tiles, f.ring, f.recv, f.smem};
   for (int i = 0; i < 11; ++i) out[i] = v[i];
   return 0;

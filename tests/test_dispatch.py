@@ -40,7 +40,7 @@ FEW_KEYS = ("served", "rows", "ranges", "stages", "cluster", "fetched", "in_memo
 FEW_TOKENS = (1, 2, 7, 8, 9, 16, 17, 24, 33, 40, 48, 64, 65, 72, 96, 104, 128)
 
 
-def few_plan(T, N, K, adds=False, in_memory=True):
+def few_plan(T, N, K, adds=False, in_memory=True, gated=False):
     """The plan on a device of 148 SMs that holds 74, 33 and 15 clusters of 2, 4 and 8 CTAs with one CTA to an SM and 148, 71 and 33
     with two."""
     import ctypes
@@ -50,7 +50,7 @@ def few_plan(T, N, K, adds=False, in_memory=True):
     lib.ilb_gemm_tc_sums_in_memory(1 if in_memory else 0)
     try:
         out = (ctypes.c_int * len(FEW_KEYS))()
-        assert lib.ilb_gemm_few_plan(T, N, K, 1 if adds else 0, (ctypes.c_int * 7)(SMS, 74, 33, 15, 148, 71, 33), out) == 0
+        assert lib.ilb_gemm_few_plan(T, N, K, 2 if gated else 1 if adds else 0, (ctypes.c_int * 7)(SMS, 74, 33, 15, 148, 71, 33), out) == 0
         return dict(zip(FEW_KEYS, out))
     finally:
         lib.ilb_gemm_tc_sums_in_memory(1)
@@ -114,7 +114,8 @@ def test_shared_memory_of_a_plan_holds_what_the_kernel_lays_out():
                     stage = (padded + p["rows"]) * 128
                     assert p["rows"] % 16 == 0 and 16 <= p["rows"] <= 256 and (p["tiles"] - 1) * p["rows"] < N <= p["tiles"] * p["rows"], what
                     assert 1 <= p["ranges"] <= blocks and 1 <= p["stages"] <= 12, what
-                    assert 1023 + p["ring"] + p["shares"] + (2 * 12 + 4) * 8 <= p["smem"] <= 112 * 1024, what
+                    deep = T > 64 and p["in_memory"] and p["tiles"] * p["ranges"] <= SMS
+                    assert 1023 + p["ring"] + p["shares"] + (2 * 12 + 4) * 8 <= p["smem"] <= (224 if deep else 112) * 1024, what
                     assert p["ring"] >= max(p["stages"] * stage, (p["stages"] - 1) * stage + (64 if T <= 64 else 128) * 128), what
                     if p["cluster"] == 1:
                         assert p["ring"] >= T * (p["rows"] + 4) * 4 and p["shares"] == 0 and not p["fetched"], what
@@ -126,6 +127,23 @@ def test_shared_memory_of_a_plan_holds_what_the_kernel_lays_out():
                             assert p["shares"] >= p["ranges"] * -(-chunks // p["ranges"]) * padded * 64, what
                     forms.add((p["cluster"] > 1, p["fetched"], p["in_memory"]))
     assert forms == {(False, 0, 0), (False, 0, 1), (True, 0, 0), (True, 1, 0)}
+
+
+def test_plans_of_products_that_had_become_slower():
+    """Products that the kernel of few tokens took longer over than the kernels before it (4,096 x 512 adding at 64 tokens 7.9 -> 9.5 us,
+    5,120 x 17,408 adding at 128 38.1 -> 40.9, 6,144 x 1,024 gated at 24 6.65 -> 7.05, 3,072 x 4,096 at 1 token 8.0 -> 8.6): more
+    of the SMs' slots, a deeper ring, gated tiles that are fetched in whole blocks."""
+    for T in (57, 64):
+        plan = few_plan(T, 4096, 512, adds=True)
+        assert plan["tiles"] * plan["ranges"] >= 220, plan
+    for T in (72, 80, 96, 112, 128):
+        for N, K in ((4096, 12288), (5120, 5120), (5120, 8192), (5120, 17408), (5120, 25600)):
+            plan = few_plan(T, N, K, adds=True)
+            assert plan["in_memory"] and plan["stages"] >= 5 and plan["tiles"] * plan["ranges"] <= SMS, (T, N, K, plan)
+    for T in (19, 24, 32):
+        assert few_plan(T, 6144, 1024, gated=True)["rows"] % 64 == 0, T
+    for T in (1, 2, 4, 8):
+        assert few_plan(T, 3072, 4096)["rows"] <= 144, T
 
 
 def test_no_third_cta_of_a_product_of_few_tokens_fits_an_sm():
