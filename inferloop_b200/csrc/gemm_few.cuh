@@ -489,7 +489,7 @@ bool few_memory(int T, int k_range, FewPlan& f) {
   return f.smem <= most;
 }
 
-// What ranks the plans of a product (it is no time): a fit to 16,000 timed plans of 29 weights (256 to 51,200 rows, 256 to 25,600
+// What ranks the plans of a product (it is no time): a fit to 12,000 timed plans of 29 weights (256 to 51,200 rows, 256 to 25,600
 // deep) at 18 token counts from 1 to 128.  The plan it picks is on average 1.5 % slower than the fastest that
 // was timed, 22 % at worst (1,280 x 256 at 112 tokens, 5.2 against 4.3 us).  What decides is not an SM's share of the bytes
 // but how long a CTA's stream is against its ring (a round trip for `stages` blocks of 64), how many MMAs are issued (four a block,

@@ -1498,15 +1498,18 @@ ILB_EXPORT int ilb_gemm_tc_sums_in_memory(int on) {
 // tiles, tiles handled stream-K fashion, whether the K ranges of a tile are added in memory;
 // out[9..10] = pairs of CTAs and K ranges per tile when the product runs on pairs (else 0, 0;
 // an output that TMA cannot reach keeps the single-CTA tiles whatever this says).
+// out[11] = the kernel: 0 gemm_tc_kernel, 1 gemm_pair_kernel, 2 gemm_few_kernel; out[12..15], for the last one only (else 0) = weight rows
+// of a tile, K ranges of a tile, stages of the ring, whether a cluster's shares are fetched.  For the last one out[0] keeps apart
+// what it did for the kernels before it: 0 for 65 to 128 tokens whose ranges meet in memory, else 1.
 ILB_EXPORT int ilb_gemm_tc_plan(int M, int N, int K, int epilogue, int* out) {
   ILB_REQUIRE(M > 0 && N > 0 && K > 0 && out != nullptr && epilogue >= 0 && epilogue <= 2, "gemm_tc: bad sizes for a plan");
   Params p{};
   p.M = M; p.N = N; p.K = K; p.k_blocks = (K + kBlockK - 1) / kBlockK; p.epilogue = epilogue;
   FewPlan few;
   if (few_plan(M, N, K, epilogue == 1, epilogue == 2, few_device(), few)) {
-    // (65 to 128 tokens whose ranges meet in memory are reported as a product of many tokens, which also let them meet there)
     out[0] = M <= 64 || !few.red; out[1] = (M + 7) / 8 * 8; out[2] = 1; out[3] = few.grid; out[4] = few.cluster;
     out[5] = 0; out[6] = few.tiles; out[7] = few.red ? few.tiles : 0; out[8] = few.red; out[9] = 0; out[10] = 0;
+    out[11] = 2; out[12] = few.rows; out[13] = few.split; out[14] = few.stages; out[15] = few.late;
     return 0;
   }
   Plan plan{};
@@ -1514,18 +1517,18 @@ ILB_EXPORT int ilb_gemm_tc_plan(int M, int N, int K, int epilogue, int* out) {
   out[0] = plan.swap ? 1 : 0; out[1] = plan.bn; out[2] = plan.ms; out[3] = (int)plan.grid; out[4] = p.cluster;
   out[5] = p.dp_waves; out[6] = p.tiles_x * p.tiles_y; out[7] = (int)(p.tiles_x * (long long)p.tiles_y - p.sk_tile0);
   out[8] = plan.additive ? 1 : 0;
-  out[9] = 0; out[10] = 0;
+  for (int i = 9; i < 16; ++i) out[i] = 0;
   PairPlan pp{};
   if (!plan.swap && g_pairs != 0 && pair_plan(M, N, K, epilogue == 1 && g_sums_in_memory, pair_capacity(), pp) &&
       pair_wanted(pp, epilogue)) {
-    out[9] = pp.n_pairs; out[10] = pp.split;
+    out[9] = pp.n_pairs; out[10] = pp.split; out[11] = 1;
     out[8] = pp.split > 1 ? 1 : 0;
   }
   return 0;
 }
 
-// The plan of a product of few tokens (epilogue 0: plain, 1: adding, 2: gated) on a device with these facts (for tests; needs no GPU): SMs, then the clusters of 2, 4 and 8 CTAs
-// that it holds at once with one CTA to an SM and with two.  out[0..10] = served, rows of a tile, K ranges, stages, cluster, shares that
+// The plan of a product of few tokens (epilogue 0: plain, 1: adding, 2: gated) on a device with these facts (for tests; needs no GPU): SMs,
+// then the clusters of 2, 4 and 8 CTAs that it holds at once with one CTA to an SM and with two.  out[0..10] = served, rows of a tile, K ranges, stages, cluster, shares that
 // are fetched from the rings, ranges that meet in memory, tiles, bytes of the ring, of the area for shares, of all shared memory.
 ILB_EXPORT int ilb_gemm_few_plan(int T, int N, int K, int epilogue, const int* facts, int* out) {
   ILB_REQUIRE(T > 0 && N > 0 && K > 0 && facts != nullptr && out != nullptr && facts[0] > 0, "gemm_tc: bad sizes for a plan");

@@ -1312,20 +1312,26 @@ def gemm_tuning(few_tokens_in_memory: Optional[int] = None, few_tokens_ranges: i
 
 def gemm_tc_plan(M: int, N: int, K: int, accumulate: bool = False, swiglu: bool = False) -> dict:
     """How `gemm_tc` deals out a product of these sizes (needs a device: the answer depends
-    on how many CTAs fit it).  Up to 128 tokens on the kernel of few tokens (gemm_few.cuh): `tile_n` is the token
-    block's height, `tiles` and `grid` its deal, `cluster` the ranges of a tile that meet in K order; `swap` is 0
-    there for 65 to 128 tokens whose ranges meet in memory.  `pairs` > 0: the product runs on that many pairs of CTAs, each
-    tile left over after the whole rounds (or every tile) cut into `pair_split` K ranges, and
-    `sums_meet_in_memory` speaks of those; the other fields then describe the single-CTA deal
+    on how many CTAs fit it).  `kernel` is the one that runs: "few_tokens" (gemm_few.cuh, up to 128 tokens), "pairs" or
+    "single" (gemm_tcgen05.cu).
+
+    "few_tokens": `tile_rows` weight rows a tile, `ranges` K ranges a tile (the CTAs of a `cluster`, their shares `fetched` or
+    sent; or, with `sums_meet_in_memory`, separate CTAs), `stages` of the ring, `tiles` and `grid` as dealt out; `tile_n` is the token
+    block's height.  `row_blocks`, `rounds`, `tiles_stream_k` and `swap` say nothing about this kernel: they keep the values
+    by which callers told the kernels before it apart (`swap` 0 for 65 to 128 tokens whose ranges meet in memory).
+    "pairs": the product runs on `pairs` pairs of CTAs, each tile left over after the whole rounds (or every tile) cut into
+    `pair_split` K ranges, and `sums_meet_in_memory` speaks of those; the other fields then describe the single-CTA deal
     that `gemm_pairs(0)` would use."""
     lib = load_module("gemm_tcgen05")
-    out = (ctypes.c_int * 11)()
+    out = (ctypes.c_int * 16)()
     lib.ilb_gemm_tc_plan.restype = ctypes.c_int
     if lib.ilb_gemm_tc_plan(_i(M), _i(N), _i(K), _i(2 if swiglu else (1 if accumulate else 0)), out) != 0:
         raise KernelError(lib.ilb_last_error().decode())
     keys = ("swap", "tile_n", "row_blocks", "grid", "cluster", "rounds", "tiles", "tiles_stream_k", "sums_meet_in_memory",
-            "pairs", "pair_split")
-    return dict(zip(keys, list(out)))
+            "pairs", "pair_split", "kernel", "tile_rows", "ranges", "stages", "fetched")
+    plan = dict(zip(keys, list(out)))
+    plan["kernel"] = ("single", "pairs", "few_tokens")[plan["kernel"]]
+    return plan
 
 
 def device_error_tensor(device) -> Optional[torch.Tensor]:

@@ -644,6 +644,32 @@ def test_gemm_tcgen05_a_row_of_few_tokens_has_the_same_bits_whatever_it_is_besid
     close(outs[9], ref.cpu(), "float32", scale=float(ref.abs().max()), what=f"few tokens in order {N}x{K} {form}")
 
 
+def test_gemm_plan_says_which_kernel_runs_and_how():
+    """The reported plan is the one that runs: the kernel, the height of a tile, the ranges and where they meet; and every form of the
+    kernel of few tokens is taken somewhere."""
+    o = ops()
+
+    def plan(M, N, K, **kw):
+        p = o.gemm_tc_plan(M, N, K, **kw)
+        if p["kernel"] == "few_tokens":
+            assert p["tiles"] == -(-N // p["tile_rows"]) and p["grid"] == p["tiles"] * p["ranges"] and p["stages"] >= 1, (M, N, K, kw, p)
+            assert p["cluster"] == (1 if p["sums_meet_in_memory"] else p["ranges"]), (M, N, K, kw, p)
+        else:
+            assert p["tile_rows"] == p["ranges"] == p["stages"] == p["fetched"] == 0, (M, N, K, kw, p)
+        return p
+    whole = plan(8, 24576, 4096, swiglu=True)
+    assert whole["kernel"] == "few_tokens" and whole["ranges"] == 1
+    sent, fetched = plan(16, 4096, 4096, accumulate=True), plan(128, 6144, 4096)
+    assert sent["kernel"] == fetched["kernel"] == "few_tokens" and sent["cluster"] > 1 and fetched["cluster"] > 1
+    assert not sent["fetched"] and fetched["fetched"]
+    for M in (8, 96):
+        meet = plan(M, 4096, 12288, accumulate=True)
+        assert meet["kernel"] == "few_tokens" and meet["sums_meet_in_memory"] and meet["ranges"] > 1
+    assert plan(8, 1408, 2048, swiglu=True)["tile_rows"] % 64 != 0           # a gated tile that ends inside a block of 64
+    assert plan(8, 151936, 4096)["kernel"] == "single" and plan(200, 6144, 4096)["kernel"] == "single"
+    assert plan(2048, 24576, 4096, swiglu=True)["kernel"] == "pairs"
+
+
 def test_gemm_tuning_knobs_move_the_plan():
     """The knobs behind the measured defaults: how many tokens send their K ranges to memory,
     and how many ranges a tile of a pair may be cut into."""
