@@ -1,5 +1,6 @@
 """Each kernel alone against a plain 64-bit statement of the same operation, at sizes
 other than the engine configurations' (GPU)."""
+import ctypes
 import math
 import random
 
@@ -642,6 +643,42 @@ def test_gemm_tcgen05_a_row_of_few_tokens_has_the_same_bits_whatever_it_is_besid
         z = ref.view(9, N // 128, 2, 64)
         ref = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(9, N // 2)
     close(outs[9], ref.cpu(), "float32", scale=float(ref.abs().max()), what=f"few tokens in order {N}x{K} {form}")
+
+
+@pytest.mark.parametrize("M", [3, 24, 96])
+@pytest.mark.parametrize("form", ["accumulate", "bias", "silu", "relu", "gelu_tanh", "clamped"])
+def test_gemm_tcgen05_few_tokens_on_strided_operands(M, form):
+    """Operands and outputs that are columns of wider matrices (what lies beside the output stays): a last unit of one column, added in
+    memory alone (3 and 96 tokens) or in order (24); every gate on tiles that begin and end inside a block of 64."""
+    o = ops()
+    gated = form not in ("accumulate", "bias")
+    N, K = (1408, 2048) if gated else (4093, 2048)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn(M, K + 24, device="cuda", generator=g).to(torch.bfloat16)[:, 8:8 + K]
+    w = (torch.randn(N, K + 40, device="cuda", generator=g) * 0.05).to(torch.bfloat16)[:, 16:16 + K]
+    b = torch.randn(N, device="cuda", generator=g) if not gated else None
+    cols, wide = (N // 2, N // 2 + 12) if gated else (N, 4100)
+    whole = torch.randn(M, wide, device="cuda", generator=g).to(torch.float32 if form == "accumulate" else torch.bfloat16)
+    out, before = whole[:, :cols], whole.clone()
+    ref = a.double().cpu() @ w.double().cpu().T
+    if gated:
+        z = ref.view(M, N // 128, 2, 64)
+        gate, up = z[:, :, 0], z[:, :, 1]
+        ref = {"silu": lambda: torch.nn.functional.silu(gate) * up, "relu": lambda: torch.relu(gate) * up,
+               "gelu_tanh": lambda: torch.nn.functional.gelu(gate, approximate="tanh") * up,
+               "clamped": lambda: gate.clamp(max=2.0) * torch.sigmoid(1.702 * gate.clamp(max=2.0)) * (up.clamp(-2.0, 2.0) + 1.0)}[form]().reshape(M, cols)
+    else:
+        ref = ref + b.double().cpu() + (before[:, :cols].double().cpu() if form == "accumulate" else 0)
+    assert o.gemm_tc_plan(M, N, K, accumulate=form == "accumulate", swiglu=gated)["sums_meet_in_memory"] == (form == "accumulate" and M != 24)
+    # (the library's entry: `gemm_tc` asks for contiguous tensors)
+    mode = {"bias": 0, "accumulate": 1, "silu": 2, "relu": 3, "clamped": 4, "gelu_tanh": 6}[form]
+    st = o._tc_state(a.device)
+    o._call("gemm_tcgen05", "ilb_gemm_tc", o._ptr(a), o._ptr(w), o._ptr(b), o._ptr(out), o._i(out.dtype == torch.float32), o._i(M), o._i(N), o._i(K),
+            o._i(a.stride(0)), o._i(w.stride(0)), o._i(out.stride(0)), o._i(mode), o._ptr(st.workspace), ctypes.c_longlong(st.floats), o._ptr(st.tickets),
+            o._i(st.n_tickets), o._ptr(st.error), o._i(0), o._f(2.0), o._f(1.702), o._f(1.0), o._stream(out))
+    o.check_device_errors()
+    close(out, ref, "float32" if form == "accumulate" else "bfloat16", scale=float(ref.abs().max()), what=f"few tokens, strided {M} {form}")
+    assert torch.equal(whole[:, cols:], before[:, cols:])
 
 
 def test_gemm_plan_says_which_kernel_runs_and_how():
