@@ -431,16 +431,19 @@ int few_clusters(int cluster, int smem) {
 }
 
 FewDevice few_device() {
+  constexpr int kMax = 64;
   static std::mutex mu;
-  static FewDevice known{};
+  static FewDevice known[kMax] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMax) dev = 0;
   std::lock_guard<std::mutex> g(mu);
-  if (known.sms == 0) {
+  if (known[dev].sms == 0) {
     FewDevice d{};
-    d.sms = sm_count();
+    if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || d.sms <= 0) d.sms = 148;
     for (int c = 1; c <= 8; c *= 2) { d.one[c] = few_clusters(c, 2 * kFewSmem); d.two[c] = few_clusters(c, kFewSmem); }
-    known = d;
+    known[dev] = d;
   }
-  return known;
+  return known[dev];
 }
 
 // How a product of few tokens is dealt out.  late: the shares of a cluster are parked in the rings and fetched.
@@ -526,11 +529,12 @@ bool few_plan(int T, int N, int K, bool can_add, bool gated, const FewDevice& d,
     if (few_ranges_in_memory(T, K, K, d) == 1) return false;
     ranges = 1;
   }
-  struct Key { long long a, b; bool operator==(const Key& o) const { return a == o.a && b == o.b; } };
-  struct Hash { size_t operator()(const Key& k) const { return std::hash<long long>()(k.a * 1000003ll ^ k.b); } };
+  struct Key { long long a, b, c; bool operator==(const Key& o) const { return a == o.a && b == o.b && c == o.c; } };
+  struct Hash { size_t operator()(const Key& k) const { return std::hash<long long>()((k.a * 1000003ll ^ k.b) * 1000003ll ^ k.c); } };
   static std::unordered_map<Key, FewPlan, Hash> cache;
   static std::mutex mu;
-  const Key key{((long long)T << 32) | (unsigned)N, ((long long)K << 16) | (gated ? 1 << 12 : 0) | (meet << 8) | ranges};
+  const Key key{((long long)T << 32) | (unsigned)N, ((long long)K << 16) | (gated ? 1 << 12 : 0) | (meet << 8) | ranges,
+                ((((long long)d.sms << 10 | d.two[2]) << 10 | d.two[4]) << 10 | d.two[8])};        // all that a plan asks of the device
   std::lock_guard<std::mutex> g(mu);
   auto it = cache.find(key);
   if (it != cache.end()) { best = it->second; return best.rows > 0; }

@@ -40,7 +40,10 @@ FEW_KEYS = ("served", "rows", "ranges", "stages", "cluster", "fetched", "in_memo
 FEW_TOKENS = (1, 2, 7, 8, 9, 16, 17, 24, 33, 40, 48, 64, 65, 72, 96, 104, 128)
 
 
-def few_plan(T, N, K, adds=False, in_memory=True, gated=False):
+B200 = (SMS, 74, 33, 15, 148, 71, 33)
+
+
+def few_plan(T, N, K, adds=False, in_memory=True, gated=False, device=B200):
     """The plan on a device of 148 SMs that holds 74, 33 and 15 clusters of 2, 4 and 8 CTAs with one CTA to an SM and 148, 71 and 33
     with two."""
     import ctypes
@@ -50,7 +53,7 @@ def few_plan(T, N, K, adds=False, in_memory=True, gated=False):
     lib.ilb_gemm_tc_sums_in_memory(1 if in_memory else 0)
     try:
         out = (ctypes.c_int * len(FEW_KEYS))()
-        assert lib.ilb_gemm_few_plan(T, N, K, 2 if gated else 1 if adds else 0, (ctypes.c_int * 7)(SMS, 74, 33, 15, 148, 71, 33), out) == 0
+        assert lib.ilb_gemm_few_plan(T, N, K, 2 if gated else 1 if adds else 0, (ctypes.c_int * 7)(*device), out) == 0
         return dict(zip(FEW_KEYS, out))
     finally:
         lib.ilb_gemm_tc_sums_in_memory(1)
@@ -188,3 +191,12 @@ def test_a_wait_that_runs_out_leaves_no_thread_of_a_product_of_few_tokens_behind
     assert found >= 12 and not around and not re.search(r"\breturn\b", body)
     end = body[body.rindex("__syncthreads("):]
     assert re.search(r"\*failed\)\s*for \(\)\s*mbar_wait\(full0", end), "requested blocks have to land before the block ends"
+
+
+def test_a_plan_belongs_to_the_device_it_was_made_for():
+    """Plans are kept by all that they depend on: one made for a device of half the size is not handed to a whole one."""
+    half = (74, 37, 16, 7, 74, 35, 16)
+    for T, N, K, gated in ((8, 18944, 1024, True), (24, 12288, 3072, False), (3, 6144, 2560, False)):
+        small = few_plan(T, N, K, gated=gated, device=half)
+        whole = few_plan(T, N, K, gated=gated)
+        assert small["tiles"] * small["ranges"] <= 2 * 74 and small["ranges"] * 2 == whole["ranges"], (T, N, K, small, whole)
