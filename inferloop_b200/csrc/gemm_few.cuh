@@ -10,15 +10,16 @@
 // columns, so that a tile may be any multiple of 16 rows up to 256.  `few_plan` picks the height for which the CTAs, two to an
 // SM, come out even; into how many K ranges a sum is cut belongs to the weight (`few_ranges`), unless the ranges meet in
 // memory.  Launch after launch on rotating weights (us; former deal -> this one; in brackets the weight's bytes at 6.54 TB/s,
-// the rate of a copy, which reads and writes: reads alone have reached 7.1): 24,576 x 4,096 gated, 8 tokens 35.1 -> 32.2
-// (30.8), 64 tokens 43.5 -> 34.8, 128 tokens 55.7 -> 39.7; 51,200 x 5,120 gated, 1 token 84.0 -> 76.1 (80.2), 72 tokens
-// 129.7 -> 84.4; 5,120 x 17,408 adding, 8 tokens 30.1 -> 28.2 (27.3), 24 tokens 35.6 -> 30.9, 64 tokens 40.2 -> 33.5;
-// 6,144 x 4,096, 8 tokens 11.8 -> 11.6 (7.7), 96 tokens 22.0 -> 15.1; 10,240 x 5,120, 64 tokens 27.8 -> 22.6 (16.0).
+// the rate of a copy, which reads and writes: reads alone have reached 7.1): 24,576 x 4,096 gated, 8 tokens 34.8 -> 32.4
+// (30.8), 64 tokens 43.8 -> 34.6, 128 tokens 54.1 -> 39.6; 51,200 x 5,120 gated, 1 token 83.6 -> 76.4 (80.2), 96 tokens
+// 129.6 -> 83.4; 5,120 x 17,408 adding, 8 tokens 30.0 -> 28.6 (27.3), 24 tokens 33.7 -> 31.0, 64 tokens 39.5 -> 33.6;
+// 6,144 x 4,096, 8 tokens 11.9 -> 11.6 (7.7), 96 tokens 22.1 -> 15.2; 10,240 x 5,120, 64 tokens 27.8 -> 22.6 (16.0).
+// Over 29 weights at 19 token counts 0.81 of the time; 20 of the 551 take 1 to 4 % longer.
 //
 // Per CTA (320 threads):
 //   warp 0     requests the weight blocks by TMA (128-byte swizzle; one box a block, or for gated weights boxes of up to 128 rows in
 //              which eight gate rows and their eight up rows alternate, so that a tile need not be whole blocks of 64; boxes of 16
-//              rows alone took 6.6 us where these take 6.0, 6,144 x 1,024 at 16 tokens) into a ring of `stages` buffers, the first ring before the kernel waits for its
+//              rows cost small weights: 6,144 x 1,024 at 24 tokens 7.05 -> 6.35 us) into a ring of `stages` buffers, the first ring before the kernel waits for its
 //              predecessor; one lane requests the token blocks behind the wait;
 //   warp 1     tensor memory; one lane issues tcgen05.mma, four to a K block of 64;
 //   warps 2-9  the write-out.  With one K range, or ranges that meet in memory (red.add), the tile goes through the
@@ -522,8 +523,8 @@ bool few_plan(int T, int N, int K, bool can_add, bool gated, const FewDevice& d,
   const int meet = can_add ? few_ranges_in_memory(T, N, K, d) : 1;
   int ranges = few_ranges(N, K, d);
   // A weight of more 128-row tiles than two CTAs to an SM: whole tiles here, but only where the adding products of its width let their
-  // ranges meet in memory, so that the rows it reads differ from run to run as it is (51,200 x 5,120 gated, 8 tokens 76.9 us
-  // here and 85.9 in `make_plan`'s form, 96 tokens 84.8 and 139.2).  Elsewhere it keeps that form, and so its bits, although 24
+  // ranges meet in memory, so that the rows it reads differ from run to run as it is (51,200 x 5,120 gated, 8 tokens 76.7 us
+  // here and 84.6 in `make_plan`'s form, 96 tokens 83.4 and 129.6).  Elsewhere it keeps that form, and so its bits, although 24
   // tokens take 91.2 us where whole tiles took 77.5.
   if (ranges == 0 && meet == 1) {
     if (few_ranges_in_memory(T, K, K, d) == 1) return false;
